@@ -336,11 +336,11 @@ __global__ void k_max_final(const double* __restrict__ part, uint32_t nparts, do
 // inside it.  A range lying wholly below h is skipped (home <= neighbour).
 // Leaves come out in ascending bin order, starting with h itself.
 //
-// Pass 1 (fill == false) counts neighbours, join work units and candidate
-// pairs per home bin; pass 2 writes the neighbour list and the units.  The
-// neighbour list of h is cut into segments of about `seg_cap` candidate
-// points, and the home bin into chunks of `chunk` points; one unit is one
-// (chunk, segment) combination.
+// Pass 1 (FILL false) counts neighbours and candidate points per home bin;
+// k_unit_plan turns them into units; pass 2 writes the neighbour list and the
+// units.  The candidate points of h's neighbour list are cut into segments of
+// equal length, and the home bin into chunks of `chunk` points; one unit is
+// one (chunk, segment) combination.
 __device__ __forceinline__ uint32_t lower_bound_u64(const uint64_t* __restrict__ a, uint32_t lo,
                                                     uint32_t hi, uint64_t v) {
   while (lo < hi) {
@@ -452,117 +452,289 @@ __device__ __forceinline__ void walk_levels(const uint64_t* __restrict__ bkey, u
   }
 }
 
-template <bool FILL>
-__global__ void __launch_bounds__(128, 8) k_enum(const uint64_t* __restrict__ bkey, const uint32_t* __restrict__ bstart,
-                       uint32_t m, EnumParams P, uint32_t* __restrict__ nbr_cnt,
-                       uint32_t* __restrict__ unit_cnt, uint32_t* __restrict__ unit_cnt_tc,
-                       unsigned long long* __restrict__ cand, const uint32_t* __restrict__ nbr_off,
-                       const uint32_t* __restrict__ unit_off, const uint32_t* __restrict__ unit_off_tc,
-                       uint32_t* __restrict__ nbr, Unit* __restrict__ units_simt, Unit* __restrict__ units_tc) {
-  const uint32_t hb = blockIdx.x * blockDim.x + threadIdx.x;
-  if (hb >= m) return;
-  const uint64_t K = bkey[hb];
-  const uint32_t asz = bstart[hb + 1] - bstart[hb];
+// The split of a home bin's work into units: home chunks of csz points (nch
+// of them, nch_s in the sample) against segments of `seg` candidate points.
+// Segment b covers the candidate ranks [b seg, (b + 1) seg) of the bin's
+// neighbour list, wherever the bin boundaries fall; unit b * nch_s + c is
+// segment b of the c-th sampled chunk.
+struct HomeSplit {
+  bool tc;             // tensor-core units
+  uint32_t csz, nch, nch_s;
+  unsigned long long rows_s, self_s;  // sampled home points, and their pairs inside the bin
+};
+
+__device__ __forceinline__ HomeSplit home_split(const EnumParams& P, uint32_t hb, uint32_t asz) {
+  HomeSplit s;
   // large home bins go to the tensor-core join (128-row chunks), the rest to the CUDA-core join
-  const bool tc = P.tc_min > 0 && asz >= P.tc_min;
-  const uint32_t csz = tc ? P.tc_chunk : P.chunk;
-  const uint32_t nchunks = (asz + csz - 1) / csz;
-  Unit* __restrict__ units = tc ? units_tc : units_simt;
-  // sampled home points: chunks taken, home points and their pairs inside the bin
-  uint32_t nchunks_s = nchunks;
-  unsigned long long rows_s = asz, self_s = (unsigned long long)asz * (asz - (asz > 0)) / 2;
+  s.tc = P.tc_min > 0 && asz >= P.tc_min;
+  s.csz = s.tc ? P.tc_chunk : P.chunk;
+  s.nch = (asz + s.csz - 1) / s.csz;
+  s.nch_s = s.nch;
+  s.rows_s = asz;
+  s.self_s = (unsigned long long)asz * (asz - (asz > 0)) / 2;
   if (P.sample > 1) {
-    nchunks_s = 0;
-    for (uint32_t ch = 0; ch < nchunks; ++ch) nchunks_s += group_sampled(hb, ch * csz / SAMPLE_GROUP, P.sample);
-    rows_s = 0;
-    self_s = 0;
+    s.nch_s = 0;
+    for (uint32_t ch = 0; ch < s.nch; ++ch) s.nch_s += group_sampled(hb, ch * s.csz / SAMPLE_GROUP, P.sample);
+    s.rows_s = 0;
+    s.self_s = 0;
     for (uint32_t g0 = 0; g0 < asz; g0 += SAMPLE_GROUP) {
       if (!group_sampled(hb, g0 / SAMPLE_GROUP, P.sample)) continue;
       const unsigned long long g1 = min(asz, g0 + SAMPLE_GROUP), c = g1 - g0;
-      rows_s += c;
-      self_s += c * (asz - 1) - (g0 + g1 - 1) * c / 2;  // pairs (p, q) of the bin with p in the group, q > p
+      s.rows_s += c;
+      s.self_s += c * (asz - 1) - (g0 + g1 - 1) * c / 2;  // pairs (p, q) of the bin with p in the group, q > p
     }
   }
+  return s;
+}
 
+// Writes the units of segment b that end at (s1, o1) -- when b >= 0 -- and
+// the start (s0, o0) of those of segment b + 1, when there is one.  lane and
+// lanes: the threads that share the work.
+__device__ __forceinline__ void write_cut(Unit* __restrict__ units, const EnumParams& P, const HomeSplit& s,
+                                          uint32_t hb, int b, uint32_t nseg, uint32_t s1, uint32_t o1, uint32_t s0,
+                                          uint32_t o0, uint32_t lane, uint32_t lanes) {
+  for (uint32_t c = lane; c < s.nch; c += lanes) {
+    uint32_t r = c;  // rank of chunk c among the sampled ones
+    if (P.sample > 1) {
+      if (!group_sampled(hb, c * s.csz / SAMPLE_GROUP, P.sample)) continue;
+      r = 0;
+      for (uint32_t e = 0; e < c; ++e) r += group_sampled(hb, e * s.csz / SAMPLE_GROUP, P.sample);
+    }
+    if (b >= 0) {
+      Unit& u = units[(size_t)b * s.nch_s + r];
+      u.s1 = s1;
+      u.o1 = o1;
+    }
+    if ((uint32_t)(b + 1) < nseg) {
+      Unit& u = units[(size_t)(b + 1) * s.nch_s + r];
+      u.h = hb;
+      u.chunk = c;
+      u.s0 = s0;
+      u.o0 = o0;
+    }
+  }
+}
 
-  uint32_t cnt = 0, nseg = 0, seg_fill = 0, seg_begin = 0;
-  unsigned long long c = 0;
-  uint32_t w_nbr = FILL ? nbr_off[hb] : 0;
-  uint32_t w_unit = FILL ? (tc ? unit_off_tc[hb] : unit_off[hb]) : 0;
+// Adds the home bin's candidate points, once per home chunk, to its class's
+// total (the segment lengths are chosen from it).
+__device__ __forceinline__ void add_work(idx::EnumTotals* tot, unsigned long long v, bool tc) {
+  unsigned long long w[2] = {tc ? 0ull : v, tc ? v : 0ull};
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) w[k] += __shfl_xor_sync(FULL_MASK, w[k], o);
+    if ((threadIdx.x & 31) == 0 && w[k]) atomicAdd(&tot->work[k], w[k]);
+  }
+}
 
-  // Visits neighbour bin `a` (ascending, a >= hb): candidate count, segment
-  // split and, in pass 2, the neighbour list and the units.
-  auto leaf = [&](uint32_t a) {
-    const uint32_t bsz = bstart[a + 1] - bstart[a];
-    c += (a == hb) ? self_s : rows_s * bsz;
-    if (seg_fill > 0 && seg_fill + bsz > (tc ? P.seg_cap_tc : P.seg_cap)) {
+template <bool FILL>
+__global__ void __launch_bounds__(128, 8) k_enum(const uint64_t* __restrict__ bkey, const uint32_t* __restrict__ bstart,
+                       uint32_t m, EnumParams P, uint32_t* __restrict__ npts, uint32_t* __restrict__ nbr_cnt,
+                       idx::EnumTotals* __restrict__ tot, const uint32_t* __restrict__ nbr_off,
+                       const uint32_t* __restrict__ unit_off, const uint32_t* __restrict__ unit_off_tc,
+                       uint32_t* __restrict__ nbr, Unit* __restrict__ units_simt, Unit* __restrict__ units_tc) {
+  const uint32_t hb = blockIdx.x * blockDim.x + threadIdx.x;
+  unsigned long long work = 0;
+  bool tc = false;
+  if (hb < m) {
+    const uint64_t K = bkey[hb];
+    const uint32_t asz = bstart[hb + 1] - bstart[hb];
+    const HomeSplit hsp = home_split(P, hb, asz);
+    tc = hsp.tc;
+    uint32_t cnt = 0, pts = 0;
+    const uint32_t n0 = FILL ? nbr_off[hb] : 0u;
+    const uint32_t seg = FILL ? tot->seg[tc ? 1 : 0] : 0u;
+    const uint32_t total = FILL ? npts[hb] : 0u;
+    const uint32_t nseg = FILL ? (uint32_t)(((unsigned long long)total + seg - 1) / seg) : 0u;
+    Unit* units = FILL ? (tc ? units_tc + unit_off_tc[hb] : units_simt + unit_off[hb]) : nullptr;
+    unsigned long long cut = seg;  // candidate rank of the next segment boundary
+    int b = 0;
+    if (FILL) write_cut(units, P, hsp, hb, -1, nseg, 0, 0, n0, 0, 0, 1);
+
+    // Visits neighbour bin `a` (ascending, a >= hb): its points, and in pass
+    // 2 the neighbour list and the segment boundaries that fall inside it.
+    auto leaf = [&](uint32_t a) {
+      const uint32_t bsz = bstart[a + 1] - bstart[a];
       if (FILL) {
-        for (uint32_t ch = 0; ch < nchunks; ++ch)
-          if (group_sampled(hb, ch * csz / SAMPLE_GROUP, P.sample))
-            units[w_unit++] = Unit{hb, ch, nbr_off[hb] + seg_begin, nbr_off[hb] + cnt};
-      }
-      ++nseg;
-      seg_fill = 0;
-      seg_begin = cnt;
-    }
-    seg_fill += bsz;
-    if (FILL) nbr[w_nbr++] = a;
-    ++cnt;
-  };
-
-  if (P.k == 0) {
-    leaf(hb);  // no key fields: one bin holding every point
-  } else if (P.p == 0) {
-    walk_levels<3>(bkey, K, hb, P, 0, 0u, m, 0ull, leaf);
-  } else {
-    // prefixes in ascending order: field j offset by digit j of c in base 3
-    // (field 0 most significant)
-    uint32_t n3 = 1;
-    for (int q = 0; q < P.p; ++q) n3 *= 3;
-    for (uint32_t cb = 0; cb < n3; ++cb) {
-      uint32_t rem = cb, pw = n3 / 3, idx = 0;
-      uint64_t pre = 0;
-      bool ok = true;
-      for (int q = 0; q < P.p; ++q) {
-        const uint32_t t = rem / pw;
-        rem -= t * pw;
-        pw /= 3;
-        const int cv = key_field(K, P, q) + (int)t - 1;
-        if (cv < 0 || (uint32_t)cv > P.maxkey[q]) {
-          ok = false;
-          break;
+        nbr[n0 + cnt] = a;
+        for (; cut <= (unsigned long long)pts + bsz; cut += seg, ++b) {
+          const uint32_t o = (uint32_t)(cut - pts);  // 1 .. bsz
+          write_cut(units, P, hsp, hb, b, nseg, n0 + cnt + 1, o, n0 + cnt + (o == bsz), o == bsz ? 0u : o, 0, 1);
         }
-        idx += (uint32_t)cv * P.stride[q];
-        pre |= (uint64_t)cv << P.shift[q];
+        if (pts + bsz == total && b < (int)nseg)  // the list ends inside segment b
+          write_cut(units, P, hsp, hb, b, nseg, n0 + cnt + 1, bsz, 0, 0, 0, 1);
       }
-      if (!ok) continue;
-      const uint32_t r0 = P.ptab[idx], r1 = P.ptab[idx + 1];
-      if (r0 == r1 || r1 <= hb) continue;
-      if (P.p == P.k) {  // every field fixed: the single bin r0 (>= hb)
-        leaf(r0);
-        continue;
+      pts += bsz;
+      ++cnt;
+    };
+
+    if (P.k == 0) {
+      leaf(hb);  // no key fields: one bin holding every point
+    } else if (P.p == 0) {
+      walk_levels<3>(bkey, K, hb, P, 0, 0u, m, 0ull, leaf);
+    } else {
+      // prefixes in ascending order: field j offset by digit j of c in base 3
+      // (field 0 most significant)
+      uint32_t n3 = 1;
+      for (int q = 0; q < P.p; ++q) n3 *= 3;
+      for (uint32_t cb = 0; cb < n3; ++cb) {
+        uint32_t rem = cb, pw = n3 / 3, idx = 0;
+        uint64_t pre = 0;
+        bool ok = true;
+        for (int q = 0; q < P.p; ++q) {
+          const uint32_t t = rem / pw;
+          rem -= t * pw;
+          pw /= 3;
+          const int cv = key_field(K, P, q) + (int)t - 1;
+          if (cv < 0 || (uint32_t)cv > P.maxkey[q]) {
+            ok = false;
+            break;
+          }
+          idx += (uint32_t)cv * P.stride[q];
+          pre |= (uint64_t)cv << P.shift[q];
+        }
+        if (!ok) continue;
+        const uint32_t r0 = P.ptab[idx], r1 = P.ptab[idx + 1];
+        if (r0 == r1 || r1 <= hb) continue;
+        if (P.p == P.k) {  // every field fixed: the single bin r0 (>= hb)
+          leaf(r0);
+          continue;
+        }
+        walk_levels<3>(bkey, K, hb, P, P.p, r0, r1, pre, leaf);
       }
-      walk_levels<3>(bkey, K, hb, P, P.p, r0, r1, pre, leaf);
+    }
+    if (!FILL) {
+      nbr_cnt[hb] = cnt;
+      npts[hb] = pts;
+      work = (unsigned long long)hsp.nch_s * pts;
     }
   }
-  if (cnt > 0) {
+  if (!FILL) add_work(tot, work, tc);
+}
+
+// The same enumeration with a warp per home bin: the keys from the bin itself
+// up to the last one whose field 0 is within one of its own are read 32 at a
+// time and every field is compared.  A thread's walk takes up to 3^k
+// dependent steps, and with few bins nothing hides them: at 62 bins, k = 8,
+// the two passes took 7.4 ms, at 292 bins, k = 6, 0.8 ms.
+constexpr int FLAT_WARPS = 4;
+template <bool FILL>
+__global__ void __launch_bounds__(FLAT_WARPS * 32)
+k_enum_flat(const uint64_t* __restrict__ bkey, const uint32_t* __restrict__ bstart, uint32_t m, EnumParams P,
+            uint32_t* __restrict__ npts, uint32_t* __restrict__ nbr_cnt, idx::EnumTotals* __restrict__ tot,
+            const uint32_t* __restrict__ nbr_off, const uint32_t* __restrict__ unit_off,
+            const uint32_t* __restrict__ unit_off_tc, uint32_t* __restrict__ nbr, Unit* __restrict__ units_simt,
+            Unit* __restrict__ units_tc) {
+  const uint32_t hb = blockIdx.x * FLAT_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (hb >= m) return;  // warp-uniform
+  const uint64_t K = bkey[hb];
+  const uint32_t asz = bstart[hb + 1] - bstart[hb];
+  const HomeSplit hsp = home_split(P, hb, asz);
+  uint32_t end = m;
+  if (P.k > 0) {
+    const uint64_t f0 = (uint64_t)key_field(K, P, 0) + 2;
+    if (f0 <= P.maxkey[0]) end = lower_bound_u64(bkey, hb, m, f0 << P.shift[0]);
+  }
+  uint32_t cnt = 0, pts = 0;
+  const uint32_t n0 = FILL ? nbr_off[hb] : 0u;
+  const uint32_t seg = FILL ? tot->seg[hsp.tc ? 1 : 0] : 0u;
+  const uint32_t total = FILL ? npts[hb] : 0u;
+  const uint32_t nseg = FILL ? (uint32_t)(((unsigned long long)total + seg - 1) / seg) : 0u;
+  Unit* units = FILL ? (hsp.tc ? units_tc + unit_off_tc[hb] : units_simt + unit_off[hb]) : nullptr;
+  unsigned long long cut = seg;
+  int b = 0;
+  if (FILL) write_cut(units, P, hsp, hb, -1, nseg, 0, 0, n0, 0, lane, 32);
+  for (uint32_t c0 = hb; c0 < end; c0 += 32) {
+    const uint32_t a = c0 + lane;
+    bool ok = a < end;
+    const uint64_t Ka = ok ? bkey[a] : 0ull;
+    for (int j = 0; j < P.k && __any_sync(FULL_MASK, ok); ++j) {
+      const int df = key_field(Ka, P, j) - key_field(K, P, j);
+      ok = ok && df >= -1 && df <= 1;
+    }
+    const uint32_t hit = __ballot_sync(FULL_MASK, ok);
+    if (!hit) continue;
+    const uint32_t bsz = ok ? bstart[a + 1] - bstart[a] : 0u;
+    uint32_t incl = bsz;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(FULL_MASK, incl, o);
+      if (lane >= (uint32_t)o) incl += y;
+    }
+    const uint32_t step = __shfl_sync(FULL_MASK, incl, 31);
     if (FILL) {
-      for (uint32_t ch = 0; ch < nchunks; ++ch)
-        if (group_sampled(hb, ch * csz / SAMPLE_GROUP, P.sample))
-          units[w_unit++] = Unit{hb, ch, nbr_off[hb] + seg_begin, nbr_off[hb] + cnt};
+      const uint32_t pos = n0 + cnt + __popc(hit & ((1u << lane) - 1u));
+      if (ok) nbr[pos] = a;
+      // segment boundaries among these bins' points (warp-uniform loop)
+      for (; cut <= (unsigned long long)pts + step; cut += seg, ++b) {
+        const uint32_t r = (uint32_t)(cut - pts);  // 1 .. step: inside the first bin whose inclusive end reaches r
+        const int src = __ffs(__ballot_sync(FULL_MASK, ok && incl >= r)) - 1;
+        const uint32_t e = __shfl_sync(FULL_MASK, pos, src), z = __shfl_sync(FULL_MASK, bsz, src);
+        const uint32_t o = r - (__shfl_sync(FULL_MASK, incl, src) - z);
+        write_cut(units, P, hsp, hb, b, nseg, e + 1, o, e + (o == z), o == z ? 0u : o, lane, 32);
+      }
+      if (pts + step == total && b < (int)nseg) {  // the list ends inside segment b
+        const int src = 31 - __clz(hit);
+        write_cut(units, P, hsp, hb, b, nseg, __shfl_sync(FULL_MASK, pos, src) + 1, __shfl_sync(FULL_MASK, bsz, src), 0,
+                  0, lane, 32);
+      }
     }
-    ++nseg;
+    pts += step;
+    cnt += __popc(hit);
   }
-  if (!FILL) {
-    // a bin's unit count saturates at 2^32 - 1; the 64-bit totals of the
-    // three count arrays (k_count_totals) then exceed the 32-bit offsets the
-    // work lists use, and the call fails with MISTIC_ERR_TOO_LARGE
-    const unsigned long long nu = (unsigned long long)nseg * nchunks_s;
-    const uint32_t nu32 = nu > 0xffffffffull ? 0xffffffffu : (uint32_t)nu;
+  if (!FILL && lane == 0) {
     nbr_cnt[hb] = cnt;
-    unit_cnt[hb] = tc ? 0u : nu32;
-    unit_cnt_tc[hb] = tc ? nu32 : 0u;
-    cand[hb] = c;
+    npts[hb] = pts;
+    const unsigned long long work = (unsigned long long)hsp.nch_s * pts;
+    if (work) atomicAdd(&tot->work[hsp.tc ? 1 : 0], work);
+  }
+}
+
+// Segment lengths from the work totals, and the units and candidate pairs of
+// every home bin.  A join of little work gets segments short enough for
+// want_units units of each class: with 4096-point segments the 100,000 x 18
+// uniform join had 2,145 CUDA-core units on 4,864 resident warps and ran as
+// long as its slowest one (1.78 ms).
+__global__ void k_unit_plan(const uint32_t* __restrict__ bstart, uint32_t m, EnumParams P,
+                            const uint32_t* __restrict__ npts, const uint32_t* __restrict__ nbr_cnt,
+                            uint32_t* __restrict__ unit_cnt, uint32_t* __restrict__ unit_cnt_tc,
+                            idx::EnumTotals* __restrict__ tot) {
+  uint32_t seg[2];
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    seg[c] = P.seg_max[c];
+    if (P.want_units[c]) {
+      const unsigned long long fair = (tot->work[c] / P.want_units[c] + 127) & ~127ull;
+      seg[c] = (uint32_t)min((unsigned long long)P.seg_max[c], max((unsigned long long)P.seg_min[c], fair));
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x < 2) tot->seg[threadIdx.x] = seg[threadIdx.x];
+  unsigned long long s[4] = {0, 0, 0, 0};
+  for (uint32_t hb = blockIdx.x * blockDim.x + threadIdx.x; hb < m; hb += gridDim.x * blockDim.x) {
+    const uint32_t asz = bstart[hb + 1] - bstart[hb];
+    const HomeSplit h = home_split(P, hb, asz);
+    const uint32_t sg = seg[h.tc ? 1 : 0];
+    const unsigned long long nu = (unsigned long long)h.nch_s * (((unsigned long long)npts[hb] + sg - 1) / sg);
+    // a bin's unit count saturates at 2^32 - 1; the 64-bit totals then exceed
+    // the 32-bit offsets the work lists use, and the call fails with
+    // MISTIC_ERR_TOO_LARGE
+    const uint32_t nu32 = nu > 0xffffffffull ? 0xffffffffu : (uint32_t)nu;
+    unit_cnt[hb] = h.tc ? 0u : nu32;
+    unit_cnt_tc[hb] = h.tc ? nu32 : 0u;
+    s[0] += h.self_s + h.rows_s * (npts[hb] - asz);
+    s[1] += nbr_cnt[hb];
+    s[2] += h.tc ? 0u : nu32;
+    s[3] += h.tc ? nu32 : 0u;
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) s[k] += __shfl_xor_sync(FULL_MASK, s[k], o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    if (s[0]) atomicAdd(&tot->cand, s[0]);
+    for (int k = 0; k < 3; ++k)
+      if (s[k + 1]) atomicAdd(&tot->n[k], s[k + 1]);
   }
 }
 
@@ -579,26 +751,6 @@ __global__ void k_prefix_count(const uint64_t* __restrict__ bkey, uint32_t m, En
     v += (uint32_t)((K >> P.shift[j]) & ((1ull << w) - 1ull)) * P.stride[j];
   }
   atomicAdd(&cnt[v], 1u);
-}
-
-// 64-bit sums of the three per-bin count arrays of the enumeration (the
-// scans that turn them into offsets are 32-bit).
-__global__ void k_count_totals(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b,
-                               const uint32_t* __restrict__ c, uint32_t m, unsigned long long* __restrict__ tot) {
-  unsigned long long s[3] = {0, 0, 0};
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
-    s[0] += a[i];
-    s[1] += b[i];
-    s[2] += c[i];
-  }
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-#pragma unroll
-    for (int o = 16; o; o >>= 1) s[k] += __shfl_xor_sync(FULL_MASK, s[k], o);
-  }
-  if ((threadIdx.x & 31) == 0)
-    for (int k = 0; k < 3; ++k)
-      if (s[k]) atomicAdd(&tot[k], s[k]);
 }
 
 // ------------------------------------------------------------ host launchers
@@ -692,18 +844,41 @@ void prefix_table(mistic_handle_s* h, const uint64_t* bkey, uint32_t m, const En
   exclusive_scan<uint32_t>(h, ptab, ptab, (size_t)entries + 1, nullptr);
 }
 
-void enumerate(mistic_handle_s* h, const uint64_t* bkey, const uint32_t* bstart, uint32_t m,
-               const EnumParams& P, uint32_t* nbr_cnt, uint32_t* unit_cnt, uint32_t* unit_cnt_tc,
-               unsigned long long* cand, const uint32_t* nbr_off, const uint32_t* unit_off,
-               const uint32_t* unit_off_tc, uint32_t* nbr, Unit* units, Unit* units_tc, bool fill) {
-  const unsigned nb = (m + 127) / 128;
-  if (!fill)
-    k_enum<false><<<nb, 128, 0, h->stream>>>(bkey, bstart, m, P, nbr_cnt, unit_cnt, unit_cnt_tc, cand, nullptr,
-                                             nullptr, nullptr, nullptr, nullptr, nullptr);
+// A warp per bin reads every key whose field 0 lies near (m^2 work); a thread
+// per bin takes up to 3^k dependent steps whatever m is.  Both passes and the
+// scans, ms, warp / thread per bin: k = 2: 7,131 bins 0.060 / 0.091, 21,565
+// 0.100 / 0.097; k = 3: 87,584 bins 1.20 / 0.19; k = 6: 11,483 bins 0.30 /
+// 0.89, 28,343 1.04 / 0.93, 46,583 2.20 / 1.01; k = 8: 5,593 bins 0.23 / 5.68.
+bool enum_flat(uint32_t m, const EnumParams& P) { return m <= 4096u * (uint32_t)std::min(std::max(P.k, 1), 6); }
+
+void enum_count(mistic_handle_s* h, const uint64_t* bkey, const uint32_t* bstart, uint32_t m, const EnumParams& P,
+                uint32_t* npts, uint32_t* nbr_cnt, uint32_t* unit_cnt, uint32_t* unit_cnt_tc, EnumTotals* tot) {
+  MCK(cudaMemsetAsync(tot, 0, sizeof(EnumTotals), h->stream));
+  if (enum_flat(m, P))
+    k_enum_flat<false><<<(m + FLAT_WARPS - 1) / FLAT_WARPS, FLAT_WARPS * 32, 0, h->stream>>>(
+        bkey, bstart, m, P, npts, nbr_cnt, tot, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
   else
-    k_enum<true><<<nb, 128, 0, h->stream>>>(bkey, bstart, m, P, nullptr, nullptr, nullptr, nullptr, nbr_off,
-                                            unit_off, unit_off_tc, nbr, units, units_tc);
-  launched(h, fill ? "enum_fill" : "enum_count");
+    k_enum<false><<<(m + 127) / 128, 128, 0, h->stream>>>(bkey, bstart, m, P, npts, nbr_cnt, tot, nullptr, nullptr,
+                                                          nullptr, nullptr, nullptr, nullptr);
+  launched(h, "enum_count");
+  const unsigned nb = std::max(1u, std::min((m + 255) / 256, 4u * (unsigned)h->sms));
+  k_unit_plan<<<nb, 256, 0, h->stream>>>(bstart, m, P, npts, nbr_cnt, unit_cnt, unit_cnt_tc, tot);
+  launched(h, "unit_plan");
+  exclusive_scan3(h, nbr_cnt, unit_cnt, unit_cnt_tc, m);
+}
+
+void enum_fill(mistic_handle_s* h, const uint64_t* bkey, const uint32_t* bstart, uint32_t m, const EnumParams& P,
+               const uint32_t* npts, const uint32_t* nbr_off, const uint32_t* unit_off, const uint32_t* unit_off_tc,
+               const EnumTotals* tot, uint32_t* nbr, Unit* units, Unit* units_tc) {
+  uint32_t* np = const_cast<uint32_t*>(npts);
+  EnumTotals* t = const_cast<EnumTotals*>(tot);
+  if (enum_flat(m, P))
+    k_enum_flat<true><<<(m + FLAT_WARPS - 1) / FLAT_WARPS, FLAT_WARPS * 32, 0, h->stream>>>(
+        bkey, bstart, m, P, np, nullptr, t, nbr_off, unit_off, unit_off_tc, nbr, units, units_tc);
+  else
+    k_enum<true><<<(m + 127) / 128, 128, 0, h->stream>>>(bkey, bstart, m, P, np, nullptr, t, nbr_off, unit_off,
+                                                         unit_off_tc, nbr, units, units_tc);
+  launched(h, "enum_fill");
 }
 
 // Points per log2 bin-size class: hist[c] += size of every bin with
@@ -725,14 +900,6 @@ void bin_hist(mistic_handle_s* h, const uint32_t* bstart, uint32_t m, unsigned l
   const unsigned nb = std::max(1u, std::min((m + 255) / 256, 4u * (unsigned)h->sms));
   k_bin_hist<<<nb, 256, 0, h->stream>>>(bstart, m, hist);
   launched(h, "bin_hist");
-}
-
-void count_totals(mistic_handle_s* h, const uint32_t* nbr_cnt, const uint32_t* unit_cnt, const uint32_t* unit_cnt_tc,
-                  uint32_t m, unsigned long long* tot) {
-  MCK(cudaMemsetAsync(tot, 0, 3 * sizeof(unsigned long long), h->stream));
-  const unsigned nb = std::max(1u, std::min((m + 255) / 256, 4u * (unsigned)h->sms));
-  k_count_totals<<<nb, 256, 0, h->stream>>>(nbr_cnt, unit_cnt, unit_cnt_tc, m, tot);
-  launched(h, "count_totals");
 }
 
 }  // namespace idx

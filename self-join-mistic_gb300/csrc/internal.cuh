@@ -61,14 +61,30 @@ struct KeyLayout {
   uint32_t maxkey[MAX_K]; // largest stored field value (after subtraction)
 };
 
-// One join work unit: a chunk of up to `CH` points of home bin `h` against
-// the neighbour bins nbr[s0 .. s1) (all of index >= h).
+// One join work unit: a chunk of up to `CH` points of home bin `h` against a
+// run of its neighbour bins' points (bins of index >= h): the bins
+// nbr[s0 .. s1), the first from its point o0 on, the last up to its point o1
+// (exclusive).  A bin of many points is cut across units, so no unit holds
+// more candidates than its segment length whatever the bin sizes.
 struct Unit {
   uint32_t h;
   uint32_t chunk;
   uint32_t s0;
   uint32_t s1;
+  uint32_t o0;
+  uint32_t o1;
 };
+
+// Points [first, first + size) of neighbour entry `e` (an index into nbr) as
+// one unit sees them.
+__device__ __forceinline__ void unit_bin(const Unit& U, const uint32_t* nbr, const uint32_t* bstart, uint32_t e,
+                                         uint32_t* bin, uint32_t* first, uint32_t* size) {
+  const uint32_t b = nbr[e], st = bstart[b];
+  const uint32_t lo = e == U.s0 ? U.o0 : 0u, hi = e + 1 == U.s1 ? U.o1 : bstart[b + 1] - st;
+  *bin = b;
+  *first = st + lo;
+  *size = hi - lo;
+}
 
 // Counters the join kernels accumulate on the device.
 struct JoinCounters {
@@ -102,8 +118,10 @@ struct EnumParams {
   int k;
   int shift[MAX_K];
   uint32_t maxkey[MAX_K];
-  uint32_t seg_cap;     // candidate points per neighbour segment (CUDA-core units)
-  uint32_t seg_cap_tc;  // the same for tensor-core units
+  // candidate points per neighbour segment: the longest segment, the shortest,
+  // and the number of units that small joins shorten their segments for (0:
+  // always the longest), for CUDA-core [0] and tensor-core [1] units
+  uint32_t seg_max[2], seg_min[2], want_units[2];
   uint32_t chunk;    // home points per CUDA-core unit
   uint32_t tc_min;   // home bins with at least this many points get tensor-core units (0: none)
   uint32_t tc_chunk; // home points per tensor-core unit
@@ -277,6 +295,8 @@ void allow_max_dyn_smem(K kern) {
 // ---- scan.cu
 template <class T>
 void exclusive_scan(mistic_handle_s* h, const T* in, T* out, size_t n, T* total_dev);
+// In place, over three arrays of n elements at once.
+void exclusive_scan3(mistic_handle_s* h, uint32_t* a, uint32_t* b, uint32_t* c, size_t n);
 size_t scan_partials_count(size_t n);
 
 // ---- sort.cu: LSD radix sort of 64-bit keys over the low `bits` bits with
@@ -304,15 +324,26 @@ void gather(mistic_handle_s*, const void* x, mistic_dtype, size_t n, uint32_t d,
 // values into ptab
 void prefix_table(mistic_handle_s*, const uint64_t* bkey, uint32_t m, const EnumParams&, uint32_t* ptab,
                   uint32_t entries);
-void enumerate(mistic_handle_s*, const uint64_t* bkey, const uint32_t* bstart, uint32_t m,
-               const EnumParams&, uint32_t* nbr_cnt, uint32_t* unit_cnt, uint32_t* unit_cnt_tc,
-               unsigned long long* cand, const uint32_t* nbr_off, const uint32_t* unit_off,
-               const uint32_t* unit_off_tc, uint32_t* nbr, Unit* units, Unit* units_tc, bool fill);
+// Whether m bins are enumerated by a warp per bin over the sorted keys (no
+// prefix table) rather than by a thread per bin.
+bool enum_flat(uint32_t m, const EnumParams&);
+// Neighbour enumeration, first half: neighbours and units per home bin, as
+// exclusive prefix sums in nbr_cnt, unit_cnt and unit_cnt_tc, and the totals
+// (see EnumTotals); npts is scratch of m entries.
+struct EnumTotals {
+  unsigned long long cand;      // candidate pairs
+  unsigned long long n[3];      // neighbour bins, CUDA-core units, tensor-core units
+  unsigned long long work[2];   // sum over home chunks of their candidate points, by unit class
+  uint32_t seg[2];              // segment lengths chosen
+};
+void enum_count(mistic_handle_s*, const uint64_t* bkey, const uint32_t* bstart, uint32_t m, const EnumParams&,
+                uint32_t* npts, uint32_t* nbr_cnt, uint32_t* unit_cnt, uint32_t* unit_cnt_tc, EnumTotals* tot);
+// Second half: the neighbour list and the units.
+void enum_fill(mistic_handle_s*, const uint64_t* bkey, const uint32_t* bstart, uint32_t m, const EnumParams&,
+               const uint32_t* npts, const uint32_t* nbr_off, const uint32_t* unit_off, const uint32_t* unit_off_tc,
+               const EnumTotals* tot, uint32_t* nbr, Unit* units, Unit* units_tc);
 // points per log2 bin-size class (32 classes) into hist
 void bin_hist(mistic_handle_s*, const uint32_t* bstart, uint32_t m, unsigned long long* hist);
-// 64-bit totals of the enumeration's three per-bin count arrays into tot[3]
-void count_totals(mistic_handle_s*, const uint32_t* nbr_cnt, const uint32_t* unit_cnt, const uint32_t* unit_cnt_tc,
-                  uint32_t m, unsigned long long* tot);
 }  // namespace idx
 
 // ---- mistic.cu: FP32 filter thresholds (accept at or below t_lo, re-decide

@@ -205,10 +205,11 @@ __device__ __forceinline__ uint32_t home_mask(uint32_t na, bool self, uint32_t q
   return CH >= 32 ? m : (m & ((1u << CH) - 1u));
 }
 
-// Candidate stream of one unit: the points of the neighbour bins
-// nbr[s .. s1) in order, 32 per tile, lanes filled across bin boundaries
+// Candidate stream of one unit: the points of its neighbour bins from entry s
+// on in order, 32 per tile, lanes filled across bin boundaries
 // (bins average a few points, so one bin per tile would leave most lanes
-// idle).  `s` and `off` (next bin, offset inside it) are warp-uniform.
+// idle).  `s` and `off` (next bin, offset inside the unit's part of it) are
+// warp-uniform.
 // Each lane gets its candidate's sorted position q, or qv = false past the
 // end.  Lane l finds its bin by a binary search over the warp's inclusive
 // scan of up to 32 bin sizes.
@@ -217,15 +218,14 @@ struct CandTile {
   bool qv;
 };
 
-__device__ __forceinline__ CandTile next_tile(const uint32_t* nbr, const uint32_t* bstart, uint32_t& s, uint32_t& off,
-                                              uint32_t s1) {
+__device__ __forceinline__ CandTile next_tile(const Unit& U, const uint32_t* nbr, const uint32_t* bstart, uint32_t& s,
+                                              uint32_t& off) {
   const int lane = threadIdx.x & 31;
-  const uint32_t bj = s + lane;
+  const uint32_t bj = s + lane, s1 = U.s1;
   uint32_t start = 0, size = 0;
   if (bj < s1) {
-    const uint32_t b = nbr[bj];
-    start = bstart[b];
-    size = bstart[b + 1] - start;
+    uint32_t b;
+    unit_bin(U, nbr, bstart, bj, &b, &start, &size);
     if (lane == 0) {
       start += off;
       size -= off;
@@ -330,7 +330,7 @@ k_join_f32(const JoinParams P) {
     __syncwarp();
     uint32_t s = U.s0, off = 0;
     while (s < U.s1) {
-      const CandTile t = next_tile(V.nbr, V.bstart, s, off, U.s1);
+      const CandTile t = next_tile(U, V.nbr, V.bstart, s, off);
       const uint32_t q = t.q;
       const float4* qrow = X + (size_t)(t.qv ? q : a0) * nq4;
       float acc[CH];
@@ -397,7 +397,7 @@ k_join_f32r(const JoinParams P) {
     __syncwarp();
     uint32_t s = U.s0, off = 0;
     while (s < U.s1) {
-      const CandTile t = next_tile(V.nbr, V.bstart, s, off, U.s1);
+      const CandTile t = next_tile(U, V.nbr, V.bstart, s, off);
       const uint32_t q = t.q;
       const ulonglong2* qrow = reinterpret_cast<const ulonglong2*>(X + (size_t)(t.qv ? q : a0) * DQ);
       ulonglong2 qq[DQ];  // the candidate row as pairs of floats
@@ -526,7 +526,7 @@ k_join_f64(const JoinParams P) {
     __syncwarp();
     uint32_t s = U.s0, off = 0;
     while (s < U.s1) {
-      const CandTile t = next_tile(V.nbr, V.bstart, s, off, U.s1);
+      const CandTile t = next_tile(U, V.nbr, V.bstart, s, off);
       const uint32_t q = t.q;
       const double2* qrow = X + (size_t)(t.qv ? q : a0) * nq2;
       double acc[CH];

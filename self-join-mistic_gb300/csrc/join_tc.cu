@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
           if (max(hr0, pos) < min(hr1, pos + ncols)) {
             const uint32_t lo = max(hr0, pos) - pos, hi = min(hr1, pos + ncols) - pos;
             *hcr = lo | (hi << 8);
-            *hq = hs + (pos + lo - hr0);
+            *hq = S.w_start[w_hj] + (pos + lo - hr0);
           }
         }
       };
@@ -462,11 +462,7 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
           const long long cw0 = T.prof ? clock64() : 0;
           const uint32_t nb = min((uint32_t)WIN, U.s1 - seg_next);
           uint32_t st0 = 0, sz0 = 0, bn = 0xffffffffu;
-          if ((uint32_t)tid < nb) {
-            bn = nbr[seg_next + tid];
-            st0 = bstart[bn];
-            sz0 = bstart[bn + 1] - st0;
-          }
+          if ((uint32_t)tid < nb) unit_bin(U, nbr, bstart, seg_next + tid, &bn, &st0, &sz0);
           const uint32_t incl = warp_scan_incl(sz0);
           if (lane == 31) S.scan_ws[warp] = incl;
           prod_sync();
@@ -780,11 +776,7 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
           const long long cw0 = T.prof ? clock64() : 0;
           const uint32_t nb = min((uint32_t)WIN, U.s1 - seg_next);
           uint32_t st0 = 0, sz0 = 0, bn = 0xffffffffu;
-          if ((uint32_t)tid < nb) {
-            bn = nbr[seg_next + tid];
-            st0 = bstart[bn];
-            sz0 = bstart[bn + 1] - st0;
-          }
+          if ((uint32_t)tid < nb) unit_bin(U, nbr, bstart, seg_next + tid, &bn, &st0, &sz0);
           const uint32_t incl = warp_scan_incl(sz0);
           if (lane == 31) S.scan_ws[warp] = incl;
           prod_sync();
@@ -869,7 +861,7 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
             const uint32_t lo = max(hr0, w_pos) - w_pos, hi = min(hr1, w_pos + ncols) - w_pos;
             if (max(hr0, w_pos) < min(hr1, w_pos + ncols)) {
               hcr = lo | (hi << 8);
-              hq = hs + (w_pos + lo - hr0);
+              hq = S.w_start[w_hj] + (w_pos + lo - hr0);
             }
           }
           S.hx[issued & 3][0] = hcr;

@@ -592,7 +592,7 @@ bool tune_lookup(mistic_handle_s* h, const mistic_opts& o, uint32_t d, mistic_dt
   }
   const int eps_cls = (eps2 > 0 && R > 0) ? (int)std::floor(std::log2(R * R / eps2)) : 0;
   char key[160];
-  snprintf(key, sizeof key, "v4 d=%u dt=%d %s bins=%d,%d r2e=%d", d, (int)dt, wide ? "tcw" : "tc", c50, c90, eps_cls);
+  snprintf(key, sizeof key, "v4 d=%u dt=%d %s bins=%d,%d r2e=%d s2", d, (int)dt, wide ? "tcw" : "tc", c50, c90, eps_cls);
   if (tune_cache().find(key, out)) return true;
   // candidates
   std::vector<TuneCandidate> cands;
@@ -963,20 +963,29 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
   // ---- neighbour enumeration -> work units
   const int CH = join::chunk_for(fp64, fp64 ? dpad64 : dpad32);
   ep.chunk = (uint32_t)CH;
-  ep.seg_cap = 4096;
+  ep.seg_max[0] = 4096;
   // tensor-core units of large joins take longer segments: each unit reloads
   // and converts its home rows and drains the tile pipeline once, which cost
   // 4 ms of the 5M x 18 join at 4096 points against 16384; small joins keep
   // short segments so that the persistent grid has units enough to balance,
   // and the pair ring keeps them so that a unit's pairs fit it
-  ep.seg_cap_tc = (n >= (1u << 20) && o.ring_capacity == 0) ? 16384u : 4096u;
-  if (const char* e = getenv("MISTIC_SEG_CAP_TC")) ep.seg_cap_tc = (uint32_t)std::max(128l, strtol(e, nullptr, 10));
+  ep.seg_max[1] = (n >= (1u << 20) && o.ring_capacity == 0) ? 16384u : 4096u;
+  if (const char* e = getenv("MISTIC_SEG_CAP_TC")) ep.seg_max[1] = (uint32_t)std::max(128l, strtol(e, nullptr, 10));
+  if (o.ring_capacity == 0) {
+    // units enough for a few a resident worker (32 warps, or one tensor-core
+    // CTA, an SM); a segment still covers several tiles of 32 or 128 columns
+    ep.seg_min[0] = 256;
+    ep.seg_min[1] = 512;
+    // (an instance of a fused batch shares the grid with the others)
+    ep.want_units[0] = (ex ? 16u : 128u) * (uint32_t)h->sms;
+    ep.want_units[1] = (ex ? 1u : 6u) * (uint32_t)h->sms;
+  }
   ep.sample = o.home_sample;
   ep.tc_min = use_tc ? tc_min_bin(d, wide) : 0u;
   ep.tc_chunk = use_tc ? (wide ? 256u : join::tc_rows(d)) : 128;
   // prefix table of the enumeration: the first p <= 5 key fields (3^p
   // lookups a bin) while the table stays within 16 entries a bin and 2^24
-  {
+  if (!idx::enum_flat(m, ep)) {
     const unsigned long long lim = std::min<unsigned long long>(1ull << 24, 16ull * m + 4096);
     unsigned long long entries = 1;
     int p = 0;
@@ -1001,38 +1010,31 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
   Unit* units_tc = nullptr;
   // count -> 64-bit totals check -> scans -> fill, into the arena's work lists
   auto enumerate_units = [&](const EnumParams& e) {
+    uint32_t* npts = abuf<uint32_t>(h, "nbr_pts", m + 1);
     uint32_t* nbr_cnt = abuf<uint32_t>(h, "nbr_cnt", m + 1);
     uint32_t* unit_cnt = abuf<uint32_t>(h, "unit_cnt", m + 1);
     uint32_t* unit_cnt_tc = abuf<uint32_t>(h, "unit_cnt_tc", m + 1);
-    unsigned long long* cand = abuf<unsigned long long>(h, "cand", m + 1);
-    idx::enumerate(h, bkey, bstart, m, e, nbr_cnt, unit_cnt, unit_cnt_tc, cand, nullptr, nullptr, nullptr, nullptr,
-                   nullptr, nullptr, false);
-    uint32_t* tot32 = abuf<uint32_t>(h, "tot32", 3);
-    unsigned long long* tot64 = abuf<unsigned long long>(h, "tot64", 4);
+    idx::EnumTotals* tot_dev = abuf<idx::EnumTotals>(h, "enum_tot", 1);
+    idx::enum_count(h, bkey, bstart, m, e, npts, nbr_cnt, unit_cnt, unit_cnt_tc, tot_dev);
     // 64-bit totals first: the work lists index neighbours and units with
     // 32-bit offsets, which a total of 2^32 or more would wrap
-    idx::count_totals(h, nbr_cnt, unit_cnt, unit_cnt_tc, m, tot64 + 1);
-    exclusive_scan<uint32_t>(h, nbr_cnt, nbr_cnt, m, tot32);
-    exclusive_scan<uint32_t>(h, unit_cnt, unit_cnt, m, tot32 + 1);
-    exclusive_scan<uint32_t>(h, unit_cnt_tc, unit_cnt_tc, m, tot32 + 2);
-    exclusive_scan<unsigned long long>(h, cand, cand, m, tot64);
-    unsigned long long tot_all[4] = {0, 0, 0, 0};
-    d2h(h, tots, tot32, sizeof tots);
-    d2h(h, tot_all, tot64, sizeof tot_all);
-    totc = tot_all[0];
+    idx::EnumTotals ht{};
+    d2h(h, &ht, tot_dev, sizeof ht);
+    totc = ht.cand;
     // MISTIC_TEST_WORKLIST_LIMIT=k lowers the limit (tests of this check)
     unsigned long long lim = 0xffffffffull - 1;
     if (const char* ev = getenv("MISTIC_TEST_WORKLIST_LIMIT")) lim = std::min(lim, strtoull(ev, nullptr, 10));
-    for (int i = 0; i < 3; ++i)
-      if (tot_all[1 + i] > lim || tot_all[1 + i] != (unsigned long long)tots[i])
+    for (int i = 0; i < 3; ++i) {
+      if (ht.n[i] > lim)
         throw Error(MISTIC_ERR_TOO_LARGE,
                     "neighbour-bin or work-unit list beyond the 32-bit offsets of the join work lists "
                     "(raise eps resolution: more reference points, or split the input)");
+      tots[i] = (uint32_t)ht.n[i];
+    }
     nbr = abuf<uint32_t>(h, "nbr", (size_t)tots[0] + 1);
     units = abuf<Unit>(h, "units", (size_t)tots[1] + 1);
     units_tc = abuf<Unit>(h, "units_tc", (size_t)tots[2] + 1);
-    idx::enumerate(h, bkey, bstart, m, e, nullptr, nullptr, nullptr, nullptr, nbr_cnt, unit_cnt, unit_cnt_tc, nbr,
-                   units, units_tc, true);
+    idx::enum_fill(h, bkey, bstart, m, e, npts, nbr_cnt, unit_cnt, unit_cnt_tc, tot_dev, nbr, units, units_tc);
   };
 
   // ---- join parameters
