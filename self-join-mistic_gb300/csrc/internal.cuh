@@ -299,11 +299,20 @@ void exclusive_scan(mistic_handle_s* h, const T* in, T* out, size_t n, T* total_
 void exclusive_scan3(mistic_handle_s* h, uint32_t* a, uint32_t* b, uint32_t* c, size_t n);
 size_t scan_partials_count(size_t n);
 
-// ---- sort.cu: LSD radix sort of 64-bit keys over the low `bits` bits with
-// an optional 32-bit payload.  If vals_in is null the payload is the input
-// position.  Returns which buffer (0/1) holds the result.
-int radix_sort_u64(mistic_handle_s* h, uint64_t* keys[2], uint32_t* vals[2],
-                   bool has_vals, bool iota_vals, size_t n, int bits);
+// ---- sort.cu: LSD radix sort of 64-bit keys over the low `bits` bits; the
+// 32-bit payload vals is each key's input position.  Returns which buffer
+// (0/1) holds the result.
+int radix_sort_u64(mistic_handle_s* h, uint64_t* keys[2], uint32_t* vals[2], size_t n, int bits);
+
+// ---- rows.cu: np packed pairs (i << 32 | j, i < j < n), sorted by (i, j) in
+// place and stored in memory order (i, j); in a fused batch (row0 of n_inst
+// instances) with ids relative to their instance.
+void sort_pairs_ij(mistic_handle_s* h, unsigned long long* pairs, size_t np, size_t n, const uint32_t* row0,
+                   uint32_t n_inst);
+// The neighbour table of the pairs: 2 np + n ids, ascending within each row
+// (its own id included), and n + 1 row offsets.
+void neighbour_table(mistic_handle_s* h, const unsigned long long* pairs, size_t np, size_t n, uint32_t* nbrs,
+                     unsigned long long* offs);
 
 // ---- index.cu
 namespace idx {

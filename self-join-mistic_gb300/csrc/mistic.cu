@@ -38,9 +38,6 @@
 namespace mistic {
 
 void pairs_to_ij(mistic_handle_s* h, unsigned long long* p, size_t n);
-void csr_edges(mistic_handle_s* h, const unsigned long long* pairs, size_t np, size_t n, unsigned long long* e);
-void csr_split(mistic_handle_s* h, const unsigned long long* e, size_t E, uint32_t* nbrs, unsigned long long* offs,
-               size_t n);
 
 // ------------------------------------------------------------------ plumbing
 
@@ -896,7 +893,7 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
   // ---- sort points by key
   int cur = 0;
   if (total_bits > 0) {
-    cur = radix_sort_u64(h, keys, vals, true, true, n, total_bits);
+    cur = radix_sort_u64(h, keys, vals, n, total_bits);
   } else {
     idx::iota(h, vals[0], n);
   }
@@ -1568,13 +1565,9 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
     if (hc.pairs > cap) tail = MISTIC_ERR_PAIR_OVERFLOW;
     const unsigned long long E = 2 * np + n;
     if (E >= 0xffffffffull) throw Error(MISTIC_ERR_TOO_LARGE, "neighbour table beyond 2^32 entries");
-    uint64_t* ek[2] = {abuf<uint64_t>(h, "csr_e0", E), abuf<uint64_t>(h, "csr_e1", E)};
-    csr_edges(h, pbuf, np, n, (unsigned long long*)ek[0]);
-    uint32_t* ev[2] = {nullptr, nullptr};
-    const int c = radix_sort_u64(h, ek, ev, false, false, E, 32 + std::max(1, bit_length(n - 1)));
     uint64_t* offs = abuf<uint64_t>(h, "csr_off", n + 1);
     uint32_t* nbs = abuf<uint32_t>(h, "csr_nbr", E);
-    csr_split(h, (const unsigned long long*)ek[c], E, nbs, (unsigned long long*)offs, n);
+    neighbour_table(h, pbuf, np, n, nbs, (unsigned long long*)offs);
     if (o.csr == MISTIC_PAIRS_HOST) {
       r->csr_offsets = (uint64_t*)malloc((n + 1) * sizeof(uint64_t));
       r->csr_nbrs = (uint32_t*)malloc(std::max<size_t>(1, E * sizeof(uint32_t)));
@@ -1603,14 +1596,10 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
   } else if (want_pairs) {
     const unsigned long long stored = std::min<unsigned long long>(hc.pairs, cap);
     if (hc.pairs > cap) tail = MISTIC_ERR_PAIR_OVERFLOW;
-    if (o.sort_pairs && stored > 1) {
-      uint64_t* pk[2] = {(uint64_t*)pbuf, abuf<uint64_t>(h, "pairs_tmp", stored)};
-      uint32_t* pv[2] = {nullptr, nullptr};
-      const int bits = bit_length(n - 1);
-      int c = radix_sort_u64(h, pk, pv, false, false, stored, 32 + bits);
-      if (c == 1) MCK(cudaMemcpyAsync(pbuf, pk[1], stored * 8, cudaMemcpyDeviceToDevice, h->stream));
-    }
-    pairs_to_ij(h, pbuf, stored);
+    if (o.sort_pairs && stored > 1)
+      sort_pairs_ij(h, pbuf, stored, n, nullptr, 0);
+    else
+      pairs_to_ij(h, pbuf, stored);
     r->pairs_len = stored;
     if (o.pairs == MISTIC_PAIRS_HOST) {
       uint32_t* hp = (uint32_t*)pinned_cache().acquire(std::max<size_t>(1, stored * 8));
@@ -1669,23 +1658,6 @@ __global__ void k_unit_inst(const unsigned long long* __restrict__ off, uint32_t
     if (off[mid] <= t) lo = mid; else hi = mid - 1;
   }
   unit_inst[t] = gidx[lo];
-}
-
-// Sorted packed pairs of global row ids -> local ids of their instance
-// (row0 of the instance subtracted from both halves) in memory order (i, j).
-__global__ void k_localize(unsigned long long* __restrict__ p, size_t np, const uint32_t* __restrict__ row0,
-                           uint32_t n_inst) {
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= np) return;
-  const unsigned long long v = p[t];
-  const uint32_t gi = (uint32_t)(v >> 32), gj = (uint32_t)v;
-  uint32_t lo = 0, hi = n_inst - 1;
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi + 1) >> 1;
-    if (row0[mid] <= gi) lo = mid; else hi = mid - 1;
-  }
-  const uint32_t r0 = row0[lo];
-  p[t] = ((unsigned long long)(gj - r0) << 32) | (gi - r0);
 }
 
 // All instances of a batch in one pass of the join kernels.  Phase one
@@ -2005,14 +1977,10 @@ mistic_status run_batch_fused(mistic_handle h, const mistic_instance* inst, uint
   // ---- per-instance results
   std::vector<unsigned long long> pstart(G + 1, 0);
   if (want_pairs && hc.pairs) {
-    uint64_t* pk[2] = {(uint64_t*)pbuf, abuf<uint64_t>(h, "b_pairs_tmp", hc.pairs)};
-    uint32_t* pv[2] = {nullptr, nullptr};
-    const int c = radix_sort_u64(h, pk, pv, false, false, hc.pairs, 32 + bit_length(tot_n ? row0.back() + inst[m - 1].n : 1));
-    unsigned long long* sorted = (unsigned long long*)pk[c];
+    const unsigned long long* sorted = pbuf;
     for (uint32_t g = 0; g < G; ++g) pstart[g + 1] = pstart[g] + ipairs[g];
     if (pstart[G] != hc.pairs) throw Error(MISTIC_ERR_INTERNAL, "per-instance pair counts do not add up");
-    k_localize<<<(unsigned)((hc.pairs + 255) / 256), 256, 0, h->stream>>>(sorted, hc.pairs, d_row0, G);
-    launched(h, "localize");
+    sort_pairs_ij(h, pbuf, hc.pairs, (size_t)row0.back() + inst[m - 1].n, d_row0, G);
     for (uint32_t g = 0; g < G; ++g) {
       mistic_result& r = results[gl[g]];
       const unsigned long long np = ipairs[g];
@@ -2053,46 +2021,6 @@ mistic_status run_batch_fused(mistic_handle h, const mistic_instance* inst, uint
 }
 
 }  // namespace
-
-// Directed edges of the neighbour table: both orientations of every pair
-// plus every point's self edge, packed (src << 32 | dst).
-__global__ void k_csr_edges(const unsigned long long* __restrict__ pairs, size_t np, size_t n,
-                            unsigned long long* __restrict__ e) {
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < np) {
-    const unsigned long long v = pairs[t];
-    e[2 * t] = v;
-    e[2 * t + 1] = (v << 32) | (v >> 32);
-  } else if (t < np + n) {
-    const unsigned long long p = t - np;
-    e[2 * np + p] = (p << 32) | p;
-  }
-}
-
-// Sorted edges -> neighbour ids and row offsets (every row has its self edge,
-// so every row starts somewhere).
-__global__ void k_csr_split(const unsigned long long* __restrict__ e, size_t E, uint32_t* __restrict__ nbrs,
-                            unsigned long long* __restrict__ offs, size_t n) {
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= E) return;
-  const unsigned long long v = e[t];
-  nbrs[t] = (uint32_t)v;
-  const unsigned long long src = v >> 32;
-  if (t == 0 || (e[t - 1] >> 32) != src) offs[src] = t;
-  if (t == 0) offs[n] = E;
-}
-
-void csr_edges(mistic_handle_s* h, const unsigned long long* pairs, size_t np, size_t n, unsigned long long* e) {
-  const size_t tot = np + n;
-  k_csr_edges<<<(unsigned)((tot + 255) / 256), 256, 0, h->stream>>>(pairs, np, n, e);
-  launched(h, "csr_edges");
-}
-
-void csr_split(mistic_handle_s* h, const unsigned long long* e, size_t E, uint32_t* nbrs, unsigned long long* offs,
-               size_t n) {
-  k_csr_split<<<(unsigned)((E + 255) / 256), 256, 0, h->stream>>>(e, E, nbrs, offs, n);
-  launched(h, "csr_split");
-}
 
 __global__ void k_pairs_to_ij(unsigned long long* p, size_t n) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;

@@ -1,10 +1,9 @@
 // Device exclusive scan and LSD radix sort of 64-bit bin keys.
 //
-// The reference sorts with thrust (host `thrust::omp` sorts of bin numbers in
-// src/nodes.cu:372,505 and device `sort_by_key` of result pairs in
-// src/launcher.cu:3468,3488).  Here the bin keys of all n points are sorted
-// once on the device: 8-bit digits, one histogram pass and one stable scatter
-// pass per digit, only over the bits the packed key actually uses.
+// The reference sorts bin numbers with thrust (host `thrust::omp` sorts,
+// src/nodes.cu:372,505).  Here the bin keys of all n points are sorted once on
+// the device: 8-bit digits, one histogram pass and one stable scatter pass per
+// digit, only over the bits the packed key actually uses.
 //
 // Scatter ranking: each warp owns a contiguous run of 512 elements and ranks
 // them 32 at a time with __match_any_sync, keeping per-warp digit counters in
@@ -212,7 +211,7 @@ __global__ void k_rs_hist(const uint64_t* __restrict__ keys, size_t n, int shift
   hist[(size_t)threadIdx.x * tiles + blockIdx.x] = cnt[threadIdx.x];
 }
 
-template <bool HAS_VALS, bool IOTA>
+template <bool IOTA>
 __global__ void __launch_bounds__(RS_THREADS)
 k_rs_scatter(const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin,
              uint64_t* __restrict__ kout, uint32_t* __restrict__ vout, size_t n,
@@ -231,7 +230,7 @@ k_rs_scatter(const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin,
     const size_t idx = base + r * 32 + lane;
     const bool valid = idx < n;
     key[r] = valid ? kin[idx] : 0ull;
-    if (HAS_VALS) val[r] = valid ? (IOTA ? (uint32_t)idx : vin[idx]) : 0u;
+    val[r] = valid ? (IOTA ? (uint32_t)idx : vin[idx]) : 0u;
     // out-of-range lanes get a private sentinel digit so they match nobody
     const uint32_t dg = valid ? (uint32_t)((key[r] >> shift) & 0xff) : (RS_BINS + lane);
     const unsigned peers = __match_any_sync(FULL_MASK, dg);
@@ -262,39 +261,32 @@ k_rs_scatter(const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin,
       const uint32_t dg = (uint32_t)((key[r] >> shift) & 0xff);
       const size_t pos = (size_t)offs[(size_t)dg * tiles + blockIdx.x] + wcnt[w][dg] + rank[r];
       kout[pos] = key[r];
-      if (HAS_VALS) vout[pos] = val[r];
+      vout[pos] = val[r];
     }
   }
 }
 
-int radix_sort_u64(mistic_handle_s* h, uint64_t* keys[2], uint32_t* vals[2], bool has_vals,
-                   bool iota_vals, size_t n, int bits) {
+int radix_sort_u64(mistic_handle_s* h, uint64_t* keys[2], uint32_t* vals[2], size_t n, int bits) {
   if (n <= 1 || bits <= 0) {
-    if (n == 1 && has_vals && iota_vals) MCK(cudaMemsetAsync(vals[0], 0, sizeof(uint32_t), h->stream));
+    if (n == 1) MCK(cudaMemsetAsync(vals[0], 0, sizeof(uint32_t), h->stream));
     return 0;
   }
   if (n > 0xffffffffull) throw Error(MISTIC_ERR_TOO_LARGE, "radix sort supports < 2^32 elements");
   const uint32_t tiles = (uint32_t)((n + RS_TILE - 1) / RS_TILE);
   uint32_t* hist = (uint32_t*)h->arena.get("rs_hist", (size_t)RS_BINS * tiles * sizeof(uint32_t));
   int cur = 0;
-  bool first = true;
   for (int shift = 0; shift < bits; shift += 8) {
     k_rs_hist<<<tiles, RS_THREADS, 0, h->stream>>>(keys[cur], n, shift, hist, tiles);
     launched(h, "rs_hist");
     exclusive_scan<uint32_t>(h, hist, hist, (size_t)RS_BINS * tiles, nullptr);
-    if (!has_vals) {
-      k_rs_scatter<false, false><<<tiles, RS_THREADS, 0, h->stream>>>(
-          keys[cur], nullptr, keys[cur ^ 1], nullptr, n, shift, hist, tiles);
-    } else if (first && iota_vals) {
-      k_rs_scatter<true, true><<<tiles, RS_THREADS, 0, h->stream>>>(
-          keys[cur], nullptr, keys[cur ^ 1], vals[cur ^ 1], n, shift, hist, tiles);
-    } else {
-      k_rs_scatter<true, false><<<tiles, RS_THREADS, 0, h->stream>>>(
-          keys[cur], vals[cur], keys[cur ^ 1], vals[cur ^ 1], n, shift, hist, tiles);
-    }
+    if (shift == 0)
+      k_rs_scatter<true><<<tiles, RS_THREADS, 0, h->stream>>>(keys[cur], nullptr, keys[cur ^ 1], vals[cur ^ 1], n,
+                                                              shift, hist, tiles);
+    else
+      k_rs_scatter<false><<<tiles, RS_THREADS, 0, h->stream>>>(keys[cur], vals[cur], keys[cur ^ 1], vals[cur ^ 1], n,
+                                                               shift, hist, tiles);
     launched(h, "rs_scatter");
     cur ^= 1;
-    first = false;
   }
   return cur;
 }
