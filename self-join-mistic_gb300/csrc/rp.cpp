@@ -42,27 +42,108 @@ struct SplitMix {
   }
 };
 
-// Modified Gram-Schmidt on the k columns of V (d x k, column-major).
-void orthonormalise(std::vector<double>& V, uint32_t d, uint32_t k, SplitMix& rng) {
+// Sum of a_i b_i in four independent chains (one chain is bound by the FMA
+// latency, not by its throughput).
+double dot(const double* a, const double* b, uint32_t d) {
+  double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
+  uint32_t i = 0;
+  for (; i + 4 <= d; i += 4) {
+    s0 += a[i] * b[i];
+    s1 += a[i + 1] * b[i + 1];
+    s2 += a[i + 2] * b[i + 2];
+    s3 += a[i + 3] * b[i + 3];
+  }
+  for (; i < d; ++i) s0 += a[i] * b[i];
+  return (s0 + s1) + (s2 + s3);
+}
+
+// Modified Gram-Schmidt on the k columns of V (d x k, column-major); returns
+// the sum of the columns' norms before they were scaled.
+double orthonormalise(std::vector<double>& V, uint32_t d, uint32_t k, SplitMix& rng, int passes) {
+  double sum = 0;
   for (uint32_t c = 0; c < k; ++c) {
     double* v = &V[(size_t)c * d];
-    for (int pass = 0; pass < 2; ++pass) {
+    for (int pass = 0; pass < passes; ++pass) {
       for (uint32_t p = 0; p < c; ++p) {
         const double* u = &V[(size_t)p * d];
-        double dot = 0;
-        for (uint32_t i = 0; i < d; ++i) dot += u[i] * v[i];
-        for (uint32_t i = 0; i < d; ++i) v[i] -= dot * u[i];
+        const double t = dot(u, v, d);
+        for (uint32_t i = 0; i < d; ++i) v[i] -= t * u[i];
       }
     }
-    double nrm = 0;
-    for (uint32_t i = 0; i < d; ++i) nrm += v[i] * v[i];
-    nrm = sqrt(nrm);
+    const double nrm = sqrt(dot(v, v, d));
     if (nrm < 1e-300) {  // degenerate direction: replace with a random one
       for (uint32_t i = 0; i < d; ++i) v[i] = rng.normal();
       --c;  // redo this column
       continue;
     }
+    sum += nrm;
     for (uint32_t i = 0; i < d; ++i) v[i] /= nrm;
+  }
+  return sum;
+}
+
+// W = cov V for the k columns of V (both d x k, column-major), eight columns
+// and two rows of cov at a time: 16 sums in registers per pass over a row.
+void cov_times(const std::vector<double>& cov, uint32_t d, uint32_t k, const std::vector<double>& V,
+               std::vector<double>& W, std::vector<double>& T) {
+  T.resize((size_t)d * 8);
+  for (uint32_t c0 = 0; c0 < k; c0 += 8) {
+    const uint32_t nc = std::min(8u, k - c0);
+    for (uint32_t b = 0; b < d; ++b)
+      for (uint32_t c = 0; c < 8; ++c) T[(size_t)b * 8 + c] = c < nc ? V[(size_t)(c0 + c) * d + b] : 0.0;
+    for (uint32_t a = 0; a < d; a += 2) {
+      const double* r0 = &cov[(size_t)a * d];
+      const double* r1 = a + 1 < d ? r0 + d : r0;
+      double s0[8] = {0, 0, 0, 0, 0, 0, 0, 0}, s1[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      const double* t = T.data();
+      for (uint32_t b = 0; b < d; ++b, t += 8) {
+        const double x0 = r0[b], x1 = r1[b];
+        for (int c = 0; c < 8; ++c) {
+          s0[c] += x0 * t[c];
+          s1[c] += x1 * t[c];
+        }
+      }
+      for (uint32_t c = 0; c < nc; ++c) {
+        W[(size_t)(c0 + c) * d + a] = s0[c];
+        if (a + 1 < d) W[(size_t)(c0 + c) * d + a + 1] = s1[c];
+      }
+    }
+  }
+}
+
+// Eigenvectors of the symmetric k x k matrix H (row-major, destroyed) by
+// cyclic Jacobi rotations (the textbook method), as the columns of Q.
+void jacobi(std::vector<double>& H, uint32_t k, std::vector<double>& Q) {
+  Q.assign((size_t)k * k, 0.0);
+  for (uint32_t i = 0; i < k; ++i) Q[(size_t)i * k + i] = 1.0;
+  for (int sweep = 0; sweep < 30; ++sweep) {
+    double off = 0, diag = 0;
+    for (uint32_t p = 0; p < k; ++p)
+      for (uint32_t q = 0; q < k; ++q) (p == q ? diag : off) += H[(size_t)p * k + q] * H[(size_t)p * k + q];
+    if (!(off > 1e-24 * diag)) break;
+    for (uint32_t p = 0; p < k; ++p)
+      for (uint32_t q = p + 1; q < k; ++q) {
+        const double hpq = H[(size_t)p * k + q];
+        if (hpq == 0.0) continue;
+        const double th = (H[(size_t)q * k + q] - H[(size_t)p * k + p]) / (2.0 * hpq);
+        const double t = (th >= 0 ? 1.0 : -1.0) / (fabs(th) + sqrt(th * th + 1.0));
+        const double c = 1.0 / sqrt(t * t + 1.0), s = t * c;
+        for (uint32_t i = 0; i < k; ++i) {
+          const double x = H[(size_t)i * k + p], y = H[(size_t)i * k + q];
+          H[(size_t)i * k + p] = c * x - s * y;
+          H[(size_t)i * k + q] = s * x + c * y;
+        }
+        for (uint32_t i = 0; i < k; ++i) {
+          const double x = H[(size_t)p * k + i], y = H[(size_t)q * k + i];
+          H[(size_t)p * k + i] = c * x - s * y;
+          H[(size_t)q * k + i] = s * x + c * y;
+        }
+        for (uint32_t i = 0; i < k; ++i) {
+          const double x = Q[(size_t)i * k + p], y = Q[(size_t)i * k + q];
+          Q[(size_t)i * k + p] = c * x - s * y;
+          Q[(size_t)i * k + q] = s * x + c * y;
+        }
+      }
   }
 }
 
@@ -87,38 +168,44 @@ void select_reference_points(const mistic_opts& o, uint32_t d, uint32_t k, const
       for (uint32_t i = 0; i < d; ++i) rps[(size_t)j * d + i] = mn[i] + (mx[i] - mn[i]) * rng.uniform();
     return;
   }
-  // PCA: orthogonal iteration for the top-kk eigenvectors of cov.
-  const uint32_t kk = std::min(k, d);
-  std::vector<double> V((size_t)kk * d), W((size_t)kk * d);
+  // PCA: orthogonal iteration on a few columns more than wanted until the
+  // variance they capture stands still, then the eigenvectors of cov within
+  // their span (Rayleigh-Ritz).  The spare columns take up the slow
+  // convergence between neighbouring eigenvalues, and the index's candidate
+  // count depends on the captured variance only.  Orthogonal iteration on the
+  // wanted columns alone, a fixed 200 (d <= 64) or 60 times with one long
+  // chain per sum, took 0.4 ms at d = 18, 2.2 ms at d = 57, 46 ms at d = 384.
+  const uint32_t kk = std::min(k, d), L = std::min((kk + 15) & ~7u, d);
+  std::vector<double> V((size_t)L * d), W((size_t)L * d), T;
   for (auto& v : V) v = rng.normal();
-  orthonormalise(V, d, kk, rng);
-  const int iters = d <= 64 ? 200 : 60;
-  for (int it = 0; it < iters; ++it) {
-    for (uint32_t c = 0; c < kk; ++c) {
-      const double* v = &V[(size_t)c * d];
-      double* wv = &W[(size_t)c * d];
-      for (uint32_t a = 0; a < d; ++a) {
-        const double* row = &cov[(size_t)a * d];
-        double s = 0;
-        for (uint32_t b = 0; b < d; ++b) s += row[b] * v[b];
-        wv[a] = s;
-      }
-    }
+  orthonormalise(V, d, L, rng, 1);
+  double var = 0;
+  for (int it = 0; it < 60; ++it) {
+    cov_times(cov, d, L, V, W, T);
     std::swap(V, W);
-    orthonormalise(V, d, kk, rng);
+    const double v2 = orthonormalise(V, d, L, rng, 1);
+    if (it >= 2 && fabs(v2 - var) <= 5e-3 * v2) break;
+    var = v2;
   }
-  // Order the converged directions by Rayleigh quotient (largest first).
-  std::vector<std::pair<double, uint32_t>> rq(kk);
-  for (uint32_t c = 0; c < kk; ++c) {
-    const double* v = &V[(size_t)c * d];
-    double s = 0;
-    for (uint32_t a = 0; a < d; ++a) {
-      double r = 0;
-      for (uint32_t b = 0; b < d; ++b) r += cov[(size_t)a * d + b] * v[b];
-      s += v[a] * r;
+  orthonormalise(V, d, L, rng, 1);
+  cov_times(cov, d, L, V, W, T);
+  std::vector<double> H((size_t)L * L), Q;
+  for (uint32_t p = 0; p < L; ++p)
+    for (uint32_t q = p; q < L; ++q)
+      H[(size_t)p * L + q] = H[(size_t)q * L + p] = dot(&V[(size_t)p * d], &W[(size_t)q * d], d);
+  jacobi(H, L, Q);
+  std::vector<std::pair<double, uint32_t>> rq(L);  // largest eigenvalue first
+  for (uint32_t c = 0; c < L; ++c) {
+    rq[c] = {-H[(size_t)c * L + c], c};
+    double* w = &W[(size_t)c * d];
+    std::fill(w, w + d, 0.0);
+    for (uint32_t p = 0; p < L; ++p) {
+      const double f = Q[(size_t)p * L + c];
+      const double* v = &V[(size_t)p * d];
+      for (uint32_t i = 0; i < d; ++i) w[i] += f * v[i];
     }
-    rq[c] = {-s, c};
   }
+  std::swap(V, W);
   std::sort(rq.begin(), rq.end());
   double diam = 0;
   for (uint32_t i = 0; i < d; ++i) diam += (mx[i] - mn[i]) * (mx[i] - mn[i]);
