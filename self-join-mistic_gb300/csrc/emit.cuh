@@ -1,4 +1,5 @@
-// Warp-level staging of result pairs, shared by the join kernels.
+// What the join kernels share: a unit's view of its neighbour bins, and the
+// warp-level staging of result pairs.
 //
 // A warp collects accepted pairs in a small shared-memory buffer and
 // reserves space in the global pair list once per flush (one atomicAdd per
@@ -11,6 +12,22 @@
 #include "internal.cuh"
 
 namespace mistic {
+
+// Points [first, first + size) of neighbour entry `e` (an index into nbr) as
+// one unit of home chunks of `ch` points sees them.  Of the home bin's own
+// points, those before the chunk are left out: their pairs with the chunk's
+// rows are taken by the chunks they are in.  Only a list's first entry can
+// come out empty (the home bin leads its list).
+__device__ __forceinline__ void unit_bin(const Unit& U, uint32_t ch, const uint32_t* nbr, const uint32_t* bstart,
+                                         uint32_t e, uint32_t* bin, uint32_t* first, uint32_t* size) {
+  const uint32_t b = nbr[e], st = bstart[b];
+  uint32_t lo = e == U.s0 ? U.o0 : 0u;
+  const uint32_t hi = e + 1 == U.s1 ? U.o1 : bstart[b + 1] - st;
+  if (b == U.h) lo = min(hi, max(lo, U.chunk * ch));
+  *bin = b;
+  *first = st + lo;
+  *size = hi - lo;
+}
 
 constexpr uint32_t PSTAGE = 64;
 constexpr uint32_t RING_INVALID = 0xffffffffu;  // tag of a ring entry that holds no pair

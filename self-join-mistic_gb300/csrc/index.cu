@@ -455,8 +455,8 @@ __device__ __forceinline__ void walk_levels(const uint64_t* __restrict__ bkey, u
 // The split of a home bin's work into units: home chunks of csz points (nch
 // of them, nch_s in the sample) against segments of `seg` candidate points.
 // Segment b covers the candidate ranks [b seg, (b + 1) seg) of the bin's
-// neighbour list, wherever the bin boundaries fall; unit b * nch_s + c is
-// segment b of the c-th sampled chunk.
+// neighbour list, wherever the bin boundaries fall; the units are ordered by
+// segment, then chunk.
 struct HomeSplit {
   bool tc;             // tensor-core units
   uint32_t csz, nch, nch_s;
@@ -487,33 +487,72 @@ __device__ __forceinline__ HomeSplit home_split(const EnumParams& P, uint32_t hb
   return s;
 }
 
-// Writes the units of segment b that end at (s1, o1) -- when b >= 0 -- and
-// the start (s0, o0) of those of segment b + 1, when there is one.  lane and
-// lanes: the threads that share the work.
-__device__ __forceinline__ void write_cut(Unit* __restrict__ units, const EnumParams& P, const HomeSplit& s,
-                                          uint32_t hb, int b, uint32_t nseg, uint32_t s1, uint32_t o1, uint32_t s0,
-                                          uint32_t o0, uint32_t lane, uint32_t lanes) {
-  for (uint32_t c = lane; c < s.nch; c += lanes) {
-    uint32_t r = c;  // rank of chunk c among the sampled ones
-    if (P.sample > 1) {
-      if (!group_sampled(hb, c * s.csz / SAMPLE_GROUP, P.sample)) continue;
-      r = 0;
-      for (uint32_t e = 0; e < c; ++e) r += group_sampled(hb, e * s.csz / SAMPLE_GROUP, P.sample);
-    }
-    if (b >= 0) {
-      Unit& u = units[(size_t)b * s.nch_s + r];
-      u.s1 = s1;
-      u.o1 = o1;
-    }
-    if ((uint32_t)(b + 1) < nseg) {
-      Unit& u = units[(size_t)(b + 1) * s.nch_s + r];
-      u.h = hb;
-      u.chunk = c;
-      u.s0 = s0;
-      u.o0 = o0;
-    }
-  }
+// Chunks of the home bin with candidates in segment b: those whose first row
+// lies below the segment's end.  The home bin leads its own neighbour list
+// and a pair of two of its rows is taken at the smaller one, so chunk c has no
+// candidates below rank c * csz (unit_bin skips them); segments are multiples
+// of csz long.  Without this half of every home bin's own square was
+// evaluated twice: 10 % of the cells of a 1M x 384 join with 62 bins.
+__device__ __forceinline__ uint32_t seg_chunks(const HomeSplit& s, uint32_t seg, uint32_t b) {
+  return (uint32_t)min((unsigned long long)s.nch, (b + 1ull) * (seg / s.csz));
 }
+
+// Units of all nseg segments of a home bin.
+__device__ __forceinline__ unsigned long long count_units(const EnumParams& P, const HomeSplit& s, uint32_t hb,
+                                                          uint32_t seg, uint32_t nseg) {
+  const uint32_t r = seg / s.csz;
+  if (P.sample <= 1) {
+    // (b + 1) r chunks while that is at most nch, then nch
+    const unsigned long long B = min(nseg, s.nch / r);
+    return r * (B * (B + 1) / 2) + (nseg - B) * (unsigned long long)s.nch;
+  }
+  unsigned long long u = 0;
+  for (uint32_t c = 0; c < s.nch; ++c)
+    if (group_sampled(hb, c * s.csz / SAMPLE_GROUP, P.sample)) u += nseg - c / r;
+  return u;
+}
+
+// The units of one home bin while its neighbour list is walked: cut() ends
+// those of the current segment at (s1, o1) and starts the next segment's at
+// (s0, o0).  WARP: a warp's lanes share the chunks; else one thread.
+template <bool WARP>
+struct UnitWriter {
+  Unit* units;   // of the current segment
+  uint32_t hb, seg, nseg, b;
+
+  __device__ __forceinline__ uint32_t each(const EnumParams& P, const HomeSplit& s, uint32_t nc, Unit* u, bool start,
+                                           uint32_t e, uint32_t o) const {
+    uint32_t n = 0;  // sampled chunks so far
+    for (uint32_t c0 = 0; c0 < nc; c0 += WARP ? 32u : 1u) {
+      const uint32_t c = c0 + (WARP ? (threadIdx.x & 31u) : 0u);
+      const bool take = c < nc && group_sampled(hb, c * s.csz / SAMPLE_GROUP, P.sample);
+      const uint32_t m = WARP ? __ballot_sync(FULL_MASK, take) : (take ? 1u : 0u);
+      if (take) {
+        Unit& t = u[n + (WARP ? __popc(m & ((1u << (threadIdx.x & 31u)) - 1u)) : 0)];
+        if (start) {
+          t.h = hb;
+          t.chunk = c;
+          t.s0 = e;
+          t.o0 = o;
+        } else {
+          t.s1 = e;
+          t.o1 = o;
+        }
+      }
+      n += __popc(m);
+    }
+    return n;
+  }
+  __device__ __forceinline__ void begin(const EnumParams& P, const HomeSplit& s, uint32_t s0) {
+    b = 0;
+    if (nseg) each(P, s, seg_chunks(s, seg, 0), units, true, s0, 0);
+  }
+  __device__ __forceinline__ void cut(const EnumParams& P, const HomeSplit& s, uint32_t s1, uint32_t o1, uint32_t s0,
+                                      uint32_t o0) {
+    units += each(P, s, seg_chunks(s, seg, b), units, false, s1, o1);
+    if (++b < nseg) each(P, s, seg_chunks(s, seg, b), units, true, s0, o0);
+  }
+};
 
 // Adds the home bin's candidate points, once per home chunk, to its class's
 // total (the segment lengths are chosen from it).
@@ -546,10 +585,9 @@ __global__ void __launch_bounds__(128, 8) k_enum(const uint64_t* __restrict__ bk
     const uint32_t seg = FILL ? tot->seg[tc ? 1 : 0] : 0u;
     const uint32_t total = FILL ? npts[hb] : 0u;
     const uint32_t nseg = FILL ? (uint32_t)(((unsigned long long)total + seg - 1) / seg) : 0u;
-    Unit* units = FILL ? (tc ? units_tc + unit_off_tc[hb] : units_simt + unit_off[hb]) : nullptr;
+    UnitWriter<false> uw{FILL ? (tc ? units_tc + unit_off_tc[hb] : units_simt + unit_off[hb]) : nullptr, hb, seg, nseg, 0};
     unsigned long long cut = seg;  // candidate rank of the next segment boundary
-    int b = 0;
-    if (FILL) write_cut(units, P, hsp, hb, -1, nseg, 0, 0, n0, 0, 0, 1);
+    if (FILL) uw.begin(P, hsp, n0);
 
     // Visits neighbour bin `a` (ascending, a >= hb): its points, and in pass
     // 2 the neighbour list and the segment boundaries that fall inside it.
@@ -557,12 +595,11 @@ __global__ void __launch_bounds__(128, 8) k_enum(const uint64_t* __restrict__ bk
       const uint32_t bsz = bstart[a + 1] - bstart[a];
       if (FILL) {
         nbr[n0 + cnt] = a;
-        for (; cut <= (unsigned long long)pts + bsz; cut += seg, ++b) {
+        for (; cut <= (unsigned long long)pts + bsz; cut += seg) {
           const uint32_t o = (uint32_t)(cut - pts);  // 1 .. bsz
-          write_cut(units, P, hsp, hb, b, nseg, n0 + cnt + 1, o, n0 + cnt + (o == bsz), o == bsz ? 0u : o, 0, 1);
+          uw.cut(P, hsp, n0 + cnt + 1, o, n0 + cnt + (o == bsz), o == bsz ? 0u : o);
         }
-        if (pts + bsz == total && b < (int)nseg)  // the list ends inside segment b
-          write_cut(units, P, hsp, hb, b, nseg, n0 + cnt + 1, bsz, 0, 0, 0, 1);
+        if (pts + bsz == total && uw.b < nseg) uw.cut(P, hsp, n0 + cnt + 1, bsz, 0, 0);  // the list ends in segment b
       }
       pts += bsz;
       ++cnt;
@@ -640,10 +677,10 @@ k_enum_flat(const uint64_t* __restrict__ bkey, const uint32_t* __restrict__ bsta
   const uint32_t seg = FILL ? tot->seg[hsp.tc ? 1 : 0] : 0u;
   const uint32_t total = FILL ? npts[hb] : 0u;
   const uint32_t nseg = FILL ? (uint32_t)(((unsigned long long)total + seg - 1) / seg) : 0u;
-  Unit* units = FILL ? (hsp.tc ? units_tc + unit_off_tc[hb] : units_simt + unit_off[hb]) : nullptr;
+  UnitWriter<true> uw{FILL ? (hsp.tc ? units_tc + unit_off_tc[hb] : units_simt + unit_off[hb]) : nullptr, hb, seg, nseg,
+                      0};
   unsigned long long cut = seg;
-  int b = 0;
-  if (FILL) write_cut(units, P, hsp, hb, -1, nseg, 0, 0, n0, 0, lane, 32);
+  if (FILL) uw.begin(P, hsp, n0);
   for (uint32_t c0 = hb; c0 < end; c0 += 32) {
     const uint32_t a = c0 + lane;
     bool ok = a < end;
@@ -666,17 +703,16 @@ k_enum_flat(const uint64_t* __restrict__ bkey, const uint32_t* __restrict__ bsta
       const uint32_t pos = n0 + cnt + __popc(hit & ((1u << lane) - 1u));
       if (ok) nbr[pos] = a;
       // segment boundaries among these bins' points (warp-uniform loop)
-      for (; cut <= (unsigned long long)pts + step; cut += seg, ++b) {
+      for (; cut <= (unsigned long long)pts + step; cut += seg) {
         const uint32_t r = (uint32_t)(cut - pts);  // 1 .. step: inside the first bin whose inclusive end reaches r
         const int src = __ffs(__ballot_sync(FULL_MASK, ok && incl >= r)) - 1;
         const uint32_t e = __shfl_sync(FULL_MASK, pos, src), z = __shfl_sync(FULL_MASK, bsz, src);
         const uint32_t o = r - (__shfl_sync(FULL_MASK, incl, src) - z);
-        write_cut(units, P, hsp, hb, b, nseg, e + 1, o, e + (o == z), o == z ? 0u : o, lane, 32);
+        uw.cut(P, hsp, e + 1, o, e + (o == z), o == z ? 0u : o);
       }
-      if (pts + step == total && b < (int)nseg) {  // the list ends inside segment b
+      if (pts + step == total && uw.b < nseg) {  // the list ends in segment b
         const int src = 31 - __clz(hit);
-        write_cut(units, P, hsp, hb, b, nseg, __shfl_sync(FULL_MASK, pos, src) + 1, __shfl_sync(FULL_MASK, bsz, src), 0,
-                  0, lane, 32);
+        uw.cut(P, hsp, __shfl_sync(FULL_MASK, pos, src) + 1, __shfl_sync(FULL_MASK, bsz, src), 0, 0);
       }
     }
     pts += step;
@@ -707,6 +743,8 @@ __global__ void k_unit_plan(const uint32_t* __restrict__ bstart, uint32_t m, Enu
       const unsigned long long fair = (tot->work[c] / P.want_units[c] + 127) & ~127ull;
       seg[c] = (uint32_t)min((unsigned long long)P.seg_max[c], max((unsigned long long)P.seg_min[c], fair));
     }
+    const uint32_t csz = c ? P.tc_chunk : P.chunk;  // a multiple of the home chunk (seg_chunks)
+    seg[c] = (seg[c] + csz - 1) / csz * csz;
   }
   if (blockIdx.x == 0 && threadIdx.x < 2) tot->seg[threadIdx.x] = seg[threadIdx.x];
   unsigned long long s[4] = {0, 0, 0, 0};
@@ -714,7 +752,7 @@ __global__ void k_unit_plan(const uint32_t* __restrict__ bstart, uint32_t m, Enu
     const uint32_t asz = bstart[hb + 1] - bstart[hb];
     const HomeSplit h = home_split(P, hb, asz);
     const uint32_t sg = seg[h.tc ? 1 : 0];
-    const unsigned long long nu = (unsigned long long)h.nch_s * (((unsigned long long)npts[hb] + sg - 1) / sg);
+    const unsigned long long nu = count_units(P, h, hb, sg, (uint32_t)(((unsigned long long)npts[hb] + sg - 1) / sg));
     // a bin's unit count saturates at 2^32 - 1; the 64-bit totals then exceed
     // the 32-bit offsets the work lists use, and the call fails with
     // MISTIC_ERR_TOO_LARGE

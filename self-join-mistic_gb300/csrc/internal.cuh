@@ -75,17 +75,6 @@ struct Unit {
   uint32_t o1;
 };
 
-// Points [first, first + size) of neighbour entry `e` (an index into nbr) as
-// one unit sees them.
-__device__ __forceinline__ void unit_bin(const Unit& U, const uint32_t* nbr, const uint32_t* bstart, uint32_t e,
-                                         uint32_t* bin, uint32_t* first, uint32_t* size) {
-  const uint32_t b = nbr[e], st = bstart[b];
-  const uint32_t lo = e == U.s0 ? U.o0 : 0u, hi = e + 1 == U.s1 ? U.o1 : bstart[b + 1] - st;
-  *bin = b;
-  *first = st + lo;
-  *size = hi - lo;
-}
-
 // Counters the join kernels accumulate on the device.
 struct JoinCounters {
   unsigned long long pairs;      // accepted unordered pairs

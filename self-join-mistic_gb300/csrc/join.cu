@@ -218,14 +218,14 @@ struct CandTile {
   bool qv;
 };
 
-__device__ __forceinline__ CandTile next_tile(const Unit& U, const uint32_t* nbr, const uint32_t* bstart, uint32_t& s,
-                                              uint32_t& off) {
+__device__ __forceinline__ CandTile next_tile(const Unit& U, uint32_t ch, const uint32_t* nbr, const uint32_t* bstart,
+                                              uint32_t& s, uint32_t& off) {
   const int lane = threadIdx.x & 31;
   const uint32_t bj = s + lane, s1 = U.s1;
   uint32_t start = 0, size = 0;
   if (bj < s1) {
     uint32_t b;
-    unit_bin(U, nbr, bstart, bj, &b, &start, &size);
+    unit_bin(U, ch, nbr, bstart, bj, &b, &start, &size);
     if (lane == 0) {
       start += off;
       size -= off;
@@ -330,7 +330,7 @@ k_join_f32(const JoinParams P) {
     __syncwarp();
     uint32_t s = U.s0, off = 0;
     while (s < U.s1) {
-      const CandTile t = next_tile(U, V.nbr, V.bstart, s, off);
+      const CandTile t = next_tile(U, CH, V.nbr, V.bstart, s, off);
       const uint32_t q = t.q;
       const float4* qrow = X + (size_t)(t.qv ? q : a0) * nq4;
       float acc[CH];
@@ -397,7 +397,7 @@ k_join_f32r(const JoinParams P) {
     __syncwarp();
     uint32_t s = U.s0, off = 0;
     while (s < U.s1) {
-      const CandTile t = next_tile(U, V.nbr, V.bstart, s, off);
+      const CandTile t = next_tile(U, CH, V.nbr, V.bstart, s, off);
       const uint32_t q = t.q;
       const ulonglong2* qrow = reinterpret_cast<const ulonglong2*>(X + (size_t)(t.qv ? q : a0) * DQ);
       ulonglong2 qq[DQ];  // the candidate row as pairs of floats
@@ -526,7 +526,7 @@ k_join_f64(const JoinParams P) {
     __syncwarp();
     uint32_t s = U.s0, off = 0;
     while (s < U.s1) {
-      const CandTile t = next_tile(U, V.nbr, V.bstart, s, off);
+      const CandTile t = next_tile(U, CH, V.nbr, V.bstart, s, off);
       const uint32_t q = t.q;
       const double2* qrow = X + (size_t)(t.qv ? q : a0) * nq2;
       double acc[CH];

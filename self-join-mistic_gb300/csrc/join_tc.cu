@@ -462,7 +462,7 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
           const long long cw0 = T.prof ? clock64() : 0;
           const uint32_t nb = min((uint32_t)WIN, U.s1 - seg_next);
           uint32_t st0 = 0, sz0 = 0, bn = 0xffffffffu;
-          if ((uint32_t)tid < nb) unit_bin(U, nbr, bstart, seg_next + tid, &bn, &st0, &sz0);
+          if ((uint32_t)tid < nb) unit_bin(U, TM * G, nbr, bstart, seg_next + tid, &bn, &st0, &sz0);
           const uint32_t incl = warp_scan_incl(sz0);
           if (lane == 31) S.scan_ws[warp] = incl;
           prod_sync();
@@ -776,7 +776,7 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
           const long long cw0 = T.prof ? clock64() : 0;
           const uint32_t nb = min((uint32_t)WIN, U.s1 - seg_next);
           uint32_t st0 = 0, sz0 = 0, bn = 0xffffffffu;
-          if ((uint32_t)tid < nb) unit_bin(U, nbr, bstart, seg_next + tid, &bn, &st0, &sz0);
+          if ((uint32_t)tid < nb) unit_bin(U, TM * G, nbr, bstart, seg_next + tid, &bn, &st0, &sz0);
           const uint32_t incl = warp_scan_incl(sz0);
           if (lane == 31) S.scan_ws[warp] = incl;
           prod_sync();

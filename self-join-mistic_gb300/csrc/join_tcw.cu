@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(WTHREADS, 1)
         if (w_pos >= w_total) {  // next window of up to WWIN neighbour bins
           const uint32_t nb = min((uint32_t)WWIN, U.s1 - seg_next);
           uint32_t st0 = 0, sz0 = 0, bn = 0xffffffffu;
-          if (t < nb) unit_bin(U, P.nbr, P.bstart, seg_next + t, &bn, &st0, &sz0);
+          if (t < nb) unit_bin(U, WG * WM, P.nbr, P.bstart, seg_next + t, &bn, &st0, &sz0);
           const uint32_t incl = warp_scan_incl(sz0);
           if (lane == 31) S.scan_ws[warp] = incl;
           wprod_sync();
