@@ -31,58 +31,132 @@ __device__ __forceinline__ double ld(const T* p, size_t i) {
 // Per-column min, max and sum over all rows plus a finiteness flag.  Each
 // block writes its partials; a second kernel folds them in a fixed order so
 // the result (and therefore the reference points) is deterministic.
+//
+// A block reads its rows as one stream, RG = 256 / cols rows at a time, thread
+// t always at column t % cols, so that narrow rows fill the warps too (lanes
+// tied to 32 columns left 30 of 32 idle at d = 2); rows above 256 columns are
+// cut into column tiles.  FP64 values are compared as order-preserving
+// integers: FP64 compares run on the FP64 pipe, whose rate is 1/75 of FP32's,
+// and with the sum they bound the pass before HBM did.  The whole phase (this,
+// the sample covariance, the reference points): 2M x 2 FP32 0.94 -> 0.15 ms;
+// 5M x 18 FP64 1.81 -> 0.56 ms (the rows alone 0.11 ms at HBM's rate).
 
-constexpr int CS_ROWS = 8;
+constexpr int CS_THREADS = 256;
 
 template <class T>
-__global__ void k_colstats(const T* __restrict__ x, size_t n, uint32_t d, double* __restrict__ part,
-                           unsigned* __restrict__ nonfinite) {
-  // part layout: [blockIdx.y][3][d] : min, max, sum for the block's rows of column tile blockIdx.x
-  __shared__ double smin[CS_ROWS][32], smax[CS_ROWS][32], ssum[CS_ROWS][32];
-  const uint32_t col = blockIdx.x * 32 + threadIdx.x;
-  double mn = INFINITY, mx = -INFINITY, sm = 0.0;
+struct ColMinMax;
+template <>
+struct ColMinMax<float> {
+  float mn = INFINITY, mx = -INFINITY;
+  __device__ void add(float v) {  // NaN leaves both unchanged
+    mn = fminf(mn, v);
+    mx = fmaxf(mx, v);
+  }
+  __device__ double lo() const { return mn; }
+  __device__ double hi() const { return mx; }
+};
+template <>
+struct ColMinMax<double> {
+  // bits of a double, the magnitude bits of negative ones flipped: signed
+  // integer order is then the order of the values
+  static constexpr long long kInf = 0x7ff0000000000000ll;
+  long long mn, mx;
+  static __device__ long long key(double v) {
+    const long long b = __double_as_longlong(v);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+  }
+  static __device__ double val(long long k) { return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll)); }
+  __device__ ColMinMax() : mn(key(INFINITY)), mx(key(-INFINITY)) {}
+  __device__ void add(double v) {  // NaN leaves both unchanged
+    const long long k = key(v);
+    const bool num = (__double_as_longlong(v) & 0x7fffffffffffffffll) <= kInf;
+    if (num && k < mn) mn = k;
+    if (num && k > mx) mx = k;
+  }
+  __device__ double lo() const { return val(mn); }
+  __device__ double hi() const { return val(mx); }
+};
+
+__device__ __forceinline__ bool finite_bits(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
+__device__ __forceinline__ bool finite_bits(double v) {
+  return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000;
+}
+
+template <class T>
+__global__ void __launch_bounds__(CS_THREADS)
+k_colstats(const T* __restrict__ x, size_t n, uint32_t d, double* __restrict__ part, unsigned* __restrict__ nonfinite) {
+  // part layout: [blockIdx.y][3][d] : min, max, sum of the block's rows, column tile blockIdx.x
+  __shared__ double red[3][CS_THREADS];
+  const uint32_t c0 = blockIdx.x * CS_THREADS, cols = min((uint32_t)CS_THREADS, d - c0);
+  const uint32_t rg = CS_THREADS / cols;                       // rows side by side
+  const uint32_t r = threadIdx.x / cols, c = threadIdx.x % cols;
+  ColMinMax<T> mm;
+  double sm[4] = {0, 0, 0, 0};
   bool bad = false;
-  if (col < d) {
-    for (size_t r = (size_t)blockIdx.y * CS_ROWS + threadIdx.y; r < n; r += (size_t)gridDim.y * CS_ROWS) {
-      double v = ld(x, r * d + col);
-      if (!isfinite(v)) bad = true;
-      mn = fmin(mn, v);
-      mx = fmax(mx, v);
-      sm += v;
+  if (r < rg) {
+    const size_t step = (size_t)gridDim.y * rg, stride = step * d;
+    size_t row = (size_t)blockIdx.y * rg + r;
+    const T* p = x + row * d + c0 + c;
+    for (; row + 3 * step < n; row += 4 * step, p += 4 * stride) {
+      T v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[k] = p[k * stride];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        bad |= !finite_bits(v[k]);
+        mm.add(v[k]);
+        sm[k] += (double)v[k];
+      }
+    }
+    for (; row < n; row += step, p += stride) {
+      const T v = *p;
+      bad |= !finite_bits(v);
+      mm.add(v);
+      sm[0] += (double)v;
     }
   }
   if (bad) atomicOr(nonfinite, 1u);
-  smin[threadIdx.y][threadIdx.x] = mn;
-  smax[threadIdx.y][threadIdx.x] = mx;
-  ssum[threadIdx.y][threadIdx.x] = sm;
+  red[0][threadIdx.x] = mm.lo();
+  red[1][threadIdx.x] = mm.hi();
+  red[2][threadIdx.x] = (sm[0] + sm[1]) + (sm[2] + sm[3]);
   __syncthreads();
-  if (threadIdx.y == 0 && col < d) {
-    for (int r = 1; r < CS_ROWS; ++r) {
-      mn = fmin(mn, smin[r][threadIdx.x]);
-      mx = fmax(mx, smax[r][threadIdx.x]);
-      sm += ssum[r][threadIdx.x];
+  if (threadIdx.x < cols) {
+    double mn = red[0][c], mx = red[1][c], s = red[2][c];
+    for (uint32_t q = 1; q < rg; ++q) {
+      mn = fmin(mn, red[0][q * cols + c]);
+      mx = fmax(mx, red[1][q * cols + c]);
+      s += red[2][q * cols + c];
     }
-    double* p = part + (size_t)blockIdx.y * 3 * d;
-    p[col] = mn;
-    p[d + col] = mx;
-    p[2 * d + col] = sm;
+    double* o = part + (size_t)blockIdx.y * 3 * d + c0 + c;
+    o[0] = mn;
+    o[d] = mx;
+    o[2 * (size_t)d] = s;
   }
 }
 
+// A warp per column over the blocks' partials.
 __global__ void k_colstats_final(const double* __restrict__ part, uint32_t nparts, uint32_t d,
                                  size_t n, double* __restrict__ out /* mean, min, max */) {
-  const uint32_t col = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t col = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (col >= d) return;
   double mn = INFINITY, mx = -INFINITY, sm = 0.0;
-  for (uint32_t b = 0; b < nparts; ++b) {
-    const double* p = part + (size_t)b * 3 * d;
-    mn = fmin(mn, p[col]);
-    mx = fmax(mx, p[d + col]);
-    sm += p[2 * d + col];
+  for (uint32_t b = lane; b < nparts; b += 32) {
+    const double* p = part + (size_t)b * 3 * d + col;
+    mn = fmin(mn, p[0]);
+    mx = fmax(mx, p[d]);
+    sm += p[2 * (size_t)d];
   }
-  out[col] = n ? sm / (double)n : 0.0;
-  out[d + col] = mn;
-  out[2 * d + col] = mx;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    mn = fmin(mn, __shfl_xor_sync(FULL_MASK, mn, o));
+    mx = fmax(mx, __shfl_xor_sync(FULL_MASK, mx, o));
+    sm += __shfl_xor_sync(FULL_MASK, sm, o);
+  }
+  if (lane == 0) {
+    out[col] = n ? sm / (double)n : 0.0;
+    out[d + col] = mn;
+    out[2 * (size_t)d + col] = mx;
+  }
 }
 
 // ------------------------------------------------------------ sample covariance
@@ -135,44 +209,60 @@ __global__ void k_sample_cov_final(const double* __restrict__ part, uint32_t chu
 
 // ------------------------------------------------------------ reference-point distances
 // D[i][j] = FP64 ||x_i - r_j|| (sequential sum, then sqrt), with per-block
-// min/max partials per reference point.
+// min/max partials per reference point.  Bound by the FP64 pipe (2 k d
+// operations a row).  A block's 256 rows pass through shared memory RPD_COLS
+// columns at a time, each value read once for all k sums, so rows of any
+// length load coalesced: a thread reading its own row of 384 FP32 values took
+// 17.5 ms for 1M rows at k = 8, now 12.1 ms; 515k x 90 4.0 -> 1.7 ms.
 constexpr int RPD_THREADS = 256;
-constexpr uint32_t RPD_DMAX = 48;  // rows staged in shared memory up to this d
+constexpr int RPD_COLS = 32;
 
-template <class T>
+template <class T, int K>
 __global__ void __launch_bounds__(RPD_THREADS)
 k_rp_dist(const T* __restrict__ x, size_t n, uint32_t d, const double* __restrict__ rps, int k,
           double* __restrict__ D, double* __restrict__ part /* [block][2][k] */) {
-  // dynamic shared memory: k x d reference points, then a tile of rows
-  // (RPD_THREADS rows of up to RPD_DMAX coordinates) copied with coalesced loads
-  extern __shared__ double srp[];
-  double* tile = srp + (size_t)k * d;
-  for (uint32_t i = threadIdx.x; i < (uint32_t)k * d; i += blockDim.x) srp[i] = rps[i];
+  extern __shared__ double tile[];  // RPD_THREADS rows x (RPD_COLS + 1), then K x RPD_COLS reference values
+  double* srp = tile + RPD_THREADS * (RPD_COLS + 1);
   __shared__ double smn[MAX_K][RPD_THREADS / 32], smx[MAX_K][RPD_THREADS / 32];
-  const size_t row0 = (size_t)blockIdx.x * blockDim.x;
-  const uint32_t rows = (uint32_t)min((size_t)blockDim.x, n > row0 ? n - row0 : 0);
-  const bool staged = d <= RPD_DMAX;
-  if (staged) {
-    const size_t base = row0 * d;
-    for (uint32_t i = threadIdx.x; i < rows * d; i += blockDim.x) tile[i] = (double)x[base + i];
+  const size_t row0 = (size_t)blockIdx.x * RPD_THREADS;
+  const uint32_t rows = (uint32_t)min((size_t)RPD_THREADS, n - row0);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double s[K];
+#pragma unroll
+  for (int j = 0; j < K; ++j) s[j] = 0.0;
+  for (uint32_t t0 = 0; t0 < d; t0 += RPD_COLS) {
+    const uint32_t nc = min((uint32_t)RPD_COLS, d - t0);
+    __syncthreads();
+    if (nc == d) {  // whole rows: one contiguous run
+      for (uint32_t e = threadIdx.x; e < rows * d; e += RPD_THREADS)
+        tile[(e / d) * (RPD_COLS + 1) + e % d] = (double)x[row0 * d + e];
+    } else if ((uint32_t)lane < nc) {
+      for (uint32_t r = w; r < rows; r += RPD_THREADS / 32)
+        tile[r * (RPD_COLS + 1) + lane] = (double)x[(row0 + r) * d + t0 + lane];
+    }
+    for (uint32_t e = threadIdx.x; e < K * RPD_COLS; e += RPD_THREADS) {
+      const uint32_t j = e / RPD_COLS, t = e % RPD_COLS;
+      srp[e] = j < (uint32_t)k && t < nc ? rps[(size_t)j * d + t0 + t] : 0.0;
+    }
+    __syncthreads();
+    const double* xr = tile + threadIdx.x * (RPD_COLS + 1);
+    for (uint32_t t = 0; t < nc; ++t) {
+      const double xv = xr[t];
+#pragma unroll
+      for (int j = 0; j < K; ++j) {
+        if (j >= k) break;
+        const double df = xv - srp[j * RPD_COLS + t];
+        s[j] = fma(df, df, s[j]);
+      }
+    }
   }
-  __syncthreads();
   const size_t i = row0 + threadIdx.x;
   const bool valid = i < n;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int j = 0; j < k; ++j) {
-    double dist = 0.0;
-    if (valid) {
-      double s = 0.0;
-      const double* r = srp + (size_t)j * d;
-      for (uint32_t t = 0; t < d; ++t) {
-        const double xv = staged ? tile[(size_t)threadIdx.x * d + t] : (double)x[i * d + t];
-        const double df = xv - r[t];
-        s = fma(df, df, s);
-      }
-      dist = sqrt(s);
-      D[i * k + j] = dist;
-    }
+#pragma unroll
+  for (int j = 0; j < K; ++j) {
+    if (j >= k) break;
+    const double dist = sqrt(s[j]);
+    if (valid) D[i * k + j] = dist;
     double mn = valid ? dist : INFINITY, mx = valid ? dist : -INFINITY;
 #pragma unroll
     for (int o = 16; o; o >>= 1) {
@@ -796,13 +886,13 @@ namespace idx {
 
 void colstats(mistic_handle_s* h, const void* x, mistic_dtype dt, size_t n, uint32_t d,
               double* part, uint32_t nparts, double* out, unsigned* nonfinite) {
-  dim3 blk(32, CS_ROWS), grd((d + 31) / 32, nparts);
+  const dim3 grd((d + CS_THREADS - 1) / CS_THREADS, nparts);
   if (dt == MISTIC_F64)
-    k_colstats<double><<<grd, blk, 0, h->stream>>>((const double*)x, n, d, part, nonfinite);
+    k_colstats<double><<<grd, CS_THREADS, 0, h->stream>>>((const double*)x, n, d, part, nonfinite);
   else
-    k_colstats<float><<<grd, blk, 0, h->stream>>>((const float*)x, n, d, part, nonfinite);
+    k_colstats<float><<<grd, CS_THREADS, 0, h->stream>>>((const float*)x, n, d, part, nonfinite);
   launched(h, "colstats");
-  k_colstats_final<<<(d + 127) / 128, 128, 0, h->stream>>>(part, nparts, d, n, out);
+  k_colstats_final<<<(d + 7) / 8, 256, 0, h->stream>>>(part, nparts, d, n, out);
   launched(h, "colstats_final");
 }
 
@@ -825,15 +915,15 @@ void sample_cov(mistic_handle_s* h, const void* x, mistic_dtype dt, size_t n, ui
 
 void rp_dist(mistic_handle_s* h, const void* x, mistic_dtype dt, size_t n, uint32_t d,
              const double* rps, int k, double* D, double* part, uint32_t nparts, double* mm) {
-  const size_t smem = (size_t)k * d * sizeof(double) + (d <= RPD_DMAX ? (size_t)RPD_THREADS * d * sizeof(double) : 0);
-  if (dt == MISTIC_F64)  // the limit includes static shared memory: raise it whatever the size
-    allow_max_dyn_smem(k_rp_dist<double>);
-  else
-    allow_max_dyn_smem(k_rp_dist<float>);
+  auto launch = [&](auto kern, const auto* xs, int K) {
+    allow_max_dyn_smem(kern);
+    const size_t smem = (RPD_THREADS * (RPD_COLS + 1) + (size_t)K * RPD_COLS) * sizeof(double);
+    kern<<<nparts, RPD_THREADS, smem, h->stream>>>(xs, n, d, rps, k, D, part);
+  };
   if (dt == MISTIC_F64)
-    k_rp_dist<double><<<nparts, RPD_THREADS, smem, h->stream>>>((const double*)x, n, d, rps, k, D, part);
+    k <= 8 ? launch(k_rp_dist<double, 8>, (const double*)x, 8) : launch(k_rp_dist<double, 16>, (const double*)x, 16);
   else
-    k_rp_dist<float><<<nparts, RPD_THREADS, smem, h->stream>>>((const float*)x, n, d, rps, k, D, part);
+    k <= 8 ? launch(k_rp_dist<float, 8>, (const float*)x, 8) : launch(k_rp_dist<float, 16>, (const float*)x, 16);
   launched(h, "rp_dist");
   k_minmax_final<<<k, 256, 0, h->stream>>>(part, nparts, k, mm);
   launched(h, "minmax_final");

@@ -779,7 +779,7 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
   clk.mark();  // 1
 
   // ---- column statistics (+ finiteness) and, for PCA points, a sample covariance
-  const uint32_t cs_parts = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(1, n / 2048), 1024);
+  const uint32_t cs_parts = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(1, n / 256), 1216);
   double* cs_part = abuf<double>(h, "cs_part", (size_t)cs_parts * 3 * d);
   double* cs_out = abuf<double>(h, "cs_out", 3 * (size_t)d);
   unsigned* flag = abuf<unsigned>(h, "flag", 4);
