@@ -293,11 +293,11 @@ size_t scan_partials_count(size_t n);
 // (0/1) holds the result.
 int radix_sort_u64(mistic_handle_s* h, uint64_t* keys[2], uint32_t* vals[2], size_t n, int bits);
 
-// ---- rows.cu: np packed pairs (i << 32 | j, i < j < n), sorted by (i, j) in
-// place and stored in memory order (i, j); in a fused batch (row0 of n_inst
-// instances) with ids relative to their instance.
-void sort_pairs_ij(mistic_handle_s* h, unsigned long long* pairs, size_t np, size_t n, const uint32_t* row0,
-                   uint32_t n_inst);
+// ---- rows.cu: np packed pairs (i << 32 | j, i < j < n), sorted by (i, j) and
+// stored in memory order (i, j) in out (which may be pairs); in a fused batch
+// (row0 of n_inst instances) with ids relative to their instance.
+void sort_pairs_ij(mistic_handle_s* h, const unsigned long long* pairs, unsigned long long* out, size_t np, size_t n,
+                   const uint32_t* row0, uint32_t n_inst);
 // The neighbour table of the pairs: 2 np + n ids, ascending within each row
 // (its own id included), and n + 1 row offsets.
 void neighbour_table(mistic_handle_s* h, const unsigned long long* pairs, size_t np, size_t n, uint32_t* nbrs,

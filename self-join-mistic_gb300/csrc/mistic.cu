@@ -37,7 +37,7 @@
 
 namespace mistic {
 
-void pairs_to_ij(mistic_handle_s* h, unsigned long long* p, size_t n);
+void pairs_to_ij(mistic_handle_s* h, const unsigned long long* p, unsigned long long* out, size_t n);
 
 // ------------------------------------------------------------------ plumbing
 
@@ -950,8 +950,13 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
   // long rows (augmented K above one 128-wide operand tile), and every row in
   // tf32 mode, use the K-chunked kernel over rows prepared once; its operand
   // precision is picked from the bound (see tc_precision)
-  // (the fused batch join drains medium rows with the short-row kernel only)
-  const bool wide = use_tc && (tf32_mode || join::tc_kp(d) > 128 || (!ex && tcw_for_medium_rows(d, eps2, R)));
+  // The fused batch join drains medium rows with the short-row kernel only;
+  // that kernel needs about four times the K-chunked one's time a cell
+  // there, so only instances too small to repay a join of their own stay in
+  // it: at 15,000 x 90 (1e8 candidate pairs) that is 0.15 ms fused against
+  // 0.2 ms of launches and read-backs, at 168,656 x 90 about 13 against 5.5 ms.
+  const bool wide = use_tc && (tf32_mode || join::tc_kp(d) > 128 ||
+                               ((!ex || n >= 16384) && tcw_for_medium_rows(d, eps2, R)));
   const int prec = wide ? tc_precision(o.mode, d, eps2, R) : 0;
   r->mode_used = fp64 ? MISTIC_MODE_FP64
                       : (use_tc ? (tf32_mode ? MISTIC_MODE_TF32 : MISTIC_MODE_BF16) : MISTIC_MODE_FP32);
@@ -1596,10 +1601,28 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
   } else if (want_pairs) {
     const unsigned long long stored = std::min<unsigned long long>(hc.pairs, cap);
     if (hc.pairs > cap) tail = MISTIC_ERR_PAIR_OVERFLOW;
+    // A list the result owns is written to a block of its own size: the join's
+    // buffer stays with the handle at the size this data needed, where a
+    // handed-over one would be sized afresh by the next call, and the join
+    // run twice whenever a point has more than 16 pairs on average.
+    unsigned long long* out = pbuf;
+    if (o.pairs == MISTIC_PAIRS_DEVICE && !caller_buf) {
+      void* dp = nullptr;
+      if (cudaMalloc(&dp, std::max<size_t>(8, stored * 8)) == cudaSuccess)
+        out = (unsigned long long*)dp;
+      else
+        cudaGetLastError();  // no room for both: the join's buffer goes to the result
+    }
+    // the result's from here on: freed with it if the call fails
+    if (out != pbuf) {
+      r->pairs = (uint32_t*)out;
+      r->pairs_on_device = 1;
+      r->_owner = (void*)out;
+    }
     if (o.sort_pairs && stored > 1)
-      sort_pairs_ij(h, pbuf, stored, n, nullptr, 0);
+      sort_pairs_ij(h, pbuf, out, stored, n, nullptr, 0);
     else
-      pairs_to_ij(h, pbuf, stored);
+      pairs_to_ij(h, pbuf, out, stored);
     r->pairs_len = stored;
     if (o.pairs == MISTIC_PAIRS_HOST) {
       uint32_t* hp = (uint32_t*)pinned_cache().acquire(std::max<size_t>(1, stored * 8));
@@ -1614,7 +1637,7 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
       r->pairs = o.pair_buffer;  // caller keeps ownership
       r->pairs_on_device = 1;
       r->_owner = nullptr;
-    } else {
+    } else if (out == pbuf) {
       // hand the device buffer to the result; the arena forgets it
       h->arena.bufs.erase("pairs");
       r->pairs = (uint32_t*)pbuf;
@@ -1980,7 +2003,7 @@ mistic_status run_batch_fused(mistic_handle h, const mistic_instance* inst, uint
     const unsigned long long* sorted = pbuf;
     for (uint32_t g = 0; g < G; ++g) pstart[g + 1] = pstart[g] + ipairs[g];
     if (pstart[G] != hc.pairs) throw Error(MISTIC_ERR_INTERNAL, "per-instance pair counts do not add up");
-    sort_pairs_ij(h, pbuf, hc.pairs, (size_t)row0.back() + inst[m - 1].n, d_row0, G);
+    sort_pairs_ij(h, pbuf, pbuf, hc.pairs, (size_t)row0.back() + inst[m - 1].n, d_row0, G);
     for (uint32_t g = 0; g < G; ++g) {
       mistic_result& r = results[gl[g]];
       const unsigned long long np = ipairs[g];
@@ -2022,17 +2045,17 @@ mistic_status run_batch_fused(mistic_handle h, const mistic_instance* inst, uint
 
 }  // namespace
 
-__global__ void k_pairs_to_ij(unsigned long long* p, size_t n) {
+__global__ void k_pairs_to_ij(const unsigned long long* p, unsigned long long* out, size_t n) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const unsigned long long v = p[i];
   // packed (i << 32 | j) -> memory order (i, j) as two uint32
-  p[i] = (v >> 32) | (v << 32);
+  out[i] = (v >> 32) | (v << 32);
 }
 
-void pairs_to_ij(mistic_handle_s* h, unsigned long long* p, size_t n) {
+void pairs_to_ij(mistic_handle_s* h, const unsigned long long* p, unsigned long long* out, size_t n) {
   if (!n) return;
-  k_pairs_to_ij<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(p, n);
+  k_pairs_to_ij<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(p, out, n);
   launched(h, "pairs_to_ij");
 }
 

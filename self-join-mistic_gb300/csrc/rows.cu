@@ -363,11 +363,11 @@ static void sort_rows(mistic_handle_s* h, const unsigned long long* in, size_t n
   launched(h, "row_sort_long");
 }
 
-void sort_pairs_ij(mistic_handle_s* h, unsigned long long* pairs, size_t np, size_t n, const uint32_t* row0,
-                   uint32_t n_inst) {
+void sort_pairs_ij(mistic_handle_s* h, const unsigned long long* pairs, unsigned long long* out, size_t np, size_t n,
+                   const uint32_t* row0, uint32_t n_inst) {
   if (np == 0) return;
   RowOut R{};
-  R.pairs = pairs;
+  R.pairs = out;
   R.row0 = row0;
   R.n_inst = n_inst;
   sort_rows(h, pairs, np, n, R);
