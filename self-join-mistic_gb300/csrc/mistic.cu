@@ -447,18 +447,21 @@ int tc_precision(mistic_mode mode, uint32_t d, double eps2, double R) {
   return E <= 0.1 * eps2 ? 1 : 0;
 }
 
-// Rows of 32 < d <= 126 on the K-chunked kernel too, when its globally
+// Rows of 30 < d <= 126 on the K-chunked kernel too, when its globally
 // centred bound keeps the band narrow: split-bf16 error for the widest
 // columns (rows at the largest norm R) at most eps^2 / 100.  The short-row
 // kernel centres each unit on its first row, which keeps the bound small
 // whatever the coordinates, but converts every candidate tile on its CUDA
 // cores; the K-chunked kernel reads rows prepared once.  On the 515k x 90
 // workload (eps^2 = 50, R ~ 15) the short-row kernel was latency-bound on
-// that conversion (issue 28 %, tensor pipe 14 %, 237 ms).  MISTIC_TC_WIDE=0/1
+// that conversion (issue 28 %, tensor pipe 14 %, 237 ms).  d = 31 and 32 pad
+// to K = 48 in the short-row kernel (149,401 x 32: 9.9 against 6.4 ms a call);
+// from d = 30 down its K is 32 and it is the faster one (150,000 x 24: 4.4
+// against 4.7 ms; 100,000 x 18: 3.1 against 3.4).  MISTIC_TC_WIDE=0/1
 // overrides.
 bool tcw_for_medium_rows(uint32_t d, double eps2, double R) {
   if (const char* e = getenv("MISTIC_TC_WIDE")) return *e == '1';
-  if (d <= 32) return false;
+  if (d <= 30) return false;
   const double u = ldexp(1.0, -24);
   const double rs = 2.0 * R, Dp = 1.1 * sqrt(eps2);
   const double delta = 2.0 * u * R + u * rs;
