@@ -105,6 +105,20 @@ __device__ __forceinline__ void stage_flush(PairStage& ps, unsigned long long* c
   ps.n = 0;
 }
 
+// Warp-collective: adds the pair of every lane with `has` (at most one a lane).
+__device__ __forceinline__ void stage_one(PairStage& ps, bool has, unsigned long long pair, unsigned long long* counter,
+                                          unsigned long long* pairs, unsigned long long cap,
+                                          unsigned long long* inst_pairs, uint32_t inst, const RingCtx* rc) {
+  const uint32_t m = __ballot_sync(FULL_MASK, has);
+  if (!m) return;
+  const uint32_t total = __popc(m);
+  if (ps.n + total > PSTAGE || (ps.n && ps.inst != inst)) stage_flush(ps, counter, pairs, cap, inst_pairs, rc);
+  ps.inst = inst;
+  if (has && pairs) ps.buf[ps.n + __popc(m & ((1u << (threadIdx.x & 31)) - 1u))] = ps.ij ? pair_ij(pair) : pair;
+  __syncwarp();
+  ps.n += total;
+}
+
 // Warp-collective: adds this lane's `cnt` pairs, produced in order by
 // `pair_of(k)` for k = 0..cnt-1 (packed (i << 32 | j), i < j), of instance
 // `inst` (warp-uniform; 0 outside fused batch joins).

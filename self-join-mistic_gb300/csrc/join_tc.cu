@@ -29,12 +29,11 @@
 // 0.1 eps2 are re-decided entirely in FP64 (T_lo = -1, T_hi = inf).
 //
 // Data movement: operands are converted from the sorted FP32 rows into the
-// no-swizzle K-major core-matrix layout (8 rows x 16 bytes per core matrix;
-// LBO = 128 B between K-adjacent core matrices, SBO = 16*KP B between 8-row
-// groups), one elected thread issues the MMAs and commits to an mbarrier,
-// and the epilogue warps read each 128 x 128 FP32 accumulator back with
-// tcgen05.ld.  Every mbarrier wait is bounded; on expiry the CTA records an
-// error, stops, drains its MMAs and releases its tensor memory.
+// K-major layouts of chunk_off (tc_common.cuh), elected threads issue the MMAs
+// and commit to mbarriers, and the epilogue warps read each 128 x 128 FP32
+// accumulator back with tcgen05.ld.  Every mbarrier wait is bounded; on expiry
+// the CTA records an error, stops, drains its MMAs and releases its tensor
+// memory.
 #include <cuda_bf16.h>
 #include <math.h>
 
@@ -56,52 +55,85 @@ constexpr int TN = 128;          // candidate columns per tile (MMA N)
 constexpr int WIN = 256;         // neighbour bins per candidate window
 
 // ---------------------------------------------------------------- pipeline
-// One persistent CTA per SM: 8 producer warps, NEPI epilogue warps, 1 MMA warp.
-//   producers  fetch units; stage the unit's home rows (A: G chunks of 128,
-//              once per unit) and each tile's 128 candidate rows (B) in an
-//              NS-stage ring, two threads per row: raw FP32 rows arrive by
-//              cp.async (in a RAW-slot landing ring, or in the B stage
-//              itself) and are converted in place into bf16 hi/lo with the
-//              per-column threshold folded into B (column d+1 holds
-//              |q'|^2 - T(n)); up to LA tiles are in flight;
-//   MMA warp   one lane issues 3 * KP/16 tcgen05.mma per (tile, home chunk)
-//              into the next of NACC = 4 TMEM accumulators and commits;
-//   epilogue   tcgen05.ld of TMEM lane quarter w % 4, sign-bit test (D' < 0
-//              marks a candidate), home-bin rule by column range, sure
-//              accepts to the pair list, the error band to the band list.
+// One persistent CTA per SM: 8 producer warps, NEPI epilogue warps, 2 MMA warps.
+//   producers  K <= 32: 4 loader warps claim units, walk their neighbour bins
+//              and copy each tile's 128 candidate rows (raw FP32, cp.async)
+//              into a ring of RAW landing slots; 4 converter warps, a thread
+//              a row, turn a slot into the bf16 hi/lo operand rows of one of
+//              the NS B stages, with the per-column threshold folded in
+//              (column d+1 holds |q'|^2 - T(n)), and stage each unit's home
+//              rows (A: G chunks of 128).  A stage's operands go back when its
+//              MMAs are done; what the epilogue needs of it sits in a ring of
+//              its own.  K >= 48: all 8 warps do both, two
+//              threads a row, the raw rows landing in the B stages
+//              themselves where no separate slots fit;
+//   MMA warps  one lane of each issues 3 * KP/16 tcgen05.mma per (tile, home
+//              chunk) into the next of NACC = 4 TMEM accumulators and commits,
+//              the two warps taking turns: at K = 32 a lane spends about 490
+//              cycles an accumulator issuing its MMAs and half as much again
+//              on waits, metadata and commits;
+//   epilogue   groups of 4 warps, one per TMEM lane quarter, each group with
+//              its own accumulators: tcgen05.ld, sign-bit test (D' < 0 marks
+//              a candidate), home-bin rule by column range, sure accepts to
+//              the pair list, the error band to the band list.
 // Barriers (all waits bounded by a %globaltimer deadline):
-//   full[s]   producers -> MMA        (NPROD arrivals)
-//   sfree[s]  epilogue  -> producers  (NEPI arrivals after the tile's last home chunk)
-//   dfull[b]  MMA       -> epilogue   (tcgen05.commit, or a plain arrive on the terminate tile)
-//   dfree[b]  epilogue  -> MMA        (NEPI arrivals; accumulator b reusable)
-//   afull     producers -> MMA        (NPROD arrivals per unit: A written)
-//   afree     MMA       -> producers  (tcgen05.commit after a unit's last tile)
+//   rawfull[r] loaders    -> converters (each loader thread's copies landed, + 1 for the slot's metadata)
+//   rawfree[r] converters -> loaders    (4 arrivals: slot read)
+//   ubar       converters among themselves, twice a unit (128 arrivals)
+//   full[s]    producers  -> MMA        (128 arrivals, or NPROD)
+//   bfree[s]   MMA        -> converters (a tcgen05.commit by each MMA warp: stage s read)
+//   mfree[m]   epilogue   -> producers  (metadata slot m, and with it the stage of K >= 48; 48 arrivals: 12 / home
+//                                        chunks by each of a group's 4 warps)
+//   dfull[b]   MMA        -> epilogue   (tcgen05.commit, + 1 for the accumulator's metadata)
+//   dfree[b]   epilogue   -> MMA        (4 arrivals; accumulator b reusable)
+//   afull      producers  -> MMA        (128 arrivals, or NPROD, per unit: A written)
+//   afree      MMA        -> producers  (a tcgen05.commit by each MMA warp after a unit's last tile)
 constexpr int NPW = 8;     // producer warps: two threads per operand row
 constexpr int NPROD = NPW * 32;
-// NEPI epilogue warps (a template parameter: 8 or 16) cover the 4 TMEM lane
-// quarters x NEPI / 4 column-block groups; the MMA warp follows them.
+constexpr int NLOAD = 128; // K <= 32: threads of the loader warps, and of the converter warps after them
+constexpr int NUNIT = 8;   // unit slots between them (at most RAW = 4 units have tiles in flight)
+// NEPI epilogue warps (a template parameter: 8 or 16) in groups of 4; the MMA
+// warps follow them.
 constexpr int EPI0 = NPW;  // first epilogue warp (a multiple of 4: warp % 4 is its lane quarter)
-__host__ __device__ constexpr int tc_threads(int nepi) { return (EPI0 + nepi + 1) * 32; }
+constexpr int NMMA = 2;    // MMA warps
+__host__ __device__ constexpr int tc_threads(int nepi) { return (EPI0 + nepi + NMMA) * 32; }
 constexpr int NACC = 4;    // TMEM accumulators of 128 columns (512 per CTA, one CTA per SM)
 constexpr uint32_t FLAG_FIRST = 1, FLAG_LAST = 2, FLAG_END = 4;
 
-struct TileMeta {
-  uint32_t a0, na, ncols, flags, ng;  // ng: 128-row MMA tiles of this unit (1..G)
+struct __align__(16) TileMeta {
+  uint32_t a0, na, flags, ng;  // ng: 128-row MMA tiles of this unit (1..G)
+  uint32_t inst;               // instance of the unit (fused batch joins; else 0)
+  uint32_t ncols;
   uint32_t hcr, hq;  // columns [hcr & 255, hcr >> 8) hold home-bin rows, the first at sorted position hq
-  uint32_t inst;     // instance of the unit (fused batch joins; else 0)
+};
+
+// What the converters need about a unit, written by a loader.
+struct TcUnit {
+  const float* X;   // the instance's sorted rows
+  uint32_t a0, na, ng, inst;
+  TcBound tb;
+};
+
+// A raw slot's tile.
+struct TcSlot {
+  uint32_t ncols, flags, hcr, hq, unit;  // unit: index into TcShared2::units
+};
+
+// What an accumulator holds: home chunk g of the tile with metadata slot ms.
+struct __align__(16) TcAcc {
+  uint32_t ms, g, end;
 };
 
 template <int NS, int G, int RAW>
 struct TcShared2 {
+  static constexpr int NM = NS;  // metadata slots
   __align__(16) float cadd_a[128];  // -c   (A rows: x - c)
   __align__(16) float cadd_b[128];  // 2c   (B rows: -2 (x - c))
   uint32_t w_home;  // (window generation << 8) | index of the home bin in the window
   uint32_t hx[4][2];  // home column range of issued tiles (producer thread 0 only)
-  uint32_t qid[NS][TN];      // original row ids of the candidates
-  uint32_t aid[NS][TM * G];  // original row ids of the home rows (per stage: the epilogue
-                             // may still read a finished unit while producers start the next)
-  float dlt[NS][TN];  // accept when D' <= -dlt
-  TileMeta meta[NS];
+  uint32_t qid[NM][TN];  // original row ids of the candidates
+  __align__(16) float dlt[NM][TN];  // accept when D' < -dlt
+  TileMeta meta[NM];
   uint32_t rid[RAW > 0 ? RAW : 1][TN];  // candidate ids of the tiles in the raw ring
   uint32_t w_start[WIN];
   uint32_t w_pref[WIN + 1];
@@ -109,20 +141,44 @@ struct TcShared2 {
   unsigned long long unit;
   uint32_t w_total, w_pos, seg_next, w_nb;
   uint32_t ra2max;  // float bits, non-negative
+  float cadd[2][2][RAW == 4 ? 32 : 1];  // K <= 32: [unit parity][A, B] as cadd_a, cadd_b
+  uint32_t ra2[4];                      // K <= 32: largest |a|^2 by unit mod 4, float bits
+  TcUnit units[RAW == 4 ? NUNIT : 1];
+  TcSlot slot[RAW == 4 ? RAW : 1];
+  TcAcc acc[NACC];
   uint32_t abort_flag;
   uint32_t tmem_base;
   uint32_t pflag[2];  // producer-wide decisions, written by producer thread 0
   // [tile parity][K-block parity][row]: partial row norms of the two threads
-  // of a row (two-threads-a-row mode only; pair mode has one thread a row)
+  // of a row (K >= 48)
   float npart[RAW == 4 ? 1 : 2][2][RAW == 4 ? 1 : TM];
-  unsigned long long full[NS], sfree[NS], dfull[NACC], dfree[NACC], afull, afree;
+  unsigned long long full[NS], bfree[NS], mfree[NM], dfull[NACC], dfree[NACC], afull, afree;
+  unsigned long long rawfull[RAW > 0 ? RAW : 1], rawfree[RAW > 0 ? RAW : 1], ubar;
 };
+
+// Barrier of the loader warps that also returns the AND of p over them.
+__device__ __forceinline__ bool load_sync_and(bool p) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred pi, po;\n\t"
+      "setp.ne.u32 pi, %1, 0;\n\t"
+      "bar.red.and.pred po, 2, %2, pi;\n\t"
+      "selp.u32 %0, 1, 0, po;\n\t}"
+      : "=r"(r)
+      : "r"((uint32_t)p), "n"(NLOAD)
+      : "memory");
+  return r != 0u;
+}
+
+// This thread's arrival on `bar` once every cp.async it issued before has landed.
+__device__ __forceinline__ void cp_async_arrive(unsigned long long* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 
 __device__ __forceinline__ void prod_sync() { asm volatile("bar.sync 1, %0;" ::"n"(NPROD) : "memory"); }
 
-// Operand rows live in the no-swizzle K-major core-matrix layout: the
-// 16-byte chunk of row r and K block kb (8 bf16) sits at bf16 offset
-// chunk_off(r, kb).  A raw FP32 row is first copied (cp.async) into the
+// Operand rows live in the layout of chunk_off: the 16-byte chunk of row r and
+// K block kb (8 bf16) sits at bf16 offset chunk_off(r, kb).  A raw FP32 row is first copied (cp.async) into the
 // chunk slots of the row itself -- floats [8kb, 8kb+4) into the hi chunk of
 // block kb, [8kb+4, 8kb+8) into its lo chunk -- and then converted in place,
 // block by block, into the augmented bf16 hi/lo row.  Two threads share a
@@ -218,8 +274,8 @@ __device__ __forceinline__ float conv_pass1(const __nv_bfloat16* sh, const __nv_
   return acc;
 }
 
-// Whole-row forms for one thread a row (pair mode): the raw row's chunks
-// land in the row's own slots as in load_half, every K block of the row.
+// Whole-row forms for one thread a row (K <= 32): the raw row's chunks land in
+// the row's own slots as in load_half, every K block of the row.
 template <int KP>
 __device__ __forceinline__ void load_row(__nv_bfloat16* hi, __nv_bfloat16* lo, uint32_t r,
                                          const float* __restrict__ xr, uint32_t dpad) {
@@ -231,20 +287,20 @@ __device__ __forceinline__ void load_row(__nv_bfloat16* hi, __nv_bfloat16* lo, u
   }
 }
 
-// Converts row r from the raw chunks (sh, sl) into the bf16 hi/lo operand row
-// (hi, lo), K blocks in order, with placeholders pd, pd1 in the augmented
-// columns d and d + 1; returns the row norm |x - c|^2 (times scale^2).
-template <int KP>
-__device__ __forceinline__ float conv_row(const __nv_bfloat16* sh, const __nv_bfloat16* sl, __nv_bfloat16* hi,
-                                          __nv_bfloat16* lo, uint32_t r, const float* cadd, float scale, uint32_t d,
-                                          float pd, float pd1) {
+// Converts row r, its 8-float blocks given by block(kb, x), into the bf16
+// hi/lo operand row (hi, lo), K blocks in order, with placeholders pd, pd1 in
+// the augmented columns d and d + 1; returns the row norm |x - c|^2 (times
+// scale^2).
+template <int KP, class Block>
+__device__ __forceinline__ float conv_row(Block block, __nv_bfloat16* hi, __nv_bfloat16* lo, uint32_t r,
+                                          const float* cadd, float scale, uint32_t d, float pd, float pd1) {
   float acc = 0.f;
 #pragma unroll
   for (int kb = 0; kb < KP / 8; ++kb) {
     const uint32_t k0 = 8 * kb, off = chunk_off<KP>(r, kb);
     if (k0 >= d + 2) break;  // zero blocks (cleared at the start)
     float x[8], v[8];
-    unpack8(sh, sl, off, k0 < d, k0 + 4 < d, x);
+    block(kb, x);
     if (k0 + 8 <= d) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -283,10 +339,13 @@ __device__ __forceinline__ void patch_col(__nv_bfloat16* hi, __nv_bfloat16* lo, 
 
 template <int KP, int NS, int G, int RAW, int NEPI>
 __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParams P, const TcParams T) {
-  constexpr int MMA_WARP = EPI0 + NEPI;
-  extern __shared__ __align__(128) unsigned char tc_dyn[];
-  __shared__ TcShared2<NS, G, RAW> S;
-  constexpr uint32_t OPB = TM * KP;  // bf16 elements per operand buffer
+  constexpr int MMA_WARP = EPI0 + NEPI;  // the first of NMMA
+  extern __shared__ __align__(128) unsigned char tc_raw[];
+  using Shared = TcShared2<NS, G, RAW>;
+  __shared__ Shared S;
+  constexpr int NM = Shared::NM;
+  constexpr uint32_t OPB = TM * KP;  // bf16 elements per 128-row operand buffer
+  unsigned char* tc_dyn = tc_raw + ((512u - (smem_u32(tc_raw) & 511u)) & 511u);  // swizzle atoms: 512 bytes
   __nv_bfloat16* Ahi = reinterpret_cast<__nv_bfloat16*>(tc_dyn);  // G home chunks of 128 rows
   __nv_bfloat16* Alo = Ahi + G * OPB;
   __nv_bfloat16* Bhi = Alo + G * OPB;  // NS stages of hi, then NS stages of lo
@@ -298,15 +357,24 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
 
   if (tid == 0) {
     for (int i = 0; i < NS; ++i) {
-      mbar_init(&S.full[i], RAW == 4 ? TM : NPROD);  // pair mode: one group of 128 a tile
-      mbar_init(&S.sfree[i], NEPI);
+      mbar_init(&S.full[i], RAW == 4 ? NLOAD : NPROD);
+      mbar_init(&S.bfree[i], NMMA);
     }
+    for (int i = 0; i < NM; ++i) mbar_init(&S.mfree[i], 48);
     for (int i = 0; i < NACC; ++i) {
-      mbar_init(&S.dfull[i], 1);
-      mbar_init(&S.dfree[i], NEPI);
+      mbar_init(&S.dfull[i], 2);
+      mbar_init(&S.dfree[i], 4);
     }
-    mbar_init(&S.afull, NPROD);
-    mbar_init(&S.afree, 1);
+    mbar_init(&S.afull, RAW == 4 ? NLOAD : NPROD);
+    mbar_init(&S.afree, NMMA);
+    if (RAW == 4) {
+      for (int i = 0; i < RAW; ++i) {
+        mbar_init(&S.rawfull[i], NLOAD + 1);
+        mbar_init(&S.rawfree[i], 4);
+      }
+      mbar_init(&S.ubar, NLOAD);
+      for (int i = 0; i < 4; ++i) S.ra2[i] = 0;
+    }
     asm volatile("fence.mbarrier_init.release.cluster;");
     S.abort_flag = 0;
     S.w_home = 0xffffffffu;
@@ -328,318 +396,262 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
 
   if (warp < NPW) {
     if constexpr (RAW == 4) {
-    // ============================ producers, pair mode (K <= 32, four raw slots)
-    // The 256 producer threads are two groups of 128; thread (grp, pr)
-    // converts the whole row pr of one candidate tile, group grp of each
-    // pair of consecutive tiles, so a row needs no exchange and its fixed
-    // costs (finding its source row, issuing its copies, its threshold and
-    // metadata) are paid once.  Pairs never span a window of neighbour bins:
-    // when fewer than 129 candidate ranks are left in it, the pair is one
-    // tile and group 1 idles.  Two pairs are in flight, the one being
-    // converted and the next (one raw slot a tile).  Branches that lead to bar.sync depend only on values every
-    // producer thread holds or reads after the same bar.sync; barrier waits
-    // are done by thread 0 and broadcast through S.pflag.
-    const uint32_t pr = (uint32_t)tid & 127u, grp = (uint32_t)tid >> 7;
-    uint32_t tile = 0, issued = 0, unit_k = 0, pf = 0;
-    unsigned long long n_tiles = 0, n_cells = 0;
-    long long pw_sfree = 0, pc_unit = 0, pc_win = 0, pc_conv = 0, pc_ldw = 0;
-    long long pc_adv = 0, pc_bar = 0, pc_p1 = 0, pc_p2 = 0, pc_fin = 0;
-    uint32_t wgen = 0;
-    const long long p_start = T.prof ? clock64() : 0;
-    auto end_marker = [&]() {  // next tile slot: tells the MMA warp and the epilogue to stop
-      const uint32_t st = tile % NS;
-      if (tid == 0) {
-        wait_or_abort(&S.sfree[st], ((tile / NS) & 1) ^ 1, abort_flag, T.wait_limit);
-        S.meta[st].flags = FLAG_END;
-      }
-      prod_sync();
-      if (grp == 0) mbar_arrive(&S.full[st]);
-    };
-    for (;;) {
-      const long long cu0 = T.prof ? clock64() : 0;
-      const uint32_t slot = pf++ & 1;
-      if (tid == 0) {
-        const unsigned long long t = atomicAdd(&T.ctr->next_unit, 1ull);
-        const unsigned long long uu = t < T.n_def_in ? (unsigned long long)T.def_in[t] : T.main_start + (t - T.n_def_in);
-        S.unit = uu;
-        bool go = (T.claim_cap == 0 || t < T.claim_cap) && uu < T.n_units && !*abort_flag;
-        if (go && P.ring && *(volatile unsigned long long*)&P.ctr->stop) {
-          const RingCtx rc{P.pair_tags, P.deferred, P.def_out, &P.ctr->def_n, &P.ctr->stop};
-          ring_defer(&rc, P.tag_base_tc + (uint32_t)uu);
-          go = false;
-        }
-        if (go && unit_k > 0) go = wait_or_abort(&S.afree, (unit_k - 1) & 1, abort_flag, T.wait_limit);
-        S.pflag[slot] = go ? 1u : 0u;
-      }
-      prod_sync();
-      if (!S.pflag[slot]) {
-        end_marker();
-        break;
-      }
-      const unsigned long long u = S.unit;
-      const Unit U = T.units[u];
-      const float* X = (const float*)P.xs;
-      const uint32_t *bstart = P.bstart, *nbr = P.nbr, *ids = P.ids;
-      TcBound tb = T.b;
-      uint32_t inst = 0;
-      if (T.unit_inst) {
-        inst = T.unit_inst[u];
-        const InstDesc& I = P.insts[inst];
-        X = (const float*)I.xs;
-        bstart = I.bstart;
-        nbr = I.nbr;
-        ids = I.ids;
-        tb = I.tcb;
-      }
-      if (P.ring) inst = P.tag_base_tc + (uint32_t)u;
-      const uint32_t hs = bstart[U.h], he = bstart[U.h + 1];
-      const uint32_t a0 = hs + U.chunk * (TM * G);
-      const uint32_t na = min((uint32_t)(TM * G), he - a0);
-      const uint32_t ng = (na + TM - 1) / TM;
-      if (tid < (int)P.dpad) {
-        const float c = X[(size_t)a0 * P.dpad + tid];
-        S.cadd_a[tid] = -c;
-        S.cadd_b[tid] = 2.f * c;
-      }
-      if (tid == 0) S.ra2max = 0;
-      prod_sync();
-      uint32_t my_aid[G];  // original ids of home rows g * TM + pr
-#pragma unroll
-      for (int g = 0; g < G; ++g) {
-        const uint32_t r = g * TM + pr;
-        my_aid[g] = r < na ? ids[a0 + r] : 0u;
-      }
-      {  // home rows r = tid + 256 i, whole rows
-        constexpr int HR = (G * TM + NPROD - 1) / NPROD;
-#pragma unroll
-        for (int i = 0; i < HR; ++i) {
-          const uint32_t r = (uint32_t)tid + NPROD * i;
-          if (r < na)
-            load_row<KP>(Ahi + (r / TM) * OPB, Alo + (r / TM) * OPB, r % TM, X + (size_t)(a0 + r) * P.dpad, P.dpad);
-        }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        float m = 0.f;
-#pragma unroll
-        for (int i = 0; i < HR; ++i) {
-          const uint32_t r = (uint32_t)tid + NPROD * i;
-          if (r < na) {
-            __nv_bfloat16 *ah = Ahi + (r / TM) * OPB, *al = Alo + (r / TM) * OPB;
-            const float nrm = conv_row<KP>(ah, al, ah, al, r % TM, S.cadd_a, 1.f, P.d, 0.f, 1.f);
-            patch_col<KP>(ah, al, r % TM, P.d, nrm);
-            m = fmaxf(m, nrm);
+    if (tid < NLOAD) {
+      // ============================ loaders (K <= 32)
+      // Thread t copies row t of every candidate tile.  The warps meet only to
+      // claim a unit and to fill a window of neighbour bins; between those a
+      // warp waits for its slots alone, so up to RAW tiles of copies are in
+      // flight while the converters work.  A failed wait (abort) is carried in
+      // `ok` to the next meeting, where all warps leave together.
+      const uint32_t t = (uint32_t)tid;
+      uint32_t k = 0, useq = 0, wgen = 0;  // tiles, units and windows so far
+      bool ok = true;
+      for (;;) {
+        if (t == 0) {
+          // claim index -> unit: units deferred by the last ring pass first,
+          // then the list from main_start (the identity outside ring mode)
+          const unsigned long long c = atomicAdd(&T.ctr->next_unit, 1ull);
+          const unsigned long long uu =
+              c < T.n_def_in ? (unsigned long long)T.def_in[c] : T.main_start + (c - T.n_def_in);
+          S.unit = uu;
+          bool go = (T.claim_cap == 0 || c < T.claim_cap) && uu < T.n_units && !*abort_flag;
+          if (go && P.ring && *(volatile unsigned long long*)&P.ctr->stop) {  // the ring filled: leave it for the next pass
+            const RingCtx rc{P.pair_tags, P.deferred, P.def_out, &P.ctr->def_n, &P.ctr->stop};
+            ring_defer(&rc, P.tag_base_tc + (uint32_t)uu);
+            go = false;
           }
+          ok = ok && go;
         }
+        if (!load_sync_and(ok)) break;
+        const unsigned long long u = S.unit;
+        const Unit U = T.units[u];
+        // the unit's instance: its arrays and bound constants (fused batch
+        // joins), or the launch's own
+        const float* X = (const float*)P.xs;
+        const uint32_t *bstart = P.bstart, *nbr = P.nbr, *ids = P.ids;
+        uint32_t inst = 0;
+        if (T.unit_inst) {
+          inst = T.unit_inst[u];
+          const InstDesc& I = P.insts[inst];
+          X = (const float*)I.xs;
+          bstart = I.bstart;
+          nbr = I.nbr;
+          ids = I.ids;
+        }
+        const uint32_t hs = bstart[U.h], he = bstart[U.h + 1];
+        const uint32_t a0 = hs + U.chunk * (TM * G);
+        const uint32_t na = min((uint32_t)(TM * G), he - a0);
+        // the converters read the home rows when they reach the unit
+        for (uint32_t r = t; r < na; r += NLOAD)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(X + (size_t)(a0 + r) * P.dpad));
+        if (t == 0) {
+          TcUnit& W = S.units[useq % NUNIT];
+          W.X = X;
+          W.a0 = a0;
+          W.na = na;
+          W.ng = (na + TM - 1) / TM;
+          W.inst = P.ring ? P.tag_base_tc + (uint32_t)u : inst;  // the ring's tag of this unit's pairs
+          W.tb = T.unit_inst ? P.insts[inst].tcb : T.b;
+        }
+        uint32_t flags = FLAG_FIRST;
+        for (uint32_t seg = U.s0; seg < U.s1; seg += WIN) {
+          // ---- window of up to WIN neighbour bins, two a thread
+          const uint32_t nb = min((uint32_t)WIN, U.s1 - seg);
+          uint32_t st[2] = {0, 0}, sz[2] = {0, 0}, bn[2] = {0xffffffffu, 0xffffffffu};
 #pragma unroll
-        for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(FULL_MASK, m, o));
-        if (lane == 0) atomicMax(&S.ra2max, __float_as_uint(m));
-      }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      mbar_arrive(&S.afull);
-      prod_sync();
-      const float ra2max = __uint_as_float(S.ra2max);
-      if (T.prof) pc_unit += clock64() - cu0;
-
-      // ---- candidate pairs of tiles of this unit
-      uint32_t seg_next = U.s0, w_nb = 0, w_pos = 0, w_total = 0;
-      unsigned long long pq = 0;  // per pair in flight: colsA | lastA << 8 | colsB << 9 | lastB << 17
-      uint32_t pin = 0;           // pairs in flight
-      int w_hj = -1;
-      auto home_cols = [&](uint32_t pos, uint32_t ncols, uint32_t* hcr, uint32_t* hq) {
-        *hcr = 0;
-        *hq = 0;
-        if (w_hj >= 0 && ncols > 0) {
-          const uint32_t hr0 = S.w_pref[w_hj], hr1 = S.w_pref[w_hj + 1];
-          if (max(hr0, pos) < min(hr1, pos + ncols)) {
-            const uint32_t lo = max(hr0, pos) - pos, hi = min(hr1, pos + ncols) - pos;
-            *hcr = lo | (hi << 8);
-            *hq = S.w_start[w_hj] + (pos + lo - hr0);
-          }
-        }
-      };
-      // issues the next pair: returns 1, or 2 on abort
-      auto advance = [&]() -> int {
-        while (w_pos >= w_total) {
-          const long long cw0 = T.prof ? clock64() : 0;
-          const uint32_t nb = min((uint32_t)WIN, U.s1 - seg_next);
-          uint32_t st0 = 0, sz0 = 0, bn = 0xffffffffu;
-          if ((uint32_t)tid < nb) unit_bin(U, TM * G, nbr, bstart, seg_next + tid, &bn, &st0, &sz0);
-          const uint32_t incl = warp_scan_incl(sz0);
+          for (int q = 0; q < 2; ++q)
+            if (2 * t + q < nb) unit_bin(U, TM * G, nbr, bstart, seg + 2 * t + q, &bn[q], &st[q], &sz[q]);
+          const uint32_t incl = warp_scan_incl(sz[0] + sz[1]);
           if (lane == 31) S.scan_ws[warp] = incl;
-          prod_sync();
+          ok = load_sync_and(ok);  // also: every warp is done with the window before
+          if (!ok) break;
           uint32_t wp = 0;
           for (int w = 0; w < warp; ++w) wp += S.scan_ws[w];
           ++wgen;
-          if ((uint32_t)tid < nb) {
-            S.w_start[tid] = st0;
-            S.w_pref[tid + 1] = wp + incl;
-            if (bn == U.h) S.w_home = ((wgen & 0xffffffu) << 8) | (uint32_t)tid;
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            if (2 * t + q < nb) {
+              S.w_start[2 * t + q] = st[q];
+              S.w_pref[2 * t + q + 1] = wp + incl - (q == 0 ? sz[1] : 0u);
+              if (bn[q] == U.h) S.w_home = ((wgen & 0xffffffu) << 8) | (2 * t + q);
+            }
           }
-          if (tid == 0) S.w_pref[0] = 0;
-          prod_sync();
-          {
-            const uint32_t wh = S.w_home;
-            w_hj = (wh >> 8) == (wgen & 0xffffffu) ? (int)(wh & 255u) : -1;
+          if (t == 0) S.w_pref[0] = 0;
+          ok = load_sync_and(ok);
+          if (!ok) break;
+          const uint32_t wh = S.w_home, total = S.w_pref[nb];
+          const int w_hj = (wh >> 8) == (wgen & 0xffffffu) ? (int)(wh & 255u) : -1;
+          for (uint32_t pos = 0; pos < total; pos += TN, ++k) {
+            const uint32_t ncols = min((uint32_t)TN, total - pos);
+            if (pos + TN >= total && seg + nb >= U.s1) flags |= FLAG_LAST;
+            // row of candidate rank pos + t: the warp finds the bin of its
+            // first rank (two 32-way probes of the window prefix), then each
+            // lane counts the bin boundaries among the next 32 ranks
+            uint32_t q = 0xffffffffu;
+            {
+              const uint32_t r0 = pos + (t & ~31u);
+              const uint32_t step = (nb + 31) >> 5;
+              const uint32_t c = __popc(__ballot_sync(FULL_MASK, lane * step < nb && S.w_pref[lane * step] <= r0));
+              const uint32_t base = (c - 1) * step;  // w_pref[0] = 0 <= r0, so c >= 1
+              const uint32_t b0 =
+                  base + __popc(__ballot_sync(FULL_MASK, (uint32_t)lane < step && base + lane < nb &&
+                                                             S.w_pref[base + lane] <= r0)) - 1;
+              const uint32_t e = b0 + 1 + lane;  // boundary after bin b0 + lane
+              const uint32_t tt = e <= nb ? S.w_pref[e] - r0 : 32u;
+              const uint32_t bounds = __reduce_or_sync(FULL_MASK, tt < 32u ? 1u << tt : 0u);
+              if (t < ncols) {
+                const uint32_t b = b0 + __popc(bounds & ((2u << lane) - 1u));
+                q = S.w_start[b] + (r0 + lane - S.w_pref[b]);
+              }
+            }
+            const uint32_t rs = k % RAW;
+            ok = ok && wait_or_abort(&S.rawfree[rs], ((k / RAW) & 1) ^ 1, abort_flag, T.wait_limit);
+            if (ok && t < ncols) {
+              __nv_bfloat16* dh = Raw + rs * 2 * OPB;
+              asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(&S.rid[rs][t])), "l"(ids + q)
+                           : "memory");
+              load_row<KP>(dh, dh + OPB, t, X + (size_t)q * P.dpad, P.dpad);
+            }
+            cp_async_arrive(&S.rawfull[rs]);
+            if (t == 0) {
+              uint32_t hcr = 0, hq = 0;
+              if (w_hj >= 0) {
+                const uint32_t hr0 = S.w_pref[w_hj], hr1 = S.w_pref[w_hj + 1];
+                const uint32_t lo = max(hr0, pos), hi = min(hr1, pos + ncols);
+                if (lo < hi) {
+                  hcr = (lo - pos) | ((hi - pos) << 8);
+                  hq = S.w_start[w_hj] + (lo - hr0);
+                }
+              }
+              if (ok) S.slot[rs] = TcSlot{ncols, flags, hcr, hq, useq % NUNIT};
+              mbar_arrive(&S.rawfull[rs]);
+            }
+            flags = 0;
           }
-          w_nb = nb;
-          w_pos = 0;
-          w_total = S.w_pref[nb];
-          seg_next += nb;
-          if (T.prof) pc_win += clock64() - cw0;
         }
-        const long long ca0 = T.prof ? clock64() : 0;
-        const uint32_t left = w_total - w_pos;
-        const uint32_t colsA = min((uint32_t)TN, left);
-        const uint32_t colsB = left > (uint32_t)TN ? min((uint32_t)TN, left - TN) : 0u;
-        const bool more = seg_next < U.s1;  // further windows after this one
-        const bool lastA = colsB == 0 && left <= (uint32_t)TN && !more;
-        const bool lastB = colsB > 0 && left <= 2u * TN && !more;
-        const uint32_t mycols = grp ? colsB : colsA;
-        // row of candidate rank w_pos + tid (warp-wide probes of the window prefix)
-        uint32_t q = 0xffffffffu;
+        ++useq;
+      }
+      // stop marker: the next slot, with no rows
+      const uint32_t rs = k % RAW;
+      ok = wait_or_abort(&S.rawfree[rs], ((k / RAW) & 1) ^ 1, abort_flag, T.wait_limit);
+      if (t == 0) {
+        if (ok) S.slot[rs].flags = FLAG_END;
+        mbar_arrive(&S.rawfull[rs]);
+      }
+      cp_async_arrive(&S.rawfull[rs]);
+      asm volatile("cp.async.wait_all;" ::: "memory");
+    } else {
+      // ============================ converters (K <= 32): thread c, row c of every tile
+      const uint32_t c = (uint32_t)tid - NLOAD;
+      uint32_t useq = 0;
+      unsigned long long n_tiles = 0, n_cells = 0;
+      uint32_t a0 = 0, na = 0, ng = 0, inst = 0;
+      TcBound tb = T.b;
+      float ra2max = 0.f;
+      long long pw_sfree = 0, pw_raw = 0;
+      const long long p_start = T.prof ? clock64() : 0;
+      for (uint32_t tile = 0;; ++tile) {
+        const uint32_t rs = tile % RAW, st = tile % NS, ms = tile % NM;
+        const long long c0 = T.prof ? clock64() : 0;
+        if (!__all_sync(FULL_MASK, wait_or_abort(&S.rawfull[rs], (tile / RAW) & 1, abort_flag, T.wait_limit))) break;
+        const long long c1 = T.prof ? clock64() : 0;
+        const TcSlot L = S.slot[rs];
+        // the stage and metadata slot this tile goes to
         {
-          const uint32_t r0 = w_pos + ((uint32_t)tid & ~31u);
-          const uint32_t step = (w_nb + 31) >> 5;
-          const uint32_t c = __popc(__ballot_sync(FULL_MASK, lane * step < w_nb && S.w_pref[lane * step] <= r0));
-          const uint32_t base = (c - 1) * step;
-          const uint32_t b0 =
-              base + __popc(__ballot_sync(FULL_MASK, (uint32_t)lane < step && base + lane < w_nb &&
-                                                         S.w_pref[base + lane] <= r0)) - 1;
-          const uint32_t e = b0 + 1 + lane;
-          const uint32_t t = e <= w_nb ? S.w_pref[e] - r0 : 32u;
-          const uint32_t bounds = __reduce_or_sync(FULL_MASK, t < 32u ? 1u << t : 0u);
-          if (pr < mycols) {
-            const uint32_t b = b0 + __popc(bounds & ((2u << lane) - 1u));
-            q = S.w_start[b] + (r0 + lane - S.w_pref[b]);
-          }
+          const bool ok = wait_or_abort(&S.bfree[st], ((tile / NS) & 1) ^ 1, abort_flag, T.wait_limit) &&
+                          wait_or_abort(&S.mfree[ms], ((tile / NM) & 1) ^ 1, abort_flag, T.wait_limit);
+          if (!__all_sync(FULL_MASK, ok)) break;
         }
-        const uint32_t rs = (issued + grp) % RAW;
-        __nv_bfloat16* dh = Raw + rs * 2 * OPB;
-        __nv_bfloat16* dl = dh + OPB;
-        if (pr < mycols) {
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(&S.rid[rs][pr])), "l"(ids + q)
-                       : "memory");
-          load_row<KP>(dh, dl, pr, X + (size_t)q * P.dpad, P.dpad);
+        if (T.prof) {
+          pw_raw += c1 - c0;
+          pw_sfree += clock64() - c1;
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        if (tid == 0) {
-          uint32_t hcr, hq;
-          home_cols(w_pos, colsA, &hcr, &hq);
-          S.hx[issued & 3][0] = hcr;
-          S.hx[issued & 3][1] = hq;
-          home_cols(w_pos + TN, colsB, &hcr, &hq);
-          S.hx[(issued + 1) & 3][0] = hcr;
-          S.hx[(issued + 1) & 3][1] = hq;
-        }
-        pq |= (unsigned long long)(colsA | (lastA ? 0x100u : 0u) | (colsB << 9) | (lastB ? 0x20000u : 0u))
-              << (18 * pin);
-        ++pin;
-        w_pos += colsB > 0 ? 2u * TN : (uint32_t)TN;
-        issued += colsB > 0 ? 2u : 1u;
-        if (T.prof) pc_adv += clock64() - ca0;
-        return 1;
-      };
-
-      // One pair is in flight ahead of the pair being converted.  The next
-      // pair's copies and home-column entries are issued only after the
-      // barrier that ends every thread's work on the pair before it, whose
-      // raw slots and entries they reuse: a pair of one tile shifts the slots
-      // by one, so the thread that converted a slot is not always the thread
-      // that refills it.
-      bool first = true, aborted = false;
-      if (w_pos < w_total || seg_next < U.s1) advance();
-      for (;;) {
-        if (pin == 0) break;
-        const long long cc0 = T.prof ? clock64() : 0;
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        if (T.prof) pc_ldw += clock64() - cc0;
-        const uint32_t e = (uint32_t)(pq & 0x3ffffull);
-        pq >>= 18;
-        --pin;
-        const uint32_t colsA = e & 0xffu, colsB = (e >> 9) & 0xffu;
-        const bool lastA = (e & 0x100u) != 0u, lastB = (e & 0x20000u) != 0u;
-        const uint32_t nt = colsB > 0 ? 2u : 1u;
-        const long long cb0 = T.prof ? clock64() : 0;
-        const uint32_t fl = pf++ & 1;
-        if (tid == 0) {
-          const long long c0 = T.prof ? clock64() : 0;
-          bool ok = wait_or_abort(&S.sfree[tile % NS], ((tile / NS) & 1) ^ 1, abort_flag, T.wait_limit);
-          if (ok && nt == 2)
-            ok = wait_or_abort(&S.sfree[(tile + 1) % NS], (((tile + 1) / NS) & 1) ^ 1, abort_flag, T.wait_limit);
-          S.pflag[fl] = ok ? 1u : 0u;
-          if (T.prof) pw_sfree += clock64() - c0;
-        }
-        prod_sync();
-        if (T.prof) pc_bar += clock64() - cb0;
-        if (!S.pflag[fl]) {
-          aborted = true;
+        if (L.flags & FLAG_END) {
+          if (c == 0) S.meta[ms].flags = FLAG_END;
+          mbar_arrive(&S.full[st]);
           break;
         }
-        if (w_pos < w_total || seg_next < U.s1) advance();
-        if (grp < nt) {
-          const uint32_t mt = tile + grp;
-          const uint32_t st = mt % NS, rs = mt % RAW;
-          const uint32_t ncols = grp ? colsB : colsA;
-          const bool last = grp ? lastB : lastA;
-          const bool ok = pr < ncols;
-          __nv_bfloat16* bh = Bhi + st * OPB;
-          __nv_bfloat16* bl = Blo + st * OPB;
-          const long long cp0 = T.prof ? clock64() : 0;
-          if (ok) {
-            const __nv_bfloat16* sh = Raw + rs * 2 * OPB;
-            S.qid[st][pr] = S.rid[rs][pr];
-            const float nq2 = conv_row<KP>(sh, sh + OPB, bh, bl, pr, S.cadd_b, -2.f, P.d, 1.f, 0.f) * 0.25f;
-            float tcol = 0.f, dl = 0.f;
-            if (!column_threshold(tb, ra2max, nq2, &tcol, &dl)) {
-              tcol = 1e30f;   // every row of this column becomes a candidate ...
-              dl = INFINITY;  // ... and none is accepted without the FP64 check
-            }
-            patch_col<KP>(bh, bl, pr, P.d + 1, nq2 - tcol);
-            S.dlt[st][pr] = dl;
+        if (L.flags & FLAG_FIRST) {
+          // ---- a new unit: its home rows, once the MMAs are done with the last unit's
+          const TcUnit& W = S.units[L.unit];
+          const float* X = W.X;
+          a0 = W.a0, na = W.na, ng = W.ng, inst = W.inst;
+          tb = W.tb;
+          float* ca = S.cadd[useq & 1][0];
+          if (c < P.dpad) {
+            const float x = X[(size_t)a0 * P.dpad + c];
+            ca[c] = -x;
+            S.cadd[useq & 1][1][c] = 2.f * x;
           }
-          const long long cp1 = T.prof ? clock64() : 0;
+          if (c == 0) S.ra2[(useq + 2) & 3] = 0;  // last read two units ago
+          mbar_arrive(&S.ubar);
+          bool ok = wait_or_abort(&S.ubar, 0, abort_flag, T.wait_limit);  // first of its two phases a unit
+          if (ok && useq > 0) ok = wait_or_abort(&S.afree, (useq - 1) & 1, abort_flag, T.wait_limit);
+          if (!__all_sync(FULL_MASK, ok)) break;
+          float m = 0.f;
+          for (uint32_t g = 0; g < ng; ++g) {
+            const uint32_t r = g * TM + c;
+            if (r < na) {
+              const float4* xr = reinterpret_cast<const float4*>(X + (size_t)(a0 + r) * P.dpad);
+              float4 f[KP / 4];
 #pragma unroll
-          for (int g = 0; g < G; ++g) S.aid[st][g * TM + pr] = my_aid[g];
-          if (pr == 0) {
-            S.meta[st] = TileMeta{a0, na, ncols, (first && grp == 0 ? FLAG_FIRST : 0u) | (last ? FLAG_LAST : 0u), ng,
-                                  S.hx[mt & 3][0], S.hx[mt & 3][1], inst};
-            n_tiles += 1;
-            n_cells += (unsigned long long)na * ncols;
+              for (int q = 0; q < KP / 4; ++q) f[q] = 4u * q < P.dpad ? xr[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+              auto block = [&](int kb, float (&x)[8]) {
+                x[0] = f[2 * kb].x, x[1] = f[2 * kb].y, x[2] = f[2 * kb].z, x[3] = f[2 * kb].w;
+                x[4] = f[2 * kb + 1].x, x[5] = f[2 * kb + 1].y, x[6] = f[2 * kb + 1].z, x[7] = f[2 * kb + 1].w;
+              };
+              __nv_bfloat16 *ah = Ahi + g * OPB, *al = Alo + g * OPB;
+              const float nrm = conv_row<KP>(block, ah, al, c, ca, 1.f, P.d, 0.f, 1.f);
+              patch_col<KP>(ah, al, c, P.d, nrm);
+              m = fmaxf(m, nrm);
+            }
           }
+#pragma unroll
+          for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(FULL_MASK, m, o));
+          if (lane == 0) atomicMax(&S.ra2[useq & 3], __float_as_uint(m));
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          mbar_arrive(&S.full[st]);
-          if (T.prof) {
-            const long long ce = clock64();
-            pc_p1 += cp1 - cp0;
-            pc_fin += ce - cp1;
-            pc_conv += ce - cc0;
-          }
+          mbar_arrive(&S.afull);
+          mbar_arrive(&S.ubar);
+          if (!__all_sync(FULL_MASK, wait_or_abort(&S.ubar, 1, abort_flag, T.wait_limit))) break;
+          ra2max = __uint_as_float(*(volatile uint32_t*)&S.ra2[useq & 3]);
+          ++useq;
         }
-        first = false;
-        tile += nt;
+        __nv_bfloat16 *bh = Bhi + st * OPB, *bl = Blo + st * OPB;
+        if (c < L.ncols) {
+          const __nv_bfloat16* sh = Raw + rs * 2 * OPB;
+          auto block = [&](int kb, float (&x)[8]) {
+            unpack8(sh, sh + OPB, chunk_off<KP>(c, kb), 8u * kb < P.d, 8u * kb + 4 < P.d, x);
+          };
+          S.qid[ms][c] = S.rid[rs][c];
+          const float nq2 =
+              conv_row<KP>(block, bh, bl, c, S.cadd[(useq - 1) & 1][1], -2.f, P.d, 1.f, 0.f) * 0.25f;
+          float tcol = 0.f, dl = 0.f;
+          if (!column_threshold(tb, ra2max, nq2, &tcol, &dl)) {
+            tcol = 1e30f;   // every row of this column becomes a candidate ...
+            dl = INFINITY;  // ... and none is accepted without the FP64 check
+          }
+          patch_col<KP>(bh, bl, c, P.d + 1, nq2 - tcol);
+          S.dlt[ms][c] = dl;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&S.rawfree[rs]);
+        if (c == 0) {
+          n_tiles += 1;
+          n_cells += (unsigned long long)na * L.ncols;
+        }
+        if (c == 0) S.meta[ms] = TileMeta{a0, na, L.flags, ng, inst, L.ncols, L.hcr, L.hq};
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        mbar_arrive(&S.full[st]);
       }
-      asm volatile("cp.async.wait_all;" ::: "memory");
-      ++unit_k;
-      if (aborted) {
-        end_marker();
-        break;
+      if (c == 0 && n_tiles) {
+        atomicAdd(&T.ctr->tiles, n_tiles);
+        atomicAdd(&T.ctr->cells, n_cells);
       }
-    }
-    if (pr == 0 && n_tiles) {
-      atomicAdd(&T.ctr->tiles, n_tiles);
-      atomicAdd(&T.ctr->cells, n_cells);
-    }
-    if (tid == 0 && T.prof) {
-      atomicAdd(&T.ctr->prof[0], (unsigned long long)pw_sfree);
-      atomicAdd(&T.ctr->prof[1], (unsigned long long)(clock64() - p_start));
-      atomicAdd(&T.ctr->prof[7], (unsigned long long)pc_unit);
-      atomicAdd(&T.ctr->prof[8], (unsigned long long)pc_win);
-      atomicAdd(&T.ctr->prof[9], (unsigned long long)pc_conv);
-      atomicAdd(&T.ctr->prof[14], (unsigned long long)pc_ldw);
-      atomicAdd(&T.ctr->prof[16], (unsigned long long)pc_adv);
-      atomicAdd(&T.ctr->prof[17], (unsigned long long)pc_bar);
-      atomicAdd(&T.ctr->prof[18], (unsigned long long)pc_p1);
-      atomicAdd(&T.ctr->prof[19], (unsigned long long)pc_p2);
-      atomicAdd(&T.ctr->prof[20], (unsigned long long)pc_fin);
+      if (c == 0 && T.prof) {
+        atomicAdd(&T.ctr->prof[0], (unsigned long long)pw_sfree);
+        atomicAdd(&T.ctr->prof[14], (unsigned long long)pw_raw);
+        atomicAdd(&T.ctr->prof[1], (unsigned long long)(clock64() - p_start));
+      }
     }
     } else {
     // ============================ producers (NPW warps, two threads per row)
@@ -675,7 +687,7 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
     auto end_marker = [&]() {  // last tile slot: tells the MMA warp and the epilogue to stop
       const uint32_t st = tile % NS;
       if (tid == 0) {
-        wait_or_abort(&S.sfree[st], ((tile / NS) & 1) ^ 1, abort_flag, T.wait_limit);
+        wait_or_abort(&S.mfree[st], ((tile / NS) & 1) ^ 1, abort_flag, T.wait_limit);
         S.meta[st].flags = FLAG_END;
       }
       prod_sync();
@@ -733,12 +745,6 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
       }
       if (tid == 0) S.ra2max = 0;
       prod_sync();
-      uint32_t my_aid[(G + 1) / 2];  // original ids of home rows g * TM + prow, g = half, half + 2, ...
-#pragma unroll
-      for (int i = 0; i < (G + 1) / 2; ++i) {
-        const uint32_t r = (2 * i + half) * TM + prow;
-        my_aid[i] = (2 * i + (int)half < G && r < na) ? ids[a0 + r] : 0u;
-      }
       {
         for (uint32_t g = 0; g < ng; ++g) {
           const uint32_t r = g * TM + prow;
@@ -837,7 +843,7 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
           const uint32_t sl = pf++ & 1;
           if (tid == 0) {
             const long long c0 = T.prof ? clock64() : 0;
-            S.pflag[sl] = wait_or_abort(&S.sfree[st], ((issued / NS) & 1) ^ 1, abort_flag, T.wait_limit) ? 1u : 0u;
+            S.pflag[sl] = wait_or_abort(&S.mfree[st], ((issued / NS) & 1) ^ 1, abort_flag, T.wait_limit) ? 1u : 0u;
             if (T.prof) pw_sfree += clock64() - c0;
           }
           prod_sync();
@@ -906,7 +912,7 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
           const long long cb0 = T.prof ? clock64() : 0;
           if (tid == 0) {
             const long long c0 = T.prof ? clock64() : 0;
-            S.pflag[fl] = wait_or_abort(&S.sfree[st], ((tile / NS) & 1) ^ 1, abort_flag, T.wait_limit) ? 1u : 0u;
+            S.pflag[fl] = wait_or_abort(&S.mfree[st], ((tile / NS) & 1) ^ 1, abort_flag, T.wait_limit) ? 1u : 0u;
             if (T.prof) pw_sfree += clock64() - c0;
           }
           prod_sync();
@@ -934,12 +940,9 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
           pc_p2 += cp2 - cp1;
         }
         if (half == 0) S.dlt[st][prow] = dl;
-#pragma unroll
-        for (int i = 0; i < (G + 1) / 2; ++i)
-          if (2 * i + (int)half < G) S.aid[st][(2 * i + half) * TM + prow] = my_aid[i];
         if (tid == 0) {
-          S.meta[st] = TileMeta{a0, na, ncols, (first ? FLAG_FIRST : 0u) | (last ? FLAG_LAST : 0u), ng,
-                                S.hx[tile & 3][0], S.hx[tile & 3][1], inst};
+          S.meta[st] = TileMeta{a0, na, (first ? FLAG_FIRST : 0u) | (last ? FLAG_LAST : 0u), ng, inst, ncols,
+                                S.hx[tile & 3][0], S.hx[tile & 3][1]};
           n_tiles += 1;
           n_cells += (unsigned long long)na * ncols;
         }
@@ -978,75 +981,82 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
       atomicAdd(&T.ctr->prof[20], (unsigned long long)pc_fin);
     }
     }  // two threads a row
-  } else if (warp == MMA_WARP) {
-    // ============================ MMA issuer
+  } else if (warp >= MMA_WARP) {
+    // ============================ MMA issuers
     // B tiles come in stage order; each is multiplied with the unit's ng home
-    // chunks into alternating TMEM accumulators (MMA tile counter mt).
+    // chunks into a TMEM accumulator (MMA tile counter mt), warp w of the two
+    // issuing every mt = w mod 2 into accumulators w and w + 2 in turn.
+    const uint32_t me = (uint32_t)(warp - MMA_WARP);
     if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc(TM, TN);
-      constexpr uint32_t SBO = 16u * KP;
+      const uint64_t desc_a = chunk_desc<KP>(smem_u32(Ahi)), desc_b = chunk_desc<KP>(smem_u32(Bhi));
       uint32_t tile = 0, mt = 0, unit_k = 0;
+      uint32_t use[2] = {0, 0}, nxt = 0;  // uses of accumulators me, me + 2 so far; the one to take next
       int last_b = -1;
       uint32_t last_par = 0;
       long long mw_full = 0, mw_dfree = 0;
       const long long m_start = T.prof ? clock64() : 0;
       for (;;) {
-        const uint32_t st = tile % NS;
+        const uint32_t st = tile % NS, ms = tile % NM;
         const long long c0 = T.prof ? clock64() : 0;
         const bool fok = wait_or_abort(&S.full[st], (tile / NS) & 1, abort_flag, T.wait_limit);
         if (T.prof) mw_full += clock64() - c0;
-        if (!fok) {
-          mbar_arrive(&S.dfull[mt % NACC]);
-          break;
-        }
-        const uint32_t flags = S.meta[st].flags;
-        const uint32_t ng = S.meta[st].ng;
+        if (!fok) break;
+        const uint32_t flags = S.meta[ms].flags;
+        const uint32_t ng = S.meta[ms].ng;
         if (flags & FLAG_END) {
-          // wake the epilogue on the next accumulator, but only once every
-          // epilogue warp has taken that accumulator's previous use: an
-          // arrival before that would complete a second phase of dfull[b]
-          // under a warp still waiting for the first (parity aliasing)
-          const uint32_t b = mt % NACC;
-          wait_or_abort(&S.dfree[b], ((mt / NACC) & 1) ^ 1, abort_flag, T.wait_limit);
-          mbar_arrive(&S.dfull[b]);
+          // wake every epilogue group on its next accumulator, but only once
+          // the group has taken that accumulator's previous use: an arrival
+          // before that would complete a second phase of dfull[b] under a
+          // warp still waiting for the first (parity aliasing)
+          for (uint32_t j = 0; j < 2; ++j) {
+            const uint32_t b = me + 2 * j;
+            if (!wait_or_abort(&S.dfree[b], ((j ? use[1] : use[0]) & 1) ^ 1, abort_flag, T.wait_limit)) break;
+            S.acc[b].end = 1;
+            mbar_arrive_n(&S.dfull[b], 2);
+          }
           break;
         }
         bool ok = true;
         if (flags & FLAG_FIRST) ok = wait_or_abort(&S.afull, unit_k & 1, abort_flag, T.wait_limit);
-        if (!ok) {
-          mbar_arrive(&S.dfull[mt % NACC]);
-          break;
-        }
-        const uint32_t bh = smem_u32(Bhi + st * OPB), bl = smem_u32(Blo + st * OPB);
+        if (!ok) break;
+        // descriptors differ from the buffers' first ones by address / 16 alone
+        const uint64_t dbh = desc_b + st * (OPB * 2 / 16), dbl = dbh + NS * (OPB * 2 / 16);
+        constexpr uint32_t idesc = umma_idesc(TM, TN);
         for (uint32_t g = 0; g < ng && ok; ++g) {
-          const uint32_t b = mt % NACC;
-          const long long c1 = T.prof ? clock64() : 0;
-          ok = wait_or_abort(&S.dfree[b], ((mt / NACC) & 1) ^ 1, abort_flag, T.wait_limit);
-          if (T.prof) mw_dfree += clock64() - c1;
-          if (!ok) {
-            mbar_arrive(&S.dfull[b]);
-            break;
+          if (mt % NMMA != me) {
+            ++mt;
+            continue;
           }
+          const long long c1 = T.prof ? clock64() : 0;
+          const uint32_t j = nxt, par = (j ? use[1] : use[0]) & 1, b = me + 2 * j;
+          ok = wait_or_abort(&S.dfree[b], par ^ 1, abort_flag, T.wait_limit);
+          if (T.prof) mw_dfree += clock64() - c1;
+          if (!ok) break;
+          nxt = j ^ 1;
+          if (j) ++use[1]; else ++use[0];
           if (T.stall_test) {  // failure-detection test: never signal, let the waits run out
             ++mt;
             continue;
           }
           asm volatile("tcgen05.fence::after_thread_sync;");
-          const uint32_t ah = smem_u32(Ahi + g * OPB), al = smem_u32(Alo + g * OPB);
+          S.acc[b] = TcAcc{ms, g, 0u};
+          mbar_arrive(&S.dfull[b]);  // releases the metadata; the commit below completes the phase
+          const uint64_t dah = desc_a + g * (OPB * 2 / 16), dal = dah + G * (OPB * 2 / 16);
           const uint32_t dt = tbase + b * TN;
 #pragma unroll
           for (int ks = 0; ks < KP / 16; ++ks) {
-            const uint32_t o = ks * 256;
-            mma_bf16(dt, umma_desc(ah + o, SBO), umma_desc(bh + o, SBO), idesc, ks > 0 ? 1u : 0u);
-            mma_bf16(dt, umma_desc(ah + o, SBO), umma_desc(bl + o, SBO), idesc, 1u);
-            mma_bf16(dt, umma_desc(al + o, SBO), umma_desc(bh + o, SBO), idesc, 1u);
+            const uint32_t o = ks * chunk_kstep<KP>();
+            mma_bf16(dt, dah + o, dbh + o, idesc, ks > 0 ? 1u : 0u);
+            mma_bf16(dt, dah + o, dbl + o, idesc, 1u);
+            mma_bf16(dt, dal + o, dbh + o, idesc, 1u);
           }
           tc_commit(&S.dfull[b]);
           last_b = (int)b;
-          last_par = (mt / NACC) & 1;
+          last_par = par;
           ++mt;
         }
         if (!ok) break;
+        if (!T.stall_test) tc_commit(&S.bfree[st]);
         if ((flags & FLAG_LAST) && !T.stall_test) {
           tc_commit(&S.afree);
           ++unit_k;
@@ -1069,120 +1079,133 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
     __syncwarp();
   } else if (warp >= EPI0 && warp < EPI0 + NEPI) {
     // ============================ epilogue (NEPI warps)
-    // warp w reads TMEM lane quarter w % 4 (the hardware's access rule) and
-    // the 32-column blocks (w - EPI0) / 4, + NEPI / 4, ... of each 128 x 128
-    // accumulator
+    // Group e of EG = NEPI / 4 drains accumulators e, e + EG, ... in turn; its
+    // warp w reads TMEM lane quarter w % 4 (the hardware's access rule), all
+    // 128 columns in blocks of 32.  With all 16 warps on one accumulator the
+    // waits, the metadata and the slowest block of every accumulator were on
+    // every warp's path (2,550 cycles an accumulator on the 5M x 18 join);
+    // groups overlap them.  Two groups of 8 with two accumulators each measured
+    // 73.2 ms there (T = 66), four of 4 with one each 70.6.
+    constexpr uint32_t EG = NEPI / 4;
+    const uint32_t grp = (uint32_t)(warp - EPI0) / 4;
     const uint32_t quarter = warp & 3;
-    const uint32_t cblk0 = (warp - EPI0) >> 2;
     PairStage ps{pstage + (warp - EPI0) * PSTAGE, 0, 0, P.pairs_ij != 0};
     PairStage bs{pstage + (NEPI + warp - EPI0) * PSTAGE, 0};
     const RingCtx rcp_{P.pair_tags, P.deferred, P.def_out, &P.ctr->def_n, &P.ctr->stop};
     const RingCtx rcb_{P.band_tags, P.deferred, P.def_out, &P.ctr->def_n, &P.ctr->stop};
     const RingCtx* rcp = P.ring ? &rcp_ : nullptr;
     const RingCtx* rcb = P.ring ? &rcb_ : nullptr;
-    uint32_t tile = 0, mt = 0, g = 0;
-    long long ew_dfull = 0, ec_ld = 0, ec_slow = 0, ec_stage = 0;
+    long long ew_dfull = 0;
     const long long e_start = T.prof ? clock64() : 0;
-    for (;;) {
-      const uint32_t st = tile % NS, b = mt % NACC;
+    for (uint32_t n = 0;; ++n) {
+      const uint32_t b = grp + EG * (n % (NACC / EG));
       // all lanes wait; the outcome is made warp-uniform (tcgen05.ld is .sync.aligned)
       const long long cw = T.prof ? clock64() : 0;
-      const bool ok = __all_sync(FULL_MASK, wait_or_abort(&S.dfull[b], (mt / NACC) & 1, abort_flag, T.wait_limit));
+      const bool ok = __all_sync(FULL_MASK, wait_or_abort(&S.dfull[b], (n / (NACC / EG)) & 1, abort_flag, T.wait_limit));
       if (T.prof) ew_dfull += clock64() - cw;
       if (!ok) break;
-      const TileMeta M = S.meta[st];
-      if (__any_sync(FULL_MASK, (M.flags & FLAG_END) || *abort_flag)) break;
+      const TcAcc A = S.acc[b];
+      if (A.end) break;  // the same in all lanes
+      const TileMeta M = S.meta[A.ms];
       asm volatile("tcgen05.fence::after_thread_sync;");
-      const uint32_t row = g * TM + quarter * 32 + lane;  // row within the unit
-      const bool row_ok = row < M.na;
-      const uint32_t a_sorted = M.a0 + row;
+      const uint32_t row0 = A.g * TM + quarter * 32, row = row0 + lane;  // row within the unit
+      if (row0 < M.na) {
+        const bool row_ok = row < M.na;
+        const uint32_t a_sorted = M.a0 + row;
+        const uint32_t* ids = P.insts ? P.insts[M.inst].ids : P.ids;
+        const uint32_t ia = row_ok ? ids[a_sorted] : 0u;
+        // home bin: a pair (a, q) of two home rows is kept only for a < q
+        // (sorted positions); the home rows of this tile are the columns
+        // [hlo, hhi), column c at position hq + c - hlo: those below `drop`
+        // have q <= a
+        const uint32_t hlo = M.hcr & 255u, hhi = M.hcr >> 8;
+        const uint32_t drop = (hlo < hhi && a_sorted >= M.hq) ? min(hhi, hlo + min(a_sorted - M.hq, 255u) + 1) : 0u;
 #pragma unroll 1
-      for (uint32_t c0 = 32 * cblk0; c0 < TN; c0 += 32 * (NEPI / 4)) {
-      if (g * TM + quarter * 32 < M.na && c0 < M.ncols) {
-        uint32_t v[32];
-        const long long cl0 = T.prof ? clock64() : 0;
-        tmem_ld32_nowait(tbase + b * TN + ((quarter * 32u) << 16) + c0, v);
-        tmem_wait();
-        if (T.prof) ec_ld += clock64() - cl0;
-        // sign bits (D' < 0: a candidate), column c0 + j at bit j: one
-        // funnel shift per value, in four independent chains of 8
-        uint32_t m;
-        {
-          uint32_t m0 = 0, m1 = 0, m2 = 0, m3 = 0;
+        for (uint32_t c0 = 0; c0 < M.ncols; c0 += 32) {
+          uint32_t v[32];
+          tmem_ld32_nowait(tbase + b * TN + ((quarter * 32u) << 16) + c0, v);
+          tmem_wait();
+          // D' < 0 marks a candidate.  Three blocks of four hold none: a tree
+          // of three-input ORs over the signs (16 operations) finds those;
+          // extracting the 32 sign bits takes a funnel shift each, on a pipe
+          // at half the issue rate.
+          {
+            uint32_t o = v[0] | v[1];
 #pragma unroll
-          for (int j = 7; j >= 0; --j) {
-            m0 = __funnelshift_l(v[j], m0, 1);
-            m1 = __funnelshift_l(v[8 + j], m1, 1);
-            m2 = __funnelshift_l(v[16 + j], m2, 1);
-            m3 = __funnelshift_l(v[24 + j], m3, 1);
+            for (int j = 2; j < 32; j += 2) o |= v[j] | v[j + 1];
+            if (!__any_sync(FULL_MASK, (int)o < 0)) continue;
           }
-          m = m0 | (m1 << 8) | (m2 << 16) | (m3 << 24);
-        }
-        const uint32_t nvalid = min(32u, M.ncols - c0);
-        if (nvalid < 32) m &= (1u << nvalid) - 1u;
-        if (!row_ok) m = 0;
-        uint32_t acc_bits = 0, band_bits = 0;
-        const bool maybe = m != 0;
-        const long long cs0 = T.prof ? clock64() : 0;
-        const bool any_maybe = __any_sync(FULL_MASK, maybe);  // blocks without candidates skip the rest
-        if (any_maybe) {
-          if (maybe) {
-            // home bin: a pair (a, q) of two home rows is kept only for a < q
-            // (sorted positions); the home rows of this tile are the columns
-            // [hlo, hhi), column c at position hq + c - hlo
-            const uint32_t hlo = M.hcr & 255u, hhi = M.hcr >> 8;
-            if (hlo < hhi && a_sorted >= M.hq) {
-              const uint32_t lim = hlo + min(a_sorted - M.hq, 255u) + 1;  // columns < lim have q <= a
-              const int e0 = (int)max(hlo, c0) - (int)c0, e1 = (int)min(min(hhi, lim), c0 + 32) - (int)c0;
-              if (e0 < e1) m &= ~((e1 >= 32 ? FULL_MASK : ((1u << e1) - 1u)) & ~((1u << e0) - 1u));
+          // sign bits, value j at bit j, in four independent chains of 8
+          auto signs = [&]() {
+            uint32_t m0 = 0, m1 = 0, m2 = 0, m3 = 0;
+#pragma unroll
+            for (int j = 7; j >= 0; --j) {
+              m0 = __funnelshift_l(v[j], m0, 1);
+              m1 = __funnelshift_l(v[8 + j], m1, 1);
+              m2 = __funnelshift_l(v[16 + j], m2, 1);
+              m3 = __funnelshift_l(v[24 + j], m3, 1);
             }
-            while (m) {
+            return m0 | (m1 << 8) | (m2 << 16) | (m3 << 24);
+          };
+          uint32_t m = signs();
+          const uint32_t nvalid = M.ncols - c0;
+          if (nvalid < 32) m &= (1u << nvalid) - 1u;
+          if (!row_ok) m = 0;
+          if (drop > c0 && hlo < c0 + 32) {
+            const uint32_t e0 = max(hlo, c0) - c0, e1 = min(drop, c0 + 32) - c0;
+            if (e0 < e1) m &= ~((e1 >= 32 ? FULL_MASK : ((1u << e1) - 1u)) & ~((1u << e0) - 1u));
+          }
+          const float* dlt = &S.dlt[A.ms][c0];
+          const uint32_t* qid = &S.qid[A.ms][c0];
+          if (!__any_sync(FULL_MASK, (m & (m - 1)) != 0)) {
+            // at most one candidate a lane (most blocks that hold any)
+            if (!__any_sync(FULL_MASK, m != 0)) continue;
+            bool acc = false, band = false;
+            unsigned long long pr = 0;
+            if (m) {
               const int j = __ffs(m) - 1;
-              m &= m - 1;
-              if (pick32(v, j) <= -S.dlt[st][c0 + j])
-                acc_bits |= 1u << j;
-              else
-                band_bits |= 1u << j;  // decided later in FP64 (band list)
+              const uint32_t iq = qid[j];
+              acc = pick32(v, j) <= -dlt[j];
+              band = !acc;  // decided later in FP64
+              pr = ((unsigned long long)min(ia, iq) << 32) | max(ia, iq);
             }
+            stage_one(ps, acc, pr, &P.ctr->pairs, P.pairs, P.cap, P.inst_pairs, M.inst, rcp);
+            stage_one(bs, band, pr, &P.ctr->band_n, P.band_list, P.band_cap, nullptr, M.inst, rcb);
+            continue;
           }
-        }
-        __syncwarp();
-        const long long cs1 = T.prof ? clock64() : 0;
-        if (T.prof) ec_slow += cs1 - cs0;
-        const uint32_t ia = (acc_bits | band_bits) ? S.aid[st][row] : 0u;
-        auto emit = [&](PairStage& stg, uint32_t bits, unsigned long long* counter, unsigned long long* list,
-                        unsigned long long lcap, unsigned long long* ip, const RingCtx* rc) {
-          stage_pairs(
-              stg, __popc(bits),
-              [&](uint32_t) {
-                const int j = __ffs(bits) - 1;
-                bits &= bits - 1;
-                const uint32_t iq = S.qid[st][c0 + j];
-                const uint32_t lo = ia < iq ? ia : iq, hi = ia < iq ? iq : ia;
-                return ((unsigned long long)lo << 32) | hi;
-              },
-              counter, list, lcap, ip, M.inst, rc);
-        };
-        if (any_maybe && __any_sync(FULL_MASK, acc_bits != 0u))
+          // D' + dlt < 0: accepted (an infinite dlt accepts nothing)
+#pragma unroll
+          for (int j = 0; j < 32; j += 4) {
+            const float4 d4 = *reinterpret_cast<const float4*>(dlt + j);
+            v[j] = __float_as_uint(__uint_as_float(v[j]) + d4.x);
+            v[j + 1] = __float_as_uint(__uint_as_float(v[j + 1]) + d4.y);
+            v[j + 2] = __float_as_uint(__uint_as_float(v[j + 2]) + d4.z);
+            v[j + 3] = __float_as_uint(__uint_as_float(v[j + 3]) + d4.w);
+          }
+          const uint32_t acc_bits = m & signs();
+          auto emit = [&](PairStage& stg, uint32_t bits, unsigned long long* counter, unsigned long long* list,
+                          unsigned long long lcap, unsigned long long* ip, const RingCtx* rc) {
+            stage_pairs(
+                stg, __popc(bits),
+                [&](uint32_t) {
+                  const int j = __ffs(bits) - 1;
+                  bits &= bits - 1;
+                  const uint32_t iq = qid[j];
+                  return ((unsigned long long)min(ia, iq) << 32) | max(ia, iq);
+                },
+                counter, list, lcap, ip, M.inst, rc);
+          };
           emit(ps, acc_bits, &P.ctr->pairs, P.pairs, P.cap, P.inst_pairs, rcp);
-        if (any_maybe && __any_sync(FULL_MASK, band_bits != 0u))
-          emit(bs, band_bits, &P.ctr->band_n, P.band_list, P.band_cap, nullptr, rcb);
-        if (T.prof) ec_stage += clock64() - cs1;
-      }
+          // the band is decided later in FP64
+          if (__any_sync(FULL_MASK, m != acc_bits))
+            emit(bs, m & ~acc_bits, &P.ctr->band_n, P.band_list, P.band_cap, nullptr, rcb);
+        }
       }
       asm volatile("tcgen05.fence::before_thread_sync;");
       __syncwarp();
-      const bool last_g = g + 1 >= M.ng;
       if (lane == 0) {
         mbar_arrive(&S.dfree[b]);
-        if (last_g) mbar_arrive(&S.sfree[st]);  // the B stage served all home chunks
-      }
-      ++mt;
-      if (last_g) {
-        g = 0;
-        ++tile;
-      } else {
-        ++g;
+        mbar_arrive_n(&S.mfree[A.ms], 12u / M.ng);  // the tile served one of its home chunks
       }
     }
     stage_flush(ps, &P.ctr->pairs, P.pairs, P.cap, P.inst_pairs, rcp);
@@ -1190,9 +1213,6 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
     if (T.prof && lane == 0) {
       atomicAdd(&T.ctr->prof[5], (unsigned long long)ew_dfull);
       atomicAdd(&T.ctr->prof[6], (unsigned long long)(clock64() - e_start));
-      atomicAdd(&T.ctr->prof[10], (unsigned long long)ec_ld);
-      atomicAdd(&T.ctr->prof[11], (unsigned long long)ec_slow);
-      atomicAdd(&T.ctr->prof[13], (unsigned long long)ec_stage);
     }
   }
   // all roles meet here before tensor memory is released
@@ -1220,7 +1240,7 @@ template <int KP>
 void launch_tc(mistic_handle_s* h, const JoinParams& P, const TcParams& T) {
   constexpr int NS = TcShape<KP>::NS, G = TcShape<KP>::G, RAW = TcShape<KP>::RAW, NEPI = TcShape<KP>::NEPI;
   constexpr int NT = tc_threads(NEPI);
-  const size_t dyn = (2 * G + 2 * NS + 2 * RAW) * (size_t)TM * KP * sizeof(__nv_bfloat16) +
+  const size_t dyn = 512 + (2 * G + 2 * NS + 2 * RAW) * (size_t)TM * KP * sizeof(__nv_bfloat16) +
                      (size_t)2 * NEPI * PSTAGE * sizeof(unsigned long long);
   MCK(cudaFuncSetAttribute(k_join_tc<KP, NS, G, RAW, NEPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
   MCK(cudaFuncSetAttribute(k_join_tc<KP, NS, G, RAW, NEPI>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));

@@ -391,9 +391,11 @@ int bit_length(uint64_t v) {
 // it, for tuning).  A tensor-core tile costs about the same per candidate row
 // whatever its number of home rows, a CUDA-core unit costs d FMAs per cell,
 // so small bins go to the CUDA cores.  Measured on GB300 (whole join, ms):
-//   5M x 18:    T = 48: 150.2, 61: 147.0, 80: 145.2, 100: 145.1, 128: 146.8
-//   515k x 90:  T = 1: 259.9, 2: 261.9, 4: 261.9, 8: 263.3
-// hence 29000 / d^2, clamped to [1, 96].
+//   5M x 18:        T = 24: 105.7, 32: 104.1, 44: 103.4, 66: 104.7, 89: 108.0
+//   250,007 x 18:   T = 24: 2.81, 32: 2.79, 44: 2.78, 66: 2.81, 89: 2.92
+//   100,000 x 18:   T = 24: 1.98, 32: 1.99, 44: 1.99, 66: 2.01, 89: 2.05
+//   515k x 90 (short-row kernel): T = 1: 259.9, 2: 261.9, 4: 261.9, 8: 263.3
+// hence 16000 / d^2, clamped to [1, 96].
 uint32_t tc_min_bin(uint32_t d, bool wide) {
   const char* e = getenv("MISTIC_TC_MIN_BIN");
   if (e && *e) return (uint32_t)std::max(1l, strtol(e, nullptr, 10));
@@ -403,7 +405,7 @@ uint32_t tc_min_bin(uint32_t d, bool wide) {
   // large neighbour bin (one segment holds a whole bin) run on single warps:
   // on the 5M x 384 workload such units took 2.1 s of a 14 s join at T = 8.
   if (wide) return 1;
-  return (uint32_t)std::min(96.0, std::max(1.0, std::floor(29000.0 / ((double)d * d))));
+  return (uint32_t)std::min(96.0, std::max(1.0, std::floor(16000.0 / ((double)d * d))));
 }
 
 // Relative error allowance per (|a'| + |q'|)^2 + 1.2 eps2 of a tensor-core

@@ -1,10 +1,10 @@
 // Device helpers shared by the tensor-core joins (join_tc.cu: augmented K up
 // to 128 in one operand tile; join_tcw.cu: long rows in K chunks).
 //
-// tcgen05 operands live in shared memory in the no-swizzle K-major
-// core-matrix layout: a core matrix is 8 rows x 16 bytes (8 bf16), stored as
-// 128 contiguous bytes; K-adjacent core matrices are LBO = 128 B apart and
-// 8-row groups SBO = 16 * K bytes apart (K = the operand buffer's K extent).
+// No-swizzle K-major operands in shared memory: a core matrix is 8 rows x 16
+// bytes (8 bf16), stored as 128 contiguous bytes; K-adjacent core matrices are
+// LBO = 128 B apart and 8-row groups SBO = 16 * K bytes apart (K = the operand
+// buffer's K extent).
 #pragma once
 
 #include <cuda_bf16.h>
@@ -139,11 +139,31 @@ __device__ __forceinline__ bool wait_or_abort(unsigned long long* b, uint32_t pa
 }
 
 // bf16 offset of the 16-byte chunk of row r and K block kb (8 bf16) in an
-// operand buffer of K extent KX.
+// operand buffer of K extent KX.  K = 32 and K = 16: rows of 64 and 32 bytes in
+// the hardware's 64-byte and 32-byte swizzle (buffers start on 512-byte
+// boundaries); other extents: no-swizzle core matrices.
 template <int KX>
 __device__ __forceinline__ uint32_t chunk_off(uint32_t r, uint32_t kb) {
+  if (KX == 32) return r * 32 + ((kb ^ ((r >> 1) & 3u)) << 3);
+  if (KX == 16) return r * 16 + ((kb ^ ((r >> 2) & 1u)) << 3);
   return ((r >> 3) * (KX / 8) + kb) * 64 + (r & 7) * 8;
 }
+
+// Descriptor of such a buffer, and the step of its address field (16-byte
+// units) per K step of 16.
+template <int KX>
+__device__ __forceinline__ uint64_t chunk_desc(uint32_t saddr) {
+  if (KX != 32 && KX != 16) return umma_desc(saddr, 16u * KX);
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr >> 4) & 0x3FFF);
+  d |= (uint64_t)1 << 16;                      // LBO: not used by swizzled K-major layouts
+  d |= (uint64_t)((8u * KX * 2) >> 4) << 32;   // SBO: next 8-row group
+  d |= (uint64_t)1 << 46;                      // descriptor version
+  d |= (uint64_t)(KX == 32 ? 4 : 6) << 61;     // 64-byte / 32-byte swizzle
+  return d;
+}
+template <int KX>
+__host__ __device__ constexpr uint32_t chunk_kstep() { return KX == 32 || KX == 16 ? 2u : 16u; }
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
