@@ -467,33 +467,34 @@ k_join_f32r(const JoinParams P) {
 
 // ---------------------------------------------------------------- FP64 plain
 // The reference predicate for every candidate: dims in order, each
-// subtraction, product and sum rounded (no contraction).
+// subtraction, product and sum rounded (no contraction).  Bound by the FP64
+// pipe (a warp's FP64 instruction occupies it for 64 cycles).  A sum of
+// rounded non-negative terms never falls, so a home row whose partial sums
+// exceed `thr` for all 32 candidates is left out of the remaining dims (tested
+// on the high words, which order as the values do): 30,000 x 18 uniform
+// 48.5 -> 37.7 ms.  `live`: home rows to evaluate; qv: the lane holds a candidate.
 template <int CH>
 __device__ __forceinline__ void f64_dists(const double2* __restrict__ qrow, const double2* sA, uint32_t nq2,
-                                          uint32_t d, uint32_t na, double (&acc)[CH]) {
-  const uint32_t full = d >> 1;
+                                          uint32_t d, uint32_t na, bool qv, double thr, double (&acc)[CH]) {
+  const uint32_t steps = (d + 1) >> 1;  // rows are zero padded to whole pairs
+  const int hi_thr = __double2hiint(thr);
+  uint32_t live = (1u << na) - 1u;
 #pragma unroll
   for (int a = 0; a < CH; ++a) acc[a] = 0.0;
-  for (uint32_t c = 0; c < full; ++c) {
+  for (uint32_t c = 0; c < steps; ++c) {
     const double2 qq = qrow[c];
 #pragma unroll
     for (int a = 0; a < CH; ++a) {
-      if (a >= (int)na) break;
+      if (!((live >> a) & 1u)) continue;  // warp-uniform
       const double2 aa = sA[a * nq2 + c];
       double t;
       t = __dsub_rn(aa.x, qq.x); acc[a] = __dadd_rn(acc[a], __dmul_rn(t, t));
-      t = __dsub_rn(aa.y, qq.y); acc[a] = __dadd_rn(acc[a], __dmul_rn(t, t));
+      if (2 * c + 1 < d) {
+        t = __dsub_rn(aa.y, qq.y); acc[a] = __dadd_rn(acc[a], __dmul_rn(t, t));
+      }
+      if (!__any_sync(FULL_MASK, qv && __double2hiint(acc[a]) <= hi_thr)) live &= ~(1u << a);
     }
-  }
-  if (d & 1) {
-    const double2 qq = qrow[full];
-#pragma unroll
-    for (int a = 0; a < CH; ++a) {
-      if (a >= (int)na) break;
-      const double2 aa = sA[a * nq2 + full];
-      const double t = __dsub_rn(aa.x, qq.x);
-      acc[a] = __dadd_rn(acc[a], __dmul_rn(t, t));
-    }
+    if (!live) return;
   }
 }
 
@@ -530,7 +531,7 @@ k_join_f64(const JoinParams P) {
       const uint32_t q = t.q;
       const double2* qrow = X + (size_t)(t.qv ? q : a0) * nq2;
       double acc[CH];
-      f64_dists<CH>(qrow, sA, nq2, P.d, na, acc);
+      f64_dists<CH>(qrow, sA, nq2, P.d, na, t.qv, thr, acc);
       uint32_t m = 0;
 #pragma unroll
       for (int a = 0; a < CH; ++a) {
