@@ -49,7 +49,6 @@ constexpr size_t kScratchBytes = MISTIC_NOALLOC_SCRATCH_BYTES;
 constexpr size_t kHeaderBytes = 256;  // counters, then the FP32 rows
 constexpr int kThreads = 256;
 constexpr int kCH = 32;      // home points per unit
-constexpr uint32_t kSeg = 4096;  // candidate points per unit
 constexpr int kMaxDevices = 64;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
@@ -71,9 +70,9 @@ struct NaParams {
   float t_lo, t_hi;
   int all_fp64;     // 1: FP32 cannot separate the pairs; every candidate is decided in FP64
   double eps2;
-  unsigned long long* pairs;  // caller's buffer, packed (i << 32 | j)
+  unsigned long long* pairs;  // caller's buffer: i and j as two uint32
   unsigned long long cap;
-  uint32_t nseg;
+  uint32_t seg, nseg;  // candidate points per unit, units per home chunk
   unsigned long long n_units;
 };
 
@@ -129,12 +128,52 @@ __device__ __forceinline__ double na_exact(const NaParams& P, uint32_t i, uint32
   return s;
 }
 
-// Units: home chunk c (rows 32c .. 32c+31) against candidate segment s
-// (rows s*kSeg .. s*kSeg+kSeg-1), candidates restricted to j > i.
+// Squared FP32 distances of candidate row q (in registers, DQ float4 chunks)
+// to home rows r0 .. r0 + NR - 1 in shared memory, as masks of those at or
+// below t_hi and t_lo.  Packed pairs of floats: even and odd coordinates are
+// summed apart (the filter's bound holds for any order), two to an
+// instruction.
+template <int DQ, int NR>
+__device__ __forceinline__ void na_rows(const ulonglong2 (&qq)[DQ], const float4* sA, int r0, float t_lo, float t_hi,
+                                        uint32_t* m, uint32_t* lo_m) {
+  unsigned long long acc2[NR];
+#pragma unroll
+  for (int i = 0; i < NR; ++i) acc2[i] = 0ull;
+#pragma unroll
+  for (int c = 0; c < DQ; ++c) {
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+      const ulonglong2 aa = reinterpret_cast<const ulonglong2*>(sA)[(r0 + i) * DQ + c];
+      unsigned long long t;
+      asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(t) : "l"(aa.x), "l"(qq[c].x));
+      asm("fma.rn.f32x2 %0, %1, %1, %0;" : "+l"(acc2[i]) : "l"(t));
+      asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(t) : "l"(aa.y), "l"(qq[c].y));
+      asm("fma.rn.f32x2 %0, %1, %1, %0;" : "+l"(acc2[i]) : "l"(t));
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NR; ++i) {
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc2[i]));
+    const float acc = lo + hi;
+    *m |= (acc <= t_hi ? 1u : 0u) << (r0 + i);
+    *lo_m |= (acc <= t_lo ? 1u : 0u) << (r0 + i);
+  }
+}
+
+// Units: home chunk c (rows 32c .. 32c+31) against candidate segment s (rows
+// s*seg .. s*seg+seg-1), candidates restricted to j > i.  Bound by the FP32
+// pipe (a subtraction and a multiply-add a coordinate).  DQ > 0: rows of DQ
+// float4 chunks, the lane's candidate in registers and home rows in groups of
+// 8, so a shared-memory read feeds 4 packed operations; DQ = 0: longer rows,
+// a chunk at a time against all 32 home rows.  With one coordinate an
+// instruction and 4,096-point segments (3,750 units with work on 7,296 warps)
+// the 30,000 x 32 join took 2.0 ms.
+template <int DQ>
 __global__ void __launch_bounds__(kThreads) k_na_join(const NaParams P) {
   extern __shared__ float4 na_smem[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const uint32_t nq4 = P.dpad >> 2;
+  const uint32_t nq4 = DQ ? (uint32_t)DQ : P.dpad >> 2;
   float4* sA = na_smem + (size_t)w * kCH * nq4;
   const float4* X = (const float4*)P.xf;
   uint32_t band_cnt = 0;
@@ -146,7 +185,8 @@ __global__ void __launch_bounds__(kThreads) k_na_join(const NaParams P) {
     const uint32_t c = (uint32_t)(u / P.nseg), s = (uint32_t)(u % P.nseg);
     const uint32_t a0 = c * kCH;
     const uint32_t na = min((uint32_t)kCH, P.n - a0);
-    const uint32_t qlo = max(a0 + 1, s * kSeg), qhi = min(P.n, (s + 1) * kSeg);
+    const uint32_t qlo = max(a0 + 1, s * P.seg);
+    const uint32_t qhi = (uint32_t)min((unsigned long long)P.n, (s + 1ull) * P.seg);
     if (qlo >= qhi) continue;
     __syncwarp();
     for (uint32_t i = lane; i < kCH * nq4; i += 32)
@@ -155,32 +195,41 @@ __global__ void __launch_bounds__(kThreads) k_na_join(const NaParams P) {
     for (uint32_t qb = qlo; qb < qhi; qb += 32) {
       const uint32_t q = qb + lane;
       const bool qv = q < qhi;
-      const float4* qrow = X + (size_t)(qv ? q : qlo) * nq4;
-      float acc[kCH];
-#pragma unroll
-      for (int a = 0; a < kCH; ++a) acc[a] = 0.f;
-      for (uint32_t cc = 0; cc < nq4; ++cc) {
-        const float4 qq = qrow[cc];
-#pragma unroll
-        for (int a = 0; a < kCH; ++a) {
-          const float4 aa = sA[a * nq4 + cc];
-          float t;
-          t = aa.x - qq.x; acc[a] = fmaf(t, t, acc[a]);
-          t = aa.y - qq.y; acc[a] = fmaf(t, t, acc[a]);
-          t = aa.z - qq.z; acc[a] = fmaf(t, t, acc[a]);
-          t = aa.w - qq.w; acc[a] = fmaf(t, t, acc[a]);
-        }
-      }
+      const ulonglong2* qrow = reinterpret_cast<const ulonglong2*>(X + (size_t)(qv ? q : qlo) * nq4);
       uint32_t m = 0, lo = 0;
       if (P.all_fp64) {
         // the FP32 values are not usable (an offset beyond FLT_MAX is inf and
         // inf - inf is NaN): every candidate goes to the FP64 decision
         m = FULL_MASK;
+      } else if constexpr (DQ > 0) {
+        ulonglong2 qq[DQ];
+#pragma unroll
+        for (int cc = 0; cc < DQ; ++cc) qq[cc] = qrow[cc];
+#pragma unroll
+        for (int g = 0; g < kCH / 8; ++g) na_rows<DQ, 8>(qq, sA, g * 8, P.t_lo, P.t_hi, &m, &lo);
       } else {
+        unsigned long long acc2[kCH];
+#pragma unroll
+        for (int a = 0; a < kCH; ++a) acc2[a] = 0ull;
+        for (uint32_t cc = 0; cc < nq4; ++cc) {
+          const ulonglong2 qq = qrow[cc];
+#pragma unroll
+          for (int a = 0; a < kCH; ++a) {
+            const ulonglong2 aa = reinterpret_cast<const ulonglong2*>(sA)[a * nq4 + cc];
+            unsigned long long t;
+            asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(t) : "l"(aa.x), "l"(qq.x));
+            asm("fma.rn.f32x2 %0, %1, %1, %0;" : "+l"(acc2[a]) : "l"(t));
+            asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(t) : "l"(aa.y), "l"(qq.y));
+            asm("fma.rn.f32x2 %0, %1, %1, %0;" : "+l"(acc2[a]) : "l"(t));
+          }
+        }
 #pragma unroll
         for (int a = 0; a < kCH; ++a) {
-          m |= (acc[a] <= P.t_hi ? 1u : 0u) << a;
-          lo |= (acc[a] <= P.t_lo ? 1u : 0u) << a;
+          float f0, f1;
+          asm("mov.b64 {%0, %1}, %2;" : "=f"(f0), "=f"(f1) : "l"(acc2[a]));
+          const float acc = f0 + f1;
+          m |= (acc <= P.t_hi ? 1u : 0u) << a;
+          lo |= (acc <= P.t_lo ? 1u : 0u) << a;
         }
       }
       // valid home rows: a < na and a0 + a < q
@@ -207,7 +256,7 @@ __global__ void __launch_bounds__(kThreads) k_na_join(const NaParams P) {
       while (accm) {
         const int a = __ffs(accm) - 1;
         accm &= accm - 1;
-        if (pos < P.cap) P.pairs[pos] = ((unsigned long long)(a0 + a) << 32) | q;
+        if (pos < P.cap) P.pairs[pos] = ((unsigned long long)q << 32) | (a0 + a);  // (i, j) in memory order
         ++pos;
       }
     }
@@ -216,10 +265,19 @@ __global__ void __launch_bounds__(kThreads) k_na_join(const NaParams P) {
   if (lane == 0 && tot) atomicAdd(&P.hdr->band, (unsigned long long)tot);
 }
 
-// Swap each packed (i << 32 | j) into memory order (i, j) as two uint32.
-__global__ void k_na_to_ij(unsigned long long* p, unsigned long long n) {
-  const unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = (p[i] >> 32) | (p[i] << 32);
+using NaKernel = void (*)(const NaParams);
+NaKernel na_kernel(uint32_t dpad) {
+  switch (dpad / 4) {
+    case 1: return k_na_join<1>;
+    case 2: return k_na_join<2>;
+    case 3: return k_na_join<3>;
+    case 4: return k_na_join<4>;
+    case 5: return k_na_join<5>;
+    case 6: return k_na_join<6>;
+    case 7: return k_na_join<7>;
+    case 8: return k_na_join<8>;
+    default: return k_na_join<0>;
+  }
 }
 
 std::mutex g_setup_mu;
@@ -308,35 +366,35 @@ extern "C" mistic_status mistic_selfjoin_noalloc(const void* d_pts, uint64_t n, 
     P.t_hi = INFINITY;
     P.all_fp64 = 1;
   }
-  const uint32_t nchunks = (uint32_t)((n + kCH - 1) / kCH);
-  P.nseg = (uint32_t)((n + kSeg - 1) / kSeg);
-  P.n_units = (unsigned long long)nchunks * P.nseg;
+  const NaKernel kern = na_kernel(dpad);
   const size_t smem_warp = (size_t)kCH * dpad * sizeof(float);
   const int warps = (int)std::min<size_t>(kThreads / 32, std::max<size_t>(1, (160 * 1024) / smem_warp));
   const size_t smem = smem_warp * warps;
   if (smem > 48 * 1024 &&
-      (st = cuda_status(cudaFuncSetAttribute(k_na_join, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem))) != MISTIC_OK)
+      (st = cuda_status(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem))) !=
+          MISTIC_OK)
     return st;
   int dev = 0, sms = 0, per_sm = 0;
   if ((st = cuda_status(cudaGetDevice(&dev))) != MISTIC_OK) return st;
   if ((st = cuda_status(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev))) != MISTIC_OK) return st;
-  if ((st = cuda_status(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_na_join, warps * 32, smem))) !=
-      MISTIC_OK)
+  if ((st = cuda_status(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, smem))) != MISTIC_OK)
     return st;
   if (per_sm < 1) return MISTIC_ERR_TOO_LARGE;
+  // segments of 4,096 points, shorter ones (down to 256) while the resident
+  // warps would get fewer than 8 units each (half of the units lie below the
+  // diagonal and have no work)
+  const unsigned long long nchunks = (n + kCH - 1) / kCH;
+  const unsigned long long want_units = 16ull * (unsigned long long)per_sm * sms * warps;
+  const unsigned long long fair = (n * nchunks / want_units + 31) & ~31ull;
+  P.seg = (uint32_t)std::min<unsigned long long>(4096, std::max<unsigned long long>(256, fair));
+  P.nseg = (uint32_t)((n + P.seg - 1) / P.seg);
+  P.n_units = nchunks * P.nseg;
   const unsigned long long want = (P.n_units + warps - 1) / warps;
   const unsigned grid = (unsigned)std::min<unsigned long long>((unsigned long long)per_sm * sms, want);
-  k_na_join<<<grid, warps * 32, smem, s>>>(P);
+  kern<<<grid, warps * 32, smem, s>>>(P);
   if ((st = cuda_status(cudaGetLastError())) != MISTIC_OK) return st;
   if ((st = cuda_status(cudaMemcpyAsync(&hh, P.hdr, sizeof hh, cudaMemcpyDeviceToHost, s))) != MISTIC_OK) return st;
   if ((st = cuda_status(cudaStreamSynchronize(s))) != MISTIC_OK) return st;
-  const unsigned long long stored = std::min<unsigned long long>(hh.pairs, pair_capacity);
-  if (stored) {
-    k_na_to_ij<<<(unsigned)((stored + 255) / 256), 256, 0, s>>>(P.pairs, stored);
-    if ((st = cuda_status(cudaGetLastError())) != MISTIC_OK) return st;
-    if ((st = cuda_status(cudaStreamSynchronize(s))) != MISTIC_OK) return st;
-  }
   *pairs_ij = hh.pairs;
   return hh.pairs > pair_capacity ? MISTIC_ERR_PAIR_OVERFLOW : MISTIC_OK;
 }
