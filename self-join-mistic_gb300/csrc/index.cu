@@ -175,8 +175,11 @@ __global__ void k_gather_sample(const T* __restrict__ x, size_t n, uint32_t d, u
 // memory); a second kernel adds the chunk partials in a fixed order, so the
 // result - and the reference points derived from it - is deterministic.
 constexpr int COV_T = 16;
-constexpr int COV_CHUNK = 128;
+// Rows a chunk: 128, or 32 for rows of at most 32 columns, whose few tiles
+// would leave most SMs idle.
+constexpr uint32_t cov_chunk(uint32_t d) { return d <= 32 ? 32u : 128u; }
 
+template <int COV_CHUNK>
 __global__ void k_sample_cov_part(const double* __restrict__ s, uint32_t S, uint32_t d, const double* __restrict__ mu,
                                   double* __restrict__ part /* [chunks][d][d] */) {
   __shared__ double sa[COV_CHUNK][COV_T + 1], sb[COV_CHUNK][COV_T + 1];
@@ -200,24 +203,27 @@ __global__ void k_sample_cov_part(const double* __restrict__ s, uint32_t S, uint
 
 __global__ void k_sample_cov_final(const double* __restrict__ part, uint32_t chunks, uint32_t d, uint32_t S,
                                    double* __restrict__ cov) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (size_t)d * d) return;
+  // four lanes an element, each every fourth chunk
+  const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / 4;
+  const uint32_t l = threadIdx.x & 3u;
   double acc = 0.0;
-  for (uint32_t c = 0; c < chunks; ++c) acc += part[(size_t)c * d * d + i];
-  cov[i] = acc / S;
+  if (i < (size_t)d * d)
+    for (uint32_t c = l; c < chunks; c += 4) acc += part[(size_t)c * d * d + i];
+  acc += __shfl_xor_sync(FULL_MASK, acc, 1);
+  acc += __shfl_xor_sync(FULL_MASK, acc, 2);
+  if (i < (size_t)d * d && l == 0) cov[i] = acc / S;
 }
 
 // ------------------------------------------------------------ reference-point distances
 // D[i][j] = FP64 ||x_i - r_j|| (sequential sum, then sqrt), with per-block
 // min/max partials per reference point.  Bound by the FP64 pipe (2 k d
-// operations a row).  A block's 256 rows pass through shared memory RPD_COLS
+// operations a row).  A block's rows pass through shared memory RPD_COLS
 // columns at a time, each value read once for all k sums, so rows of any
 // length load coalesced: a thread reading its own row of 384 FP32 values took
 // 17.5 ms for 1M rows at k = 8, now 12.1 ms; 515k x 90 4.0 -> 1.7 ms.
-constexpr int RPD_THREADS = 256;
 constexpr int RPD_COLS = 32;
 
-template <class T, int K>
+template <class T, int K, int RPD_THREADS>
 __global__ void __launch_bounds__(RPD_THREADS)
 k_rp_dist(const T* __restrict__ x, size_t n, uint32_t d, const double* __restrict__ rps, int k,
           double* __restrict__ D, double* __restrict__ part /* [block][2][k] */) {
@@ -896,6 +902,8 @@ void colstats(mistic_handle_s* h, const void* x, mistic_dtype dt, size_t n, uint
   launched(h, "colstats_final");
 }
 
+size_t cov_parts(uint32_t S, uint32_t d) { return (S + cov_chunk(d) - 1) / cov_chunk(d); }
+
 void sample_cov(mistic_handle_s* h, const void* x, mistic_dtype dt, size_t n, uint32_t d,
                 uint32_t S, double* sbuf, const double* mu, double* part, double* cov) {
   const size_t tot = (size_t)S * d;
@@ -905,32 +913,41 @@ void sample_cov(mistic_handle_s* h, const void* x, mistic_dtype dt, size_t n, ui
   else
     k_gather_sample<float><<<nb, 256, 0, h->stream>>>((const float*)x, n, d, S, sbuf);
   launched(h, "gather_sample");
-  const uint32_t chunks = (S + COV_CHUNK - 1) / COV_CHUNK;
+  const uint32_t chunk = cov_chunk(d), chunks = (S + chunk - 1) / chunk;
   dim3 blk(COV_T, COV_T), grd((d + COV_T - 1) / COV_T, (d + COV_T - 1) / COV_T, chunks);
-  k_sample_cov_part<<<grd, blk, 0, h->stream>>>(sbuf, S, d, mu, part);
+  if (chunk == 32)
+    k_sample_cov_part<32><<<grd, blk, 0, h->stream>>>(sbuf, S, d, mu, part);
+  else
+    k_sample_cov_part<128><<<grd, blk, 0, h->stream>>>(sbuf, S, d, mu, part);
   launched(h, "sample_cov_part");
-  k_sample_cov_final<<<(unsigned)(((size_t)d * d + 255) / 256), 256, 0, h->stream>>>(part, chunks, d, S, cov);
+  k_sample_cov_final<<<(unsigned)((4 * (size_t)d * d + 255) / 256), 256, 0, h->stream>>>(part, chunks, d, S, cov);
   launched(h, "sample_cov_final");
 }
 
 void rp_dist(mistic_handle_s* h, const void* x, mistic_dtype dt, size_t n, uint32_t d,
-             const double* rps, int k, double* D, double* part, uint32_t nparts, double* mm) {
+             const double* rps, int k, double* D, double* part, double* mm) {
+  const unsigned tpb = row_block(h, n), nparts = (unsigned)((n + tpb - 1) / tpb);
   auto launch = [&](auto kern, const auto* xs, int K) {
     allow_max_dyn_smem(kern);
-    const size_t smem = (RPD_THREADS * (RPD_COLS + 1) + (size_t)K * RPD_COLS) * sizeof(double);
-    kern<<<nparts, RPD_THREADS, smem, h->stream>>>(xs, n, d, rps, k, D, part);
+    const size_t smem = (tpb * (RPD_COLS + 1) + (size_t)K * RPD_COLS) * sizeof(double);
+    kern<<<nparts, tpb, smem, h->stream>>>(xs, n, d, rps, k, D, part);
   };
-  if (dt == MISTIC_F64)
-    k <= 8 ? launch(k_rp_dist<double, 8>, (const double*)x, 8) : launch(k_rp_dist<double, 16>, (const double*)x, 16);
-  else
-    k <= 8 ? launch(k_rp_dist<float, 8>, (const float*)x, 8) : launch(k_rp_dist<float, 16>, (const float*)x, 16);
+#define MISTIC_RPD(T, K)                                             \
+  tpb == 64 ? launch(k_rp_dist<T, K, 64>, (const T*)x, K) : launch(k_rp_dist<T, K, 256>, (const T*)x, K)
+  if (dt == MISTIC_F64) {
+    if (k <= 8) MISTIC_RPD(double, 8); else MISTIC_RPD(double, 16);
+  } else {
+    if (k <= 8) MISTIC_RPD(float, 8); else MISTIC_RPD(float, 16);
+  }
+#undef MISTIC_RPD
   launched(h, "rp_dist");
   k_minmax_final<<<k, 256, 0, h->stream>>>(part, nparts, k, mm);
   launched(h, "minmax_final");
 }
 
 void pack_keys(mistic_handle_s* h, const double* D, size_t n, const PackParams& P, uint64_t* keys) {
-  k_pack_keys<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(D, n, P, keys);
+  const unsigned tpb = row_block(h, n);
+  k_pack_keys<<<(unsigned)((n + tpb - 1) / tpb), tpb, 0, h->stream>>>(D, n, P, keys);
   launched(h, "pack_keys");
 }
 
@@ -952,12 +969,12 @@ void bins(mistic_handle_s* h, const uint64_t* keys, size_t n, uint32_t* flags, u
 void gather(mistic_handle_s* h, const void* x, mistic_dtype dt, size_t n, uint32_t d,
             const uint32_t* perm, const double* center, uint32_t dpad32, float* xf, uint32_t dpad64,
             double* xd, uint32_t* ids, double* norm_part, double* rmax) {
-  const unsigned nb = (unsigned)((n + 255) / 256);
+  const unsigned tpb = row_block(h, n), nb = (unsigned)((n + tpb - 1) / tpb);
   if (dt == MISTIC_F64)
-    k_gather_points<double><<<nb, 256, 0, h->stream>>>((const double*)x, n, d, perm, center, dpad32, xf,
+    k_gather_points<double><<<nb, tpb, 0, h->stream>>>((const double*)x, n, d, perm, center, dpad32, xf,
                                                       dpad64, xd, ids, norm_part);
   else
-    k_gather_points<float><<<nb, 256, 0, h->stream>>>((const float*)x, n, d, perm, center, dpad32, xf,
+    k_gather_points<float><<<nb, tpb, 0, h->stream>>>((const float*)x, n, d, perm, center, dpad32, xf,
                                                      dpad64, xd, ids, norm_part);
   launched(h, "gather_points");
   k_max_final<<<1, 1024, 0, h->stream>>>(norm_part, nb, rmax);

@@ -231,9 +231,21 @@ T* abuf(mistic_handle_s* h, const char* name, size_t count) {
   return (T*)h->arena.get(name, count * sizeof(T));
 }
 
+// Read-back of a few values, through the handle's pinned block (a copy into
+// pageable memory is staged by the driver).
+constexpr size_t kPinnedBytes = 64u << 10;
 void d2h(mistic_handle_s* h, void* dst, const void* src, size_t bytes) {
-  MCK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, h->stream));
+  if (!h->pinned && !h->pinned_bytes) {
+    if (cudaHostAlloc(&h->pinned, kPinnedBytes, cudaHostAllocDefault) != cudaSuccess) {
+      cudaGetLastError();
+      h->pinned = nullptr;
+    }
+    h->pinned_bytes = kPinnedBytes;  // tried
+  }
+  void* to = h->pinned && bytes <= kPinnedBytes ? h->pinned : dst;
+  MCK(cudaMemcpyAsync(to, src, bytes, cudaMemcpyDeviceToHost, h->stream));
   MCK(cudaStreamSynchronize(h->stream));
+  if (to != dst) memcpy(dst, to, bytes);
 }
 
 // Host -> device copy of a caller's (pageable) array, stream-ordered on the
@@ -567,18 +579,18 @@ using TuneMeasure = std::function<void(const TuneCandidate&, uint32_t sample, do
 // Looks the shape up, or times the candidates on a sample and records the
 // fastest.  Returns false when tuning is off (the defaults then stand).
 bool tune_lookup(mistic_handle_s* h, const mistic_opts& o, uint32_t d, mistic_dtype dt, bool wide, int prec_default,
-                 const uint32_t* bstart, uint32_t m, double eps2, double R, Tuned* out,
+                 const uint32_t* bstart, uint32_t m, size_t n, double eps2, double R, Tuned* out,
                  const TuneMeasure& measure) {
   int want = o.autotune;
   if (const char* e = getenv("MISTIC_AUTOTUNE")) want = atoi(e) > 0 ? 1 : (atoi(e) < 0 || *e == '0' ? -1 : want);
   if (want < 0) return false;
+  if (want == 0 && n < 1000000ull) return false;  // small joins: the defaults, no tuning cost
   unsigned long long* hist_d = abuf<unsigned long long>(h, "tune_hist", 32);
   idx::bin_hist(h, bstart, m, hist_d);
   unsigned long long hist[32];
   d2h(h, hist, hist_d, sizeof hist);
   unsigned long long tot = 0;
   for (int i = 0; i < 32; ++i) tot += hist[i];
-  if (want == 0 && tot < 1000000ull) return false;  // small joins: the defaults, no tuning cost
   int c50 = 0, c90 = 0;
   {
     unsigned long long acc = 0;
@@ -784,35 +796,33 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
   clk.mark();  // 1
 
   // ---- column statistics (+ finiteness) and, for PCA points, a sample covariance
-  const uint32_t cs_parts = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(1, n / 256), 1216);
-  double* cs_part = abuf<double>(h, "cs_part", (size_t)cs_parts * 3 * d);
-  double* cs_out = abuf<double>(h, "cs_out", 3 * (size_t)d);
-  unsigned* flag = abuf<unsigned>(h, "flag", 4);
-  MCK(cudaMemsetAsync(flag, 0, 4 * sizeof(unsigned), h->stream));
-  idx::colstats(h, x, dt, n, d, cs_part, cs_parts, cs_out, flag);
   const bool scored = o.rp_mode == MISTIC_RP_SCORED && k > 0 && d >= 2 && d <= 1024;
   const bool pca = (o.rp_mode == MISTIC_RP_PCA || scored) && k > 0 && d >= 2 && d <= 1024;
+  const uint32_t cs_parts = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(1, n / 64), 1216);
+  double* cs_part = abuf<double>(h, "cs_part", (size_t)cs_parts * 3 * d);
+  // mean, min, max; the non-finite flag; the sample covariance: read back together
+  double* cs_out = abuf<double>(h, "cs_out", 3 * (size_t)d + 1 + (pca ? (size_t)d * d : 0));
+  unsigned* flag = (unsigned*)(cs_out + 3 * (size_t)d);
+  MCK(cudaMemsetAsync(flag, 0, sizeof(double), h->stream));
+  idx::colstats(h, x, dt, n, d, cs_part, cs_parts, cs_out, flag);
   const uint32_t S = (uint32_t)std::min<uint64_t>(n, d <= 64 ? 8192 : 4096);
   double* cov = nullptr;
   double* sbuf = nullptr;
   if (pca) {
     sbuf = abuf<double>(h, "sample", (size_t)S * d);
-    cov = abuf<double>(h, "cov", (size_t)d * d);
-    double* cpart = abuf<double>(h, "cov_part", (size_t)((S + 127) / 128) * d * d);
+    cov = cs_out + 3 * (size_t)d + 1;
+    double* cpart = abuf<double>(h, "cov_part", idx::cov_parts(S, d) * d * d);
     idx::sample_cov(h, x, dt, n, d, S, sbuf, cs_out /* full-data column means */, cpart, cov);
   }
-  std::vector<double> stats(3 * (size_t)d);
-  unsigned nonfinite = 0;
+  std::vector<double> stats(3 * (size_t)d + 1 + (pca ? (size_t)d * d : 0));
   d2h(h, stats.data(), cs_out, stats.size() * sizeof(double));
-  d2h(h, &nonfinite, flag, sizeof(unsigned));
+  unsigned nonfinite = 0;
+  memcpy(&nonfinite, &stats[3 * (size_t)d], sizeof nonfinite);
   if (nonfinite && o.check_finite) throw Error(MISTIC_ERR_NOT_FINITE, "input holds NaN or infinite coordinates");
   std::vector<double> mean(stats.begin(), stats.begin() + d), mn(stats.begin() + d, stats.begin() + 2 * d),
-      mx(stats.begin() + 2 * d, stats.end());
+      mx(stats.begin() + 2 * d, stats.begin() + 3 * d);
   std::vector<double> covh;
-  if (pca) {
-    covh.resize((size_t)d * d);
-    d2h(h, covh.data(), cov, covh.size() * sizeof(double));
-  }
+  if (pca) covh.assign(stats.begin() + 3 * d + 1, stats.end());
   std::vector<double> rps;
   if (scored) {
     std::vector<double> sh((size_t)S * d);
@@ -834,10 +844,10 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
     double* drp = abuf<double>(h, "rps", (size_t)kk * d);
     h2d(h, drp, rps.data(), rps.size() * sizeof(double));
     Dk = abuf<double>(h, "rpdist", n * kk);
-    const uint32_t nparts = (uint32_t)((n + 255) / 256);
-    double* part = abuf<double>(h, "rp_part", (size_t)nparts * 2 * kk);
+    const unsigned tpb = row_block(h, n);
+    double* part = abuf<double>(h, "rp_part", (n + tpb - 1) / tpb * 2 * kk);
     double* mm = abuf<double>(h, "rp_mm", 2 * (size_t)kk);
-    idx::rp_dist(h, x, dt, n, d, drp, (int)kk, Dk, part, nparts, mm);
+    idx::rp_dist(h, x, dt, n, d, drp, (int)kk, Dk, part, mm);
     std::vector<double> mmh(2 * (size_t)kk);
     d2h(h, mmh.data(), mm, mmh.size() * sizeof(double));
     // Field widths.  δ covers the FP64 error of the distances (relative
@@ -908,14 +918,11 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
 
   // ---- bins
   uint32_t* flags = abuf<uint32_t>(h, "binflags", n);
-  uint32_t* nb_dev = abuf<uint32_t>(h, "nbins", 1);
+  double* rmax = abuf<double>(h, "rmax", 2);  // the largest squared norm; the number of bins
+  uint32_t* nb_dev = (uint32_t*)(rmax + 1);
   uint32_t* bstart = abuf<uint32_t>(h, "bstart", n + 1);
   uint64_t* bkey = abuf<uint64_t>(h, "bkey", n);
   idx::bins(h, skeys, n, flags, nb_dev, bstart, bkey);
-  uint32_t m = 0;
-  d2h(h, &m, nb_dev, sizeof(uint32_t));
-  r->n_bins = m;
-
   // ---- mode and sorted-order gather
   bool fp64 = (o.mode == MISTIC_MODE_FP64);
   const uint32_t dpad32 = (d + 3) & ~3u, dpad64 = (d + 1) & ~1u;
@@ -927,12 +934,15 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
   uint32_t* ids = abuf<uint32_t>(h, "ids", n);
   float* xf = fp64 ? nullptr : abuf<float>(h, "xf", n * dpad32);
   double* xd = fp64 ? abuf<double>(h, "xd", n * dpad64) : nullptr;
-  const uint32_t gparts = (uint32_t)((n + 255) / 256);
-  double* npart = abuf<double>(h, "norm_part", gparts);
-  double* rmax = abuf<double>(h, "rmax", 1);
+  const unsigned gblk = row_block(h, n);
+  double* npart = abuf<double>(h, "norm_part", (n + gblk - 1) / gblk);
   idx::gather(h, x, dt, n, d, perm, dcenter, fp64 ? 0 : dpad32, xf, fp64 ? dpad64 : 0, xd, ids, npart, rmax);
-  double R2 = 0;
-  d2h(h, &R2, rmax, sizeof(double));
+  double rm[2] = {0, 0};
+  d2h(h, rm, rmax, sizeof rm);
+  const double R2 = rm[0];
+  uint32_t m = 0;
+  memcpy(&m, &rm[1], sizeof m);
+  r->n_bins = m;
   const double R = sqrt(R2) * (1.0 + 1e-12);
   float t_lo = 0, t_hi = 0;
   if (!fp64) {
@@ -1152,7 +1162,7 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
   int prec_used = prec;
   if (use_tc && !tf32_mode) {
     Tuned tu;
-    if (tune_lookup(h, o, d, dt, wide, prec, bstart, m, eps2, R, &tu, [&](const TuneCandidate& c, uint32_t S,
+    if (tune_lookup(h, o, d, dt, wide, prec, bstart, m, n, eps2, R, &tu, [&](const TuneCandidate& c, uint32_t S,
                                                                            double* ms_out, unsigned long long* cands,
                                                                            unsigned long long* nunits) {
           EnumParams e2 = ep;
@@ -1491,14 +1501,15 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
   jp.cap = cap;
   jp.pairs_ij = host_direct ? 1 : 0;
   size_band(totc);
-  JoinCounters hc{};
+  JoinCounters hcs[2]{};  // CUDA-core join and band decisions; tensor-core join
+  JoinCounters& hc = hcs[0];
   // MISTIC_TEST_JOIN_ATTEMPTS=k caps the passes (tests of the exit check below)
   int attempts = 3;
   if (const char* e = getenv("MISTIC_TEST_JOIN_ATTEMPTS")) attempts = std::max(1, atoi(e));
   bool complete = false;
   for (int attempt = 0; attempt < attempts; ++attempt) {
     launch_join(o.timing != 0);
-    d2h(h, &hc, ctr, sizeof hc);
+    d2h(h, hcs, ctr, sizeof hcs);
     if (hc.error) throw Error(MISTIC_ERR_TIMEOUT, "a tensor-core tile wait timed out");
     if (hc.band_n > jp.band_cap) {  // band list overflowed: nothing beyond it was decided, run again
       jp.band_cap = hc.band_n + hc.band_n / 4;
@@ -1531,8 +1542,7 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
   r->tc_operands = (use_tc && tots[2] > 0) ? (wide ? 1 + prec_used : 1) : 0;
   r->tc_kernel = (use_tc && tots[2] > 0) ? (wide ? 2 : 1) : 0;
   if (use_tc) {
-    JoinCounters tcc{};
-    d2h(h, &tcc, ctr + 1, sizeof tcc);
+    const JoinCounters& tcc = hcs[1];
     r->tc_tiles = tcc.tiles;
     r->tc_cells = tcc.cells;
     if (tp.prof && tp.xh) {

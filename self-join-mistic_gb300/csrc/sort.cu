@@ -5,7 +5,7 @@
 // the device: 8-bit digits, one histogram pass and one stable scatter pass per
 // digit, only over the bits the packed key actually uses.
 //
-// Scatter ranking: each warp owns a contiguous run of 512 elements and ranks
+// Scatter ranking: each warp owns a contiguous run of elements and ranks
 // them 32 at a time with __match_any_sync, keeping per-warp digit counters in
 // shared memory; a per-digit prefix over the 8 warps then gives every
 // element its position inside the tile, and the digit-major scan of the
@@ -193,13 +193,17 @@ void exclusive_scan3(mistic_handle_s* h, uint32_t* a, uint32_t* b, uint32_t* c, 
 
 constexpr int RS_THREADS = 256;
 constexpr int RS_WARPS = RS_THREADS / 32;
-constexpr int RS_ROUNDS = 16;                        // 32-element rounds per warp
-constexpr int RS_TILE = RS_THREADS * RS_ROUNDS;      // 4096 elements per block
+// Tiles of RS_THREADS * ROUNDS elements, ROUNDS 32-element rounds per warp: 16,
+// fewer for inputs whose few tiles would leave most SMs idle (4,000 elements
+// are one tile of 16 rounds, 8 of 2).
+constexpr int rs_rounds(size_t n) { return n <= 65536 ? 2 : (n <= 262144 ? 8 : 16); }
 constexpr int RS_BINS = 256;
 
+template <int RS_ROUNDS>
 __global__ void k_rs_hist(const uint64_t* __restrict__ keys, size_t n, int shift,
                           uint32_t* __restrict__ hist, uint32_t tiles) {
   __shared__ uint32_t cnt[RS_BINS];
+  constexpr int RS_TILE = RS_THREADS * RS_ROUNDS;
   cnt[threadIdx.x] = 0;
   __syncthreads();
   const size_t base = (size_t)blockIdx.x * RS_TILE;
@@ -211,7 +215,7 @@ __global__ void k_rs_hist(const uint64_t* __restrict__ keys, size_t n, int shift
   hist[(size_t)threadIdx.x * tiles + blockIdx.x] = cnt[threadIdx.x];
 }
 
-template <bool IOTA>
+template <bool IOTA, int RS_ROUNDS>
 __global__ void __launch_bounds__(RS_THREADS)
 k_rs_scatter(const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin,
              uint64_t* __restrict__ kout, uint32_t* __restrict__ vout, size_t n,
@@ -221,7 +225,7 @@ k_rs_scatter(const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin,
   __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const unsigned lt_mask = (1u << lane) - 1u;
-  const size_t base = (size_t)blockIdx.x * RS_TILE + (size_t)w * (RS_ROUNDS * 32);
+  const size_t base = (size_t)blockIdx.x * (RS_THREADS * RS_ROUNDS) + (size_t)w * (RS_ROUNDS * 32);
   uint64_t key[RS_ROUNDS];
   uint32_t val[RS_ROUNDS];
   uint32_t rank[RS_ROUNDS];
@@ -266,29 +270,39 @@ k_rs_scatter(const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin,
   }
 }
 
+template <int ROUNDS>
+static int radix_sort_rounds(mistic_handle_s* h, uint64_t* keys[2], uint32_t* vals[2], size_t n, int bits) {
+  constexpr size_t tile = (size_t)RS_THREADS * ROUNDS;
+  const uint32_t tiles = (uint32_t)((n + tile - 1) / tile);
+  uint32_t* hist = (uint32_t*)h->arena.get("rs_hist", (size_t)RS_BINS * tiles * sizeof(uint32_t));
+  int cur = 0;
+  for (int shift = 0; shift < bits; shift += 8) {
+    k_rs_hist<ROUNDS><<<tiles, RS_THREADS, 0, h->stream>>>(keys[cur], n, shift, hist, tiles);
+    launched(h, "rs_hist");
+    exclusive_scan<uint32_t>(h, hist, hist, (size_t)RS_BINS * tiles, nullptr);
+    if (shift == 0)
+      k_rs_scatter<true, ROUNDS><<<tiles, RS_THREADS, 0, h->stream>>>(keys[cur], nullptr, keys[cur ^ 1],
+                                                                      vals[cur ^ 1], n, shift, hist, tiles);
+    else
+      k_rs_scatter<false, ROUNDS><<<tiles, RS_THREADS, 0, h->stream>>>(keys[cur], vals[cur], keys[cur ^ 1],
+                                                                       vals[cur ^ 1], n, shift, hist, tiles);
+    launched(h, "rs_scatter");
+    cur ^= 1;
+  }
+  return cur;
+}
+
 int radix_sort_u64(mistic_handle_s* h, uint64_t* keys[2], uint32_t* vals[2], size_t n, int bits) {
   if (n <= 1 || bits <= 0) {
     if (n == 1) MCK(cudaMemsetAsync(vals[0], 0, sizeof(uint32_t), h->stream));
     return 0;
   }
   if (n > 0xffffffffull) throw Error(MISTIC_ERR_TOO_LARGE, "radix sort supports < 2^32 elements");
-  const uint32_t tiles = (uint32_t)((n + RS_TILE - 1) / RS_TILE);
-  uint32_t* hist = (uint32_t*)h->arena.get("rs_hist", (size_t)RS_BINS * tiles * sizeof(uint32_t));
-  int cur = 0;
-  for (int shift = 0; shift < bits; shift += 8) {
-    k_rs_hist<<<tiles, RS_THREADS, 0, h->stream>>>(keys[cur], n, shift, hist, tiles);
-    launched(h, "rs_hist");
-    exclusive_scan<uint32_t>(h, hist, hist, (size_t)RS_BINS * tiles, nullptr);
-    if (shift == 0)
-      k_rs_scatter<true><<<tiles, RS_THREADS, 0, h->stream>>>(keys[cur], nullptr, keys[cur ^ 1], vals[cur ^ 1], n,
-                                                              shift, hist, tiles);
-    else
-      k_rs_scatter<false><<<tiles, RS_THREADS, 0, h->stream>>>(keys[cur], vals[cur], keys[cur ^ 1], vals[cur ^ 1], n,
-                                                               shift, hist, tiles);
-    launched(h, "rs_scatter");
-    cur ^= 1;
+  switch (rs_rounds(n)) {
+    case 2: return radix_sort_rounds<2>(h, keys, vals, n, bits);
+    case 8: return radix_sort_rounds<8>(h, keys, vals, n, bits);
+    default: return radix_sort_rounds<16>(h, keys, vals, n, bits);
   }
-  return cur;
 }
 
 }  // namespace mistic
