@@ -881,46 +881,77 @@ __global__ void __launch_bounds__(WTHREADS, 1)
         // columns c in [hlo, lim) hold home rows q <= a (dropped: each pair once, no self pair)
         const uint32_t lim = (hlo < hhi && a_sorted >= hq0) ? min(hhi, hlo + min(a_sorted - hq0 + 1, (uint32_t)WN)) : 0u;
         if (g * WM + quarter * 32 < nrows) {
+          unsigned long long na2, neg2;
+          asm("mov.b64 %0, {%1, %1};" : "=l"(na2) : "f"(na));
+          asm("mov.b64 %0, {%1, %1};" : "=l"(neg2) : "f"(-2.f));
 #pragma unroll 1
           for (uint32_t c0 = 32 * cblk0; c0 < ncols; c0 += 32 * (WNEPI / 4)) {
             uint32_t v[32];
             tmem_ld32_nowait(tbase + g * WN + ((quarter * 32u) << 16) + c0, v);
             tmem_wait();
+            // D' = fma(-2, G, |a|^2) + (|q|^2 - T), two columns an instruction
+            // (packed FP32, each lane rounded as the scalar operations)
             uint32_t o = 0;
 #pragma unroll
             for (int j = 0; j < 32; j += 4) {
-              const float4 h4 = *reinterpret_cast<const float4*>(&Gm.hq[c0 + j]);
-              const float hv[4] = {h4.x, h4.y, h4.z, h4.w};
+              const ulonglong2 h2 = *reinterpret_cast<const ulonglong2*>(&Gm.hq[c0 + j]);
 #pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                const float dv = fmaf(-2.f, __uint_as_float(v[j + i]), na) + hv[i];
-                v[j + i] = __float_as_uint(dv);
-                o |= v[j + i];
+              for (int i = 0; i < 2; ++i) {
+                unsigned long long t;
+                asm("mov.b64 %0, {%1, %2};" : "=l"(t) : "r"(v[j + 2 * i]), "r"(v[j + 2 * i + 1]));
+                asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(t) : "l"(neg2), "l"(na2));
+                asm("add.rn.f32x2 %0, %0, %1;" : "+l"(t) : "l"(i ? h2.y : h2.x));
+                asm("mov.b64 {%0, %1}, %2;" : "=r"(v[j + 2 * i]), "=r"(v[j + 2 * i + 1]) : "l"(t));
+                o |= v[j + 2 * i] | v[j + 2 * i + 1];
               }
             }
-            uint32_t acc_bits = 0, band_bits = 0;
-            const uint32_t nvalid = min(32u, ncols - c0);
-            const bool maybe = row_ok && (o >> 31);
-            if (__any_sync(FULL_MASK, maybe)) {
-              if (maybe) {
-                uint32_t m = 0;
+            if (!__any_sync(FULL_MASK, row_ok && (o >> 31))) continue;
+            // sign bits, column c0 + j at bit j, in four independent chains of 8
+            auto signs = [&]() {
+              uint32_t m0 = 0, m1 = 0, m2 = 0, m3 = 0;
 #pragma unroll
-                for (int j = 0; j < 32; ++j) m |= (v[j] >> 31) << j;
-                m &= nvalid >= 32 ? FULL_MASK : ((1u << nvalid) - 1u);
-                const int e0 = (int)max(hlo, c0) - (int)c0, e1 = (int)min(lim, c0 + 32) - (int)c0;
-                if (e0 < e1) m &= ~((e1 >= 32 ? FULL_MASK : ((1u << e1) - 1u)) & ~((1u << e0) - 1u));
-                while (m) {
-                  const int j = __ffs(m) - 1;
-                  m &= m - 1;
-                  if (pick32(v, j) <= -Gm.dlt[c0 + j])
-                    acc_bits |= 1u << j;
-                  else
-                    band_bits |= 1u << j;  // decided later in FP64 (band list)
-                }
+              for (int j = 7; j >= 0; --j) {
+                m0 = __funnelshift_l(v[j], m0, 1);
+                m1 = __funnelshift_l(v[8 + j], m1, 1);
+                m2 = __funnelshift_l(v[16 + j], m2, 1);
+                m3 = __funnelshift_l(v[24 + j], m3, 1);
               }
+              return m0 | (m1 << 8) | (m2 << 16) | (m3 << 24);
+            };
+            uint32_t m = row_ok ? signs() : 0u;
+            const uint32_t nvalid = ncols - c0;
+            if (nvalid < 32) m &= (1u << nvalid) - 1u;
+            const int e0 = (int)max(hlo, c0) - (int)c0, e1 = (int)min(lim, c0 + 32) - (int)c0;
+            if (e0 < e1) m &= ~((e1 >= 32 ? FULL_MASK : ((1u << e1) - 1u)) & ~((1u << e0) - 1u));
+            if (!__any_sync(FULL_MASK, m != 0)) continue;
+            const float* dlt = &Gm.dlt[c0];
+            const uint32_t* qids = &Gm.qid[c0];
+            const uint32_t ia = m ? Gm.aid[row] : 0u;
+            if (!__any_sync(FULL_MASK, (m & (m - 1)) != 0)) {
+              // at most one candidate a lane (most blocks that hold any)
+              bool acc = false, band = false;
+              unsigned long long pr = 0;
+              if (m) {
+                const int j = __ffs(m) - 1;
+                const uint32_t iq = qids[j];
+                acc = pick32(v, j) <= -dlt[j];
+                band = !acc;  // decided later in FP64
+                pr = ((unsigned long long)min(ia, iq) << 32) | max(ia, iq);
+              }
+              stage_one(ps, acc, pr, &P.ctr->pairs, P.pairs, P.cap, nullptr, Gm.tag, rcp);
+              stage_one(bs, band, pr, &P.ctr->band_n, P.band_list, P.band_cap, nullptr, Gm.tag, rcb);
+              continue;
             }
-            __syncwarp();
-            const uint32_t ia = (acc_bits | band_bits) ? Gm.aid[row] : 0u;
+            // D' + dlt < 0: accepted (an infinite dlt accepts nothing)
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+              const float4 d4 = *reinterpret_cast<const float4*>(dlt + j);
+              v[j] = __float_as_uint(__uint_as_float(v[j]) + d4.x);
+              v[j + 1] = __float_as_uint(__uint_as_float(v[j + 1]) + d4.y);
+              v[j + 2] = __float_as_uint(__uint_as_float(v[j + 2]) + d4.z);
+              v[j + 3] = __float_as_uint(__uint_as_float(v[j + 3]) + d4.w);
+            }
+            const uint32_t acc_bits = m & signs();
             auto emit = [&](PairStage& stg, uint32_t bits, unsigned long long* counter, unsigned long long* list,
                             unsigned long long lcap, const RingCtx* rc) {
               stage_pairs(
@@ -928,15 +959,15 @@ __global__ void __launch_bounds__(WTHREADS, 1)
                   [&](uint32_t) {
                     const int j = __ffs(bits) - 1;
                     bits &= bits - 1;
-                    const uint32_t iq = Gm.qid[c0 + j];
-                    const uint32_t lo = ia < iq ? ia : iq, hi = ia < iq ? iq : ia;
-                    return ((unsigned long long)lo << 32) | hi;
+                    const uint32_t iq = qids[j];
+                    return ((unsigned long long)min(ia, iq) << 32) | max(ia, iq);
                   },
                   counter, list, lcap, nullptr, Gm.tag, rc);
             };
-            if (__any_sync(FULL_MASK, acc_bits != 0u)) emit(ps, acc_bits, &P.ctr->pairs, P.pairs, P.cap, rcp);
-            if (__any_sync(FULL_MASK, band_bits != 0u))
-              emit(bs, band_bits, &P.ctr->band_n, P.band_list, P.band_cap, rcb);
+            emit(ps, acc_bits, &P.ctr->pairs, P.pairs, P.cap, rcp);
+            // the band is decided later in FP64
+            if (__any_sync(FULL_MASK, m != acc_bits))
+              emit(bs, m & ~acc_bits, &P.ctr->band_n, P.band_list, P.band_cap, rcb);
           }
         }
         asm volatile("tcgen05.fence::before_thread_sync;");
