@@ -761,16 +761,19 @@ __global__ void __launch_bounds__(WTHREADS, 1)
         // held back) once accumulator 1 is free.  nd stages are deferred,
         // from global step d0; all stages deferred means the ring is full,
         // and then the lane waits.
+        // Chunk 0 leads chunk 1: by up to the whole ring while the epilogue still
+        // drains accumulator 1, by `lag` stages afterwards, and accumulator 0
+        // is handed over as soon as its own last MMA is issued, so that it is
+        // drained while chunk 1 finishes.  (Both handed over together, the
+        // next group waited for the drain: 515,345 x 90 70.3 ms against 64.3,
+        // 1M x 384 308 against 290.)  A lag of one stage pays only where a
+        // group has few stages (515,345 x 90, 3 stages: 64.3 / 65.1 ms with and
+        // without; 1M x 384, 6 stages: 296 / 290): it keeps a stage from the
+        // producers.
+        const uint32_t lag = nkc <= 3 ? 1u : 0u;
         const uint32_t step0 = step;
-        uint32_t nd = 0, d0 = 0;
-        auto catch_up = [&]() {
-          asm volatile("tcgen05.fence::after_thread_sync;");
-          for (uint32_t i = 0; i < nd; ++i) {
-            issue(1, d0 + i - step0, (d0 + i) % WNS);
-            release(d0 + i);
-          }
-          nd = 0;
-        };
+        uint32_t nd = 0;     // stages chunk 1 still has to read, the last of them step - 1
+        bool free1 = false;  // accumulator 1 taken for this group
         for (uint32_t kc = 0; kc < nkc && ok; ++kc) {
           if (kc > 0) {
             s = step % WNS;
@@ -793,36 +796,40 @@ __global__ void __launch_bounds__(WTHREADS, 1)
             asm volatile("tcgen05.fence::after_thread_sync;");
           }
           issue(0, kc, s);
+          ++step;
+          if (kc + 1 == nkc) {
+            tc_commit(&S.dfull[0]);
+            last_bar = &S.dfull[0];
+            last_par = use[0] & 1;
+          }
           if (ng > 1) {
-            if (nd > 0 && mbar_ready(&S.dfree[1], (use[1] & 1) ^ 1)) catch_up();
-            if (nd > 0) {
-              ++nd;  // this stage's chunk 1 waits too
-            } else if (kc == 0 && !mbar_ready(&S.dfree[1], (use[1] & 1) ^ 1)) {
-              nd = 1;
-              d0 = step;
-            } else {
-              if (kc == 0) asm volatile("tcgen05.fence::after_thread_sync;");
-              issue(1, kc, s);
-              release(step);
-            }
-            if (nd >= (uint32_t)WNS || (nd > 0 && kc + 1 == nkc)) {  // ring held or group done: wait for accumulator 1
+            ++nd;
+            const bool must = nd >= (uint32_t)WNS || kc + 1 == nkc;  // ring held or group done
+            if (!free1 && (must || mbar_ready(&S.dfree[1], (use[1] & 1) ^ 1))) {
               const long long c2 = T.prof ? clock64() : 0;
               ok = wait_or_abort(&S.dfree[1], (use[1] & 1) ^ 1, abort_flag, T.wait_limit);
               if (T.prof) mw_dfree += clock64() - c2;
               if (!ok) break;
-              catch_up();
+              asm volatile("tcgen05.fence::after_thread_sync;");
+              free1 = true;
+            }
+            while (free1 && nd > (kc + 1 == nkc ? 0u : lag)) {
+              const uint32_t e = step - nd;
+              issue(1, e - step0, e % WNS);
+              release(e);
+              --nd;
             }
           } else {
-            release(step);
+            release(step - 1);
           }
-          ++step;
         }
         if (!ok) break;
-        for (uint32_t g = 0; g < ng; ++g) {
-          tc_commit(&S.dfull[g]);
-          last_bar = &S.dfull[g];
-          last_par = use[g] & 1;
-          ++use[g];
+        ++use[0];
+        if (ng > 1) {
+          tc_commit(&S.dfull[1]);
+          last_bar = &S.dfull[1];
+          last_par = use[1] & 1;
+          ++use[1];
         }
         ++group;
       }
