@@ -205,67 +205,57 @@ __device__ __forceinline__ uint32_t home_mask(uint32_t na, bool self, uint32_t q
   return CH >= 32 ? m : (m & ((1u << CH) - 1u));
 }
 
-// Candidate stream of one unit: the points of its neighbour bins from entry s
-// on in order, 32 per tile, lanes filled across bin boundaries
-// (bins average a few points, so one bin per tile would leave most lanes
-// idle).  `s` and `off` (next bin, offset inside the unit's part of it) are
-// warp-uniform.
-// Each lane gets its candidate's sorted position q, or qv = false past the
-// end.  Lane l finds its bin by a binary search over the warp's inclusive
-// scan of up to 32 bin sizes.
+// Candidate stream of one unit: the points of its neighbour bins in order, 32
+// per tile, lanes filled across bin boundaries (bins average a few points, so
+// one bin per tile would leave most lanes idle).  A window of 64 bins, two a
+// lane, stays in registers until its points are handed out; a tile then costs
+// two ballots, one OR over the warp and two shuffles to find every lane's
+// bin, and no memory access.  (Reading 32 bins afresh for every tile and
+// searching them by shuffles cost as much as the distances to 6 home rows:
+// 5M x 18 CUDA-core join at T = 49 23.6 -> 22.0 ms.)
 struct CandTile {
-  uint32_t q;
-  bool qv;
+  uint32_t q;  // this lane's candidate (sorted position)
+  bool qv;     // it has one
 };
 
-__device__ __forceinline__ CandTile next_tile(const Unit& U, uint32_t ch, const uint32_t* nbr, const uint32_t* bstart,
-                                              uint32_t& s, uint32_t& off) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t bj = s + lane, s1 = U.s1;
-  uint32_t start = 0, size = 0;
-  if (bj < s1) {
-    uint32_t b;
-    unit_bin(U, ch, nbr, bstart, bj, &b, &start, &size);
-    if (lane == 0) {
-      start += off;
-      size -= off;
+struct CandStream {
+  uint32_t s, total, pos;       // next neighbour entry; points of the window, handed out so far
+  uint32_t end0, end1;          // ranks in the window at which this lane's two bins end
+  uint32_t base0, base1;        // sorted position of rank 0, were the bin extended to it
+
+  __device__ __forceinline__ explicit CandStream(const Unit& U) : s(U.s0), total(0), pos(0) {}
+
+  // The next tile; false at the unit's end.
+  __device__ __forceinline__ bool next(const Unit& U, uint32_t ch, const uint32_t* nbr, const uint32_t* bstart,
+                                       CandTile* t) {
+    const int lane = threadIdx.x & 31;
+    while (pos >= total) {
+      if (s >= U.s1) return false;
+      uint32_t b, st0 = 0, sz0 = 0, st1 = 0, sz1 = 0;
+      if (s + 2 * lane < U.s1) unit_bin(U, ch, nbr, bstart, s + 2 * lane, &b, &st0, &sz0);
+      if (s + 2 * lane + 1 < U.s1) unit_bin(U, ch, nbr, bstart, s + 2 * lane + 1, &b, &st1, &sz1);
+      end1 = warp_incl_scan_u32(sz0 + sz1);
+      end0 = end1 - sz1;
+      base0 = st0 - (end0 - sz0);
+      base1 = st1 - end0;
+      total = __shfl_sync(FULL_MASK, end1, 31);
+      pos = 0;
+      s = min(s + 64, U.s1);
     }
+    // bins that end at or before the tile's first rank, and the ends among its
+    // 32 ranks (entries past the list end where the window does)
+    const uint32_t r0 = pos, t0 = end0 - r0, t1 = end1 - r0;
+    const uint32_t done = __popc(__ballot_sync(FULL_MASK, end0 <= r0)) + __popc(__ballot_sync(FULL_MASK, end1 <= r0));
+    const uint32_t ends = __reduce_or_sync(
+        FULL_MASK, (end0 > r0 && t0 < 32u ? 1u << t0 : 0u) | (end1 > r0 && t1 < 32u ? 1u << t1 : 0u));
+    const uint32_t j = done + __popc(ends & ((2u << lane) - 1u));
+    const uint32_t p0 = __shfl_sync(FULL_MASK, base0, (j >> 1) & 31u), p1 = __shfl_sync(FULL_MASK, base1, (j >> 1) & 31u);
+    t->q = ((j & 1u) ? p1 : p0) + r0 + lane;
+    t->qv = r0 + lane < total;
+    pos += 32;
+    return true;
   }
-  const uint32_t incl = warp_incl_scan_u32(size);
-  const uint32_t total = __shfl_sync(FULL_MASK, incl, 31);
-  // j = first window bin whose inclusive end exceeds this lane's rank
-  int lo = 0, hi = 31;
-#pragma unroll
-  for (int it = 0; it < 5; ++it) {
-    const int mid = (lo + hi) >> 1;
-    const uint32_t v = __shfl_sync(FULL_MASK, incl, mid);
-    if (v <= (uint32_t)lane) lo = mid + 1; else hi = mid;
-  }
-  const int j = lo;
-  const uint32_t sj = __shfl_sync(FULL_MASK, start, j);
-  const uint32_t ej = __shfl_sync(FULL_MASK, incl, j);
-  const uint32_t zj = __shfl_sync(FULL_MASK, size, j);
-  CandTile t;
-  t.qv = (uint32_t)lane < total;
-  t.q = sj + (uint32_t)lane - (ej - zj);
-  // advance past the 32 candidates handed out
-  if (total > 32) {
-    const int j31 = __shfl_sync(FULL_MASK, j, 31);
-    const uint32_t e31 = __shfl_sync(FULL_MASK, ej, 31), z31 = __shfl_sync(FULL_MASK, zj, 31);
-    const uint32_t used = 32 - (e31 - z31);  // candidates taken from bin j31
-    if (used < z31) {
-      off = (j31 == 0 ? off : 0u) + used;
-      s += j31;
-    } else {
-      off = 0;
-      s += j31 + 1;
-    }
-  } else {
-    s = min(s + 32, s1);
-    off = 0;
-  }
-  return t;
-}
+};
 
 // ---------------------------------------------------------------- FP32 filter
 // Distance of lane candidate (qrow) to the CH staged home rows, dims
@@ -328,9 +318,9 @@ k_join_f32(const JoinParams P) {
     for (uint32_t i = lane; i < CH * nq4; i += 32)
       sA[i] = i < na * nq4 ? X[(size_t)a0 * nq4 + i] : make_float4(0.f, 0.f, 0.f, 0.f);
     __syncwarp();
-    uint32_t s = U.s0, off = 0;
-    while (s < U.s1) {
-      const CandTile t = next_tile(U, CH, V.nbr, V.bstart, s, off);
+    CandStream cs(U);
+    CandTile t;
+    while (cs.next(U, CH, V.nbr, V.bstart, &t)) {
       const uint32_t q = t.q;
       const float4* qrow = X + (size_t)(t.qv ? q : a0) * nq4;
       float acc[CH];
@@ -395,9 +385,9 @@ k_join_f32r(const JoinParams P) {
     for (uint32_t i = lane; i < CH * DQ; i += 32)
       sA[i] = i < na * DQ ? X[(size_t)a0 * DQ + i] : make_float4(0.f, 0.f, 0.f, 0.f);
     __syncwarp();
-    uint32_t s = U.s0, off = 0;
-    while (s < U.s1) {
-      const CandTile t = next_tile(U, CH, V.nbr, V.bstart, s, off);
+    CandStream cs(U);
+    CandTile t;
+    while (cs.next(U, CH, V.nbr, V.bstart, &t)) {
       const uint32_t q = t.q;
       const ulonglong2* qrow = reinterpret_cast<const ulonglong2*>(X + (size_t)(t.qv ? q : a0) * DQ);
       ulonglong2 qq[DQ];  // the candidate row as pairs of floats
@@ -525,9 +515,9 @@ k_join_f64(const JoinParams P) {
     for (uint32_t i = lane; i < CH * nq2; i += 32)
       sA[i] = i < na * nq2 ? X[(size_t)a0 * nq2 + i] : make_double2(0.0, 0.0);
     __syncwarp();
-    uint32_t s = U.s0, off = 0;
-    while (s < U.s1) {
-      const CandTile t = next_tile(U, CH, V.nbr, V.bstart, s, off);
+    CandStream cs(U);
+    CandTile t;
+    while (cs.next(U, CH, V.nbr, V.bstart, &t)) {
       const uint32_t q = t.q;
       const double2* qrow = X + (size_t)(t.qv ? q : a0) * nq2;
       double acc[CH];
