@@ -77,7 +77,8 @@ constexpr int WNPROD = WNPW * 32;
 constexpr int WNEPI = 16;    // epilogue warps: 4 TMEM lane quarters x 4 column groups
 constexpr int WEPI0 = WNPW;  // first epilogue warp (a multiple of 4: warp % 4 is its lane quarter)
 constexpr int WMMA = WEPI0 + WNEPI;
-constexpr int WTHREADS = (WMMA + 1) * 32;
+constexpr int WTMA = WMMA + 1;  // issues the stages of contiguous groups
+constexpr int WTHREADS = (WTMA + 1) * 32;
 constexpr int WGS = 2;       // group metadata slots
 // stage layout (bytes): home hi | home lo (by TMA) | candidates hi |
 // candidates lo (by cp.async), all as 64-byte rows in the 64B swizzle
@@ -111,6 +112,7 @@ struct __align__(16) WGroup {
   uint32_t a0, nrows, ncols, ng, flags;
   uint32_t hlo, hhi, hq0;  // columns [hlo, hhi) are home-bin rows, column hlo at sorted position hq0
   uint32_t tag;            // the pair ring's tag of the group's unit (0 outside ring mode)
+  uint32_t run, qf;        // run: the candidates are the sorted rows qf, qf + 1, ...; the TMA warp fetches them
 };
 
 struct WShared {
@@ -124,7 +126,7 @@ struct WShared {
   uint32_t abort_flag;
   uint32_t tmem_base;
   uint32_t pflag[2];
-  unsigned long long full[WNS], afull[WNS], sfree[WNS], dfull[WG], dfree[WG], gfree[WGS], gready[WGS];
+  unsigned long long full[WNS], afull[WNS], sfree[WNS], dfull[WG], dfree[WG], gfree[WGS], gready[WGS], tpass[WGS];
 };
 
 __device__ __forceinline__ void wprod_sync() { asm volatile("bar.sync 1, %0;" ::"n"(WNPROD) : "memory"); }
@@ -273,13 +275,18 @@ __global__ void k_tf32_rows(const float* __restrict__ xf, uint32_t dpad32, uint3
 }
 
 // ---------------------------------------------------------------- pipeline
-// One persistent CTA per SM: 8 producer warps, 16 epilogue warps, 1 MMA warp.
+// One persistent CTA per SM: 8 producer warps, 16 epilogue warps, 1 MMA warp,
+// 1 TMA warp.
 //   producers  fetch units; per group of up to 256 candidates all 8 warps
 //              compute the columns' sorted positions, ids, norms and
-//              thresholds; then, per K chunk, thread 0 issues the stage's
-//              TMA tiles (home rows, and the candidate rows of a contiguous
-//              group) against one expect_tx on afull, and every producer
-//              thread copies its scattered candidate rows by cp.async;
+//              thresholds; for scattered candidates, per K chunk, thread 0
+//              issues the home rows' TMA tiles against one expect_tx on afull
+//              and every producer thread copies its candidate rows by cp.async;
+//   TMA warp   one lane issues every stage of the groups whose candidates are
+//              one contiguous run (up to 8 TMA tiles a stage) while the
+//              producers prepare the next group: with producer thread 0 doing
+//              both, issuing took 37 % of its time at 515,345 x 90 and the MMA
+//              lane waited for stages 25 % of its own;
 //   MMA warp   one lane issues 2 x 3 tcgen05.mma (K 16, M 128, N up to 256)
 //              per home chunk and stage, commits each stage to sfree and, at
 //              a group's last stage, each accumulator to dfull;
@@ -287,13 +294,18 @@ __global__ void k_tf32_rows(const float* __restrict__ xf, uint32_t dpad32, uint3
 //              sign-bit test, home-bin rule by column range, sure accepts
 //              to the pair list, the error band to the band list.
 // Barriers (all waits bounded by a %globaltimer deadline):
-//   full[s]   producers -> MMA       (WNPROD cp.async arrivals: candidate rows landed)
-//   afull[s]  producer 0 -> MMA      (one arrive.expect_tx + the bytes of the stage's TMA tiles)
-//   gready[x] producers -> MMA       (WNPROD arrivals: group slot x written)
+//   full[s]   producers -> MMA       (WNPROD cp.async arrivals: candidate rows landed; or the TMA lane at once)
+//   afull[s]  producer 0 or TMA -> MMA  (one arrive.expect_tx + the bytes of the stage's TMA tiles)
+//   gready[x] producers -> MMA, TMA  (WNPROD arrivals: group slot x written)
+//   tpass[x]  TMA -> producers       (1 arrival: every stage up to group slot x's is issued)
+// A wait on sfree[s] tells only whether the stage's last use but one is over
+// (phases alternate), so whoever fills the stages of a group waits until the
+// groups before it are issued: the producers through tpass, the TMA lane
+// through gready, which every producer joins after its own copies.
 //   sfree[s]  MMA -> producers       (tcgen05.commit: stage s read)
 //   dfull[g]  MMA -> epilogue        (tcgen05.commit, or a plain arrive to stop)
 //   dfree[g]  epilogue -> MMA        (WNEPI arrivals; accumulator g reusable)
-//   gfree[x]  epilogue -> producers  (WNEPI arrivals; group slot x reusable)
+//   gfree[x]  epilogue, TMA -> producers  (WNEPI + 1 arrivals; group slot x reusable)
 template <int PREC>
 __global__ void __launch_bounds__(WTHREADS, 1)
     k_join_tcw(const JoinParams P, const TcParams T, const __grid_constant__ TcwMaps M) {
@@ -321,8 +333,9 @@ __global__ void __launch_bounds__(WTHREADS, 1)
       mbar_init(&S.dfree[i], WNEPI);
     }
     for (int i = 0; i < WGS; ++i) {
-      mbar_init(&S.gfree[i], WNEPI);
+      mbar_init(&S.gfree[i], WNEPI + 1);
       mbar_init(&S.gready[i], WNPROD);
+      mbar_init(&S.tpass[i], 1);
     }
     asm volatile("fence.mbarrier_init.release.cluster;");
     S.abort_flag = 0;
@@ -337,10 +350,31 @@ __global__ void __launch_bounds__(WTHREADS, 1)
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tbase = S.tmem_base;
 
+  const uint64_t map_ah = reinterpret_cast<uint64_t>(&M.ah), map_al = reinterpret_cast<uint64_t>(&M.al);
+  // issues the home rows' tiles of K chunk kc into the stage at sb
+  auto home_tiles = [&](uint32_t sb, uint32_t kc, uint32_t a0, uint32_t ng, uint32_t ab) {
+    for (uint32_t g = 0; g < ng; ++g) {
+      if (PREC == 0) {
+        tma_tile_2d(sb + g * A_CHUNK, map_ah, (int)(kc * WKC), (int)(a0 + g * WM), ab);
+        tma_tile_2d(sb + A_LO + g * A_CHUNK, map_al, (int)(kc * WKC), (int)(a0 + g * WM), ab);
+      } else {
+        tma_tile_2d(sb + g * S_ACHUNK, map_ah, (int)(kc * KST), (int)(a0 + g * WM), ab);
+      }
+    }
+  };
+  // an aborting CTA may still have TMA copies in flight into its stages: the
+  // thread that issued them waits (bounded) until they have landed
+  auto drain = [&](const uint32_t (&mine)[WNS]) {
+    if (!*abort_flag) return;
+    volatile uint32_t no_abort = 0;
+    for (int s = 0; s < WNS; ++s)
+      if (mine[s]) wait_or_abort(&S.afull[s], ((mine[s] - 1) / WNS) & 1, &no_abort, T.wait_limit);
+  };
+
   if (warp < WNPW) {
     // ============================ producers
-    // All 8 warps prepare each group (candidate positions, ids, thresholds);
-    // warp 0 then issues the group's stages as TMA copies.  Every branch that
+    // All 8 warps prepare each group (candidate positions, ids, thresholds) and
+    // copy the candidate rows of scattered ones.  Every branch that
     // leads to bar.sync is taken on a value all producer threads hold in
     // registers or read from shared memory after the same bar.sync; barrier
     // waits shared by all producers are done by thread 0 and broadcast
@@ -351,10 +385,10 @@ __global__ void __launch_bounds__(WTHREADS, 1)
     bool aborted = false;
     long long pc_grp = 0, pc_sfree = 0, pc_issue = 0, pc_pub = 0;  // cycles (T.prof)
     const long long p_start = T.prof ? clock64() : 0;
-    const uint64_t map_ah = reinterpret_cast<uint64_t>(&M.ah), map_al = reinterpret_cast<uint64_t>(&M.al);
+    uint32_t mine[WNS] = {};  // per stage: the step of this thread's last copies into it, + 1
+    bool prev_run = false;    // the group before was the TMA warp's
     // thread 0 waits on b (bounded), all producers learn the outcome; once
-    // the CTA aborts every such wait fails (thread 0 may have given up alone
-    // while issuing a contiguous group's stages)
+    // the CTA aborts every such wait fails
     auto shared_wait = [&](unsigned long long* b, uint32_t parity) -> bool {
       const uint32_t sl = pf++ & 1;
       if (tid == 0) S.pflag[sl] = (!*abort_flag && wait_or_abort(b, parity, abort_flag, T.wait_limit)) ? 1u : 0u;
@@ -516,11 +550,25 @@ __global__ void __launch_bounds__(WTHREADS, 1)
           Gm.hhi = hhi;
           Gm.hq0 = hq0;
           Gm.tag = P.ring ? P.tag_base_tc + (uint32_t)S.unit : 0u;
+          Gm.run = b_tma ? 1u : 0u;
+          Gm.qf = qf;
           n_tiles += (unsigned long long)ng * ((ncols + 127) / 128);
           n_cells += (unsigned long long)nrows * ncols;
         }
         mbar_arrive(&S.gready[gs]);  // releases this thread's writes of the group slot
+        const bool was_run = prev_run;
+        prev_run = b_tma;
         if (T.prof) pc_grp += clock64() - cg0;
+        if (b_tma) {  // the TMA warp issues this group's stages
+          step += nkc;
+          w_pos += ncols;
+          ++group;
+          continue;
+        }
+        if (was_run && !shared_wait(&S.tpass[(group - 1) % WGS], ((group - 1) / WGS) & 1)) {
+          aborted = true;
+          break;
+        }
         // ---- the group's K chunks, one stage each: the home rows as 128-row
         // TMA tiles (thread 0, against one expect_tx on afull), the candidate
         // rows by cp.async, lane l of warp w moving rows 32w + 8i + l / 4
@@ -540,58 +588,7 @@ __global__ void __launch_bounds__(WTHREADS, 1)
             b_src[i] = XS + ((size_t)qi * T.kd + 0) * ESZ + 16u * pch;
           if (prow0 + RSTEP * i < ncols) b_ok |= 1u << i;
         }
-        const uint32_t nbt = b_tma ? (ncols + WM - 1) / WM : 0u;  // candidate tiles by TMA
-        const uint32_t abytes = (ng + nbt) * 2u * A_CHUNK;  // 16 KB a 128-row tile at every precision
-        if (b_tma) {
-          // every copy of the group's stages is a TMA tile: thread 0 alone
-          // waits for each stage, issues its tiles and makes all WNPROD
-          // arrivals on its full barrier; the other producers go on to the
-          // next group (whose slot barrier thread 0 joins when done).  A
-          // failed wait leaves the CTA's abort flag set, which fails the next
-          // shared wait of every producer.
-          if (tid == 0) {
-            for (uint32_t kc = 0; kc < nkc; ++kc) {
-              const uint32_t s = step % WNS;
-              const long long cs0 = T.prof ? clock64() : 0;
-              if (!wait_or_abort(&S.sfree[s], ((step / WNS) & 1) ^ 1, abort_flag, T.wait_limit)) break;
-              const long long cs1 = T.prof ? clock64() : 0;
-              const uint32_t sb = stage_base + s * STAGE_BYTES;
-              const uint32_t ab = smem_u32(&S.afull[s]);
-              mbar_expect_tx(ab, abytes);
-              for (uint32_t g = 0; g < ng; ++g) {
-                if (PREC == 0) {
-                  tma_tile_2d(sb + g * A_CHUNK, map_ah, (int)(kc * WKC), (int)(a0 + g * WM), ab);
-                  tma_tile_2d(sb + A_LO + g * A_CHUNK, map_al, (int)(kc * WKC), (int)(a0 + g * WM), ab);
-                } else {
-                  tma_tile_2d(sb + g * S_ACHUNK, map_ah, (int)(kc * KST), (int)(a0 + g * WM), ab);
-                }
-              }
-              // the candidate rows [qf, qf + 128 nbt): rows past ncols are
-              // fetched (or zero-filled past the last row) and never read
-              for (uint32_t b = 0; b < nbt; ++b) {
-                const int y = (int)(qf + b * WM);
-                if (PREC == 0) {
-                  tma_tile_2d(sb + B_HI + b * A_CHUNK, map_ah, (int)(kc * WKC), y, ab);
-                  tma_tile_2d(sb + B_LO + b * A_CHUNK, map_al, (int)(kc * WKC), y, ab);
-                } else {
-                  tma_tile_2d(sb + S_B + b * S_ACHUNK, map_ah, (int)(kc * KST), y, ab);
-                }
-              }
-              mbar_arrive_n(&S.full[s], WNPROD);
-              ++step;
-              if (T.prof) {
-                const long long cs2 = clock64();
-                pc_sfree += cs1 - cs0;
-                pc_issue += cs2 - cs1;
-              }
-            }
-          } else {
-            step += nkc;
-          }
-          w_pos += ncols;
-          ++group;
-          continue;
-        }
+        const uint32_t abytes = ng * 2u * A_CHUNK;  // 16 KB a 128-row tile at every precision
         for (uint32_t kc = 0; kc < nkc; ++kc) {
           const uint32_t s = step % WNS;
           const long long cs0 = T.prof ? clock64() : 0;
@@ -604,14 +601,8 @@ __global__ void __launch_bounds__(WTHREADS, 1)
           if (tid == 0) {
             const uint32_t ab = smem_u32(&S.afull[s]);
             mbar_expect_tx(ab, abytes);
-            for (uint32_t g = 0; g < ng; ++g) {
-              if (PREC == 0) {
-                tma_tile_2d(sb + g * A_CHUNK, map_ah, (int)(kc * WKC), (int)(a0 + g * WM), ab);
-                tma_tile_2d(sb + A_LO + g * A_CHUNK, map_al, (int)(kc * WKC), (int)(a0 + g * WM), ab);
-              } else {
-                tma_tile_2d(sb + g * S_ACHUNK, map_ah, (int)(kc * KST), (int)(a0 + g * WM), ab);
-              }
-            }
+            home_tiles(sb, kc, a0, ng, ab);
+            mine[s] = step + 1;
           }
           if (PREC == 0) {
             const uint32_t bdst = sb + (ph ? B_LO : B_HI);
@@ -656,7 +647,8 @@ __global__ void __launch_bounds__(WTHREADS, 1)
     if (!aborted) {
       // stop marker: a group slot flagged END behind a stage with no copies
       const uint32_t gs = group % WGS, s = step % WNS;
-      bool ok = shared_wait(&S.gfree[gs], ((group / WGS) & 1) ^ 1);
+      bool ok = !prev_run || shared_wait(&S.tpass[(group - 1) % WGS], ((group - 1) / WGS) & 1);
+      if (ok) ok = shared_wait(&S.gfree[gs], ((group / WGS) & 1) ^ 1);
       if (ok) ok = shared_wait(&S.sfree[s], ((step / WNS) & 1) ^ 1);
       if (ok) {
         if (tid == 0) S.grp[gs].flags = WFLAG_END;
@@ -666,13 +658,7 @@ __global__ void __launch_bounds__(WTHREADS, 1)
       }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
-    // an aborting CTA may still have TMA copies in flight into its stages:
-    // wait (bounded) until each stage's last issued home tiles have landed
-    if (tid == 0 && *abort_flag) {
-      volatile uint32_t no_abort = 0;
-      for (uint32_t j = step > WNS ? step - WNS : 0; j < step; ++j)
-        wait_or_abort(&S.afull[j % WNS], (j / WNS) & 1, &no_abort, T.wait_limit);
-    }
+    if (tid == 0) drain(mine);
     if (tid == 0 && n_tiles) {
       atomicAdd(&T.ctr->tiles, n_tiles);
       atomicAdd(&T.ctr->cells, n_cells);
@@ -758,10 +744,8 @@ __global__ void __launch_bounds__(WTHREADS, 1)
         // Accumulator 1 may still be drained by the epilogue when the group
         // starts; rather than wait, chunk 0 runs ahead through the stages
         // already full, and chunk 1 catches up on them (their release is
-        // held back) once accumulator 1 is free.  nd stages are deferred,
-        // from global step d0; all stages deferred means the ring is full,
-        // and then the lane waits.
-        // Chunk 0 leads chunk 1: by up to the whole ring while the epilogue still
+        // held back) once accumulator 1 is free; with every stage held the
+        // lane waits.  Chunk 0 leads chunk 1: by up to the whole ring while the epilogue still
         // drains accumulator 1, by `lag` stages afterwards, and accumulator 0
         // is handed over as soon as its own last MMA is issued, so that it is
         // drained while chunk 1 finishes.  (Both handed over together, the
@@ -844,6 +828,69 @@ __global__ void __launch_bounds__(WTHREADS, 1)
       if (*abort_flag && last_bar) {
         volatile uint32_t no_abort = 0;
         wait_or_abort(last_bar, last_par, &no_abort, T.wait_limit);
+      }
+    }
+    __syncwarp();
+  } else if (warp == WTMA) {
+    // ============================ TMA issuer
+    // Walks the groups in order, counting every group's stages; those of
+    // contiguous groups are its own: wait for the stage, expect all its bytes,
+    // issue its tiles, and make all the producers' arrivals on full.
+    if (lane == 0) {
+      uint32_t step = 0, group = 0;
+      uint32_t mine[WNS] = {};
+      long long pc_sfree = 0, pc_issue = 0;
+      bool ok = true;
+      while (ok) {
+        const uint32_t gs = group % WGS;
+        if (!wait_or_abort(&S.gready[gs], (group / WGS) & 1, abort_flag, T.wait_limit)) break;
+        const WGroup& Gm = S.grp[gs];
+        if (Gm.flags & WFLAG_END) break;
+        ++group;
+        if (!Gm.run) {
+          step += nkc;
+          mbar_arrive(&S.tpass[gs]);
+          mbar_arrive(&S.gfree[gs]);
+          continue;
+        }
+        const uint32_t a0 = Gm.a0, ng = Gm.ng, qf = Gm.qf, nbt = (Gm.ncols + WM - 1) / WM;
+        const uint32_t bytes = (ng + nbt) * 2u * A_CHUNK;  // 16 KB a 128-row tile at every precision
+        for (uint32_t kc = 0; kc < nkc; ++kc, ++step) {
+          const uint32_t s = step % WNS;
+          const long long cs0 = T.prof ? clock64() : 0;
+          ok = wait_or_abort(&S.sfree[s], ((step / WNS) & 1) ^ 1, abort_flag, T.wait_limit);
+          if (!ok) break;
+          const long long cs1 = T.prof ? clock64() : 0;
+          const uint32_t sb = stage_base + s * STAGE_BYTES;
+          const uint32_t ab = smem_u32(&S.afull[s]);
+          mbar_expect_tx(ab, bytes);
+          home_tiles(sb, kc, a0, ng, ab);
+          // the candidate rows [qf, qf + 128 nbt): rows past ncols are
+          // fetched (or zero-filled past the last row) and never read
+          for (uint32_t b = 0; b < nbt; ++b) {
+            const int y = (int)(qf + b * WM);
+            if (PREC == 0) {
+              tma_tile_2d(sb + B_HI + b * A_CHUNK, map_ah, (int)(kc * WKC), y, ab);
+              tma_tile_2d(sb + B_LO + b * A_CHUNK, map_al, (int)(kc * WKC), y, ab);
+            } else {
+              tma_tile_2d(sb + S_B + b * S_ACHUNK, map_ah, (int)(kc * KST), y, ab);
+            }
+          }
+          mbar_arrive_n(&S.full[s], WNPROD);
+          mine[s] = step + 1;
+          if (T.prof) {
+            pc_sfree += cs1 - cs0;
+            pc_issue += clock64() - cs1;
+          }
+        }
+        if (!ok) break;
+        mbar_arrive(&S.tpass[gs]);
+        mbar_arrive(&S.gfree[gs]);
+      }
+      drain(mine);
+      if (T.prof) {
+        atomicAdd(&T.ctr->prof[0], (unsigned long long)pc_sfree);
+        atomicAdd(&T.ctr->prof[9], (unsigned long long)pc_issue);
       }
     }
     __syncwarp();
