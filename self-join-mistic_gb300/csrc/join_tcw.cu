@@ -77,8 +77,9 @@ constexpr int WNPROD = WNPW * 32;
 constexpr int WNEPI = 16;    // epilogue warps: 4 TMEM lane quarters x 4 column groups
 constexpr int WEPI0 = WNPW;  // first epilogue warp (a multiple of 4: warp % 4 is its lane quarter)
 constexpr int WMMA = WEPI0 + WNEPI;
-constexpr int WTMA = WMMA + 1;  // issues the stages of contiguous groups
-constexpr int WTHREADS = (WTMA + 1) * 32;
+constexpr int WTMA = WMMA + 1;  // first of the warps that issue the stages of contiguous groups
+constexpr int WNT = 2;          // one issues the home rows' tiles, one the candidates'
+constexpr int WTHREADS = (WTMA + WNT) * 32;
 constexpr int WGS = 2;       // group metadata slots
 // stage layout (bytes): home hi | home lo (by TMA) | candidates hi |
 // candidates lo (by cp.async), all as 64-byte rows in the 64B swizzle
@@ -112,7 +113,7 @@ struct __align__(16) WGroup {
   uint32_t a0, nrows, ncols, ng, flags;
   uint32_t hlo, hhi, hq0;  // columns [hlo, hhi) are home-bin rows, column hlo at sorted position hq0
   uint32_t tag;            // the pair ring's tag of the group's unit (0 outside ring mode)
-  uint32_t run, qf;        // run: the candidates are the sorted rows qf, qf + 1, ...; the TMA warp fetches them
+  uint32_t run, qf;        // run: the candidates are the sorted rows qf, qf + 1, ...; the TMA warps fetch them
 };
 
 struct WShared {
@@ -276,17 +277,18 @@ __global__ void k_tf32_rows(const float* __restrict__ xf, uint32_t dpad32, uint3
 
 // ---------------------------------------------------------------- pipeline
 // One persistent CTA per SM: 8 producer warps, 16 epilogue warps, 1 MMA warp,
-// 1 TMA warp.
+// 2 TMA warps.
 //   producers  fetch units; per group of up to 256 candidates all 8 warps
 //              compute the columns' sorted positions, ids, norms and
 //              thresholds; for scattered candidates, per K chunk, thread 0
 //              issues the home rows' TMA tiles against one expect_tx on afull
 //              and every producer thread copies its candidate rows by cp.async;
-//   TMA warp   one lane issues every stage of the groups whose candidates are
-//              one contiguous run (up to 8 TMA tiles a stage) while the
-//              producers prepare the next group: with producer thread 0 doing
-//              both, issuing took 37 % of its time at 515,345 x 90 and the MMA
-//              lane waited for stages 25 % of its own;
+//   TMA warps  one lane of each issues every stage of the groups whose
+//              candidates are one contiguous run, one the home rows' tiles, one
+//              the candidates' (up to 4 TMA tiles a stage each, about 140
+//              cycles a tile), while the producers prepare the next group.
+//              515,345 x 90 join: producer thread 0 doing all of it 64.4 ms,
+//              one TMA warp 61.0, two 60.3;
 //   MMA warp   one lane issues 2 x 3 tcgen05.mma (K 16, M 128, N up to 256)
 //              per home chunk and stage, commits each stage to sfree and, at
 //              a group's last stage, each accumulator to dfull;
@@ -295,9 +297,9 @@ __global__ void k_tf32_rows(const float* __restrict__ xf, uint32_t dpad32, uint3
 //              to the pair list, the error band to the band list.
 // Barriers (all waits bounded by a %globaltimer deadline):
 //   full[s]   producers -> MMA       (WNPROD cp.async arrivals: candidate rows landed; or the TMA lane at once)
-//   afull[s]  producer 0 or TMA -> MMA  (one arrive.expect_tx + the bytes of the stage's TMA tiles)
+//   afull[s]  producer 0 or TMA -> MMA  (WNT arrivals, with expect_tx for the bytes of the stage's TMA tiles)
 //   gready[x] producers -> MMA, TMA  (WNPROD arrivals: group slot x written)
-//   tpass[x]  TMA -> producers       (1 arrival: every stage up to group slot x's is issued)
+//   tpass[x]  TMA -> producers       (WNT arrivals: every stage up to group slot x's is issued)
 // A wait on sfree[s] tells only whether the stage's last use but one is over
 // (phases alternate), so whoever fills the stages of a group waits until the
 // groups before it are issued: the producers through tpass, the TMA lane
@@ -305,7 +307,7 @@ __global__ void k_tf32_rows(const float* __restrict__ xf, uint32_t dpad32, uint3
 //   sfree[s]  MMA -> producers       (tcgen05.commit: stage s read)
 //   dfull[g]  MMA -> epilogue        (tcgen05.commit, or a plain arrive to stop)
 //   dfree[g]  epilogue -> MMA        (WNEPI arrivals; accumulator g reusable)
-//   gfree[x]  epilogue, TMA -> producers  (WNEPI + 1 arrivals; group slot x reusable)
+//   gfree[x]  epilogue, TMA -> producers  (WNEPI + WNT arrivals; group slot x reusable)
 template <int PREC>
 __global__ void __launch_bounds__(WTHREADS, 1)
     k_join_tcw(const JoinParams P, const TcParams T, const __grid_constant__ TcwMaps M) {
@@ -325,7 +327,7 @@ __global__ void __launch_bounds__(WTHREADS, 1)
   if (tid == 0) {
     for (int i = 0; i < WNS; ++i) {
       mbar_init(&S.full[i], WNPROD);
-      mbar_init(&S.afull[i], 1);
+      mbar_init(&S.afull[i], WNT);
       mbar_init(&S.sfree[i], 1);
     }
     for (int i = 0; i < WG; ++i) {
@@ -333,9 +335,9 @@ __global__ void __launch_bounds__(WTHREADS, 1)
       mbar_init(&S.dfree[i], WNEPI);
     }
     for (int i = 0; i < WGS; ++i) {
-      mbar_init(&S.gfree[i], WNEPI + 1);
+      mbar_init(&S.gfree[i], WNEPI + WNT);
       mbar_init(&S.gready[i], WNPROD);
-      mbar_init(&S.tpass[i], 1);
+      mbar_init(&S.tpass[i], WNT);
     }
     asm volatile("fence.mbarrier_init.release.cluster;");
     S.abort_flag = 0;
@@ -386,7 +388,7 @@ __global__ void __launch_bounds__(WTHREADS, 1)
     long long pc_grp = 0, pc_sfree = 0, pc_issue = 0, pc_pub = 0;  // cycles (T.prof)
     const long long p_start = T.prof ? clock64() : 0;
     uint32_t mine[WNS] = {};  // per stage: the step of this thread's last copies into it, + 1
-    bool prev_run = false;    // the group before was the TMA warp's
+    bool prev_run = false;    // the group before was the TMA warps'
     // thread 0 waits on b (bounded), all producers learn the outcome; once
     // the CTA aborts every such wait fails
     auto shared_wait = [&](unsigned long long* b, uint32_t parity) -> bool {
@@ -559,7 +561,7 @@ __global__ void __launch_bounds__(WTHREADS, 1)
         const bool was_run = prev_run;
         prev_run = b_tma;
         if (T.prof) pc_grp += clock64() - cg0;
-        if (b_tma) {  // the TMA warp issues this group's stages
+        if (b_tma) {  // the TMA warps issue this group's stages
           step += nkc;
           w_pos += ncols;
           ++group;
@@ -601,6 +603,7 @@ __global__ void __launch_bounds__(WTHREADS, 1)
           if (tid == 0) {
             const uint32_t ab = smem_u32(&S.afull[s]);
             mbar_expect_tx(ab, abytes);
+            mbar_arrive_n(&S.afull[s], WNT - 1);
             home_tiles(sb, kc, a0, ng, ab);
             mine[s] = step + 1;
           }
@@ -654,7 +657,7 @@ __global__ void __launch_bounds__(WTHREADS, 1)
         if (tid == 0) S.grp[gs].flags = WFLAG_END;
         mbar_arrive(&S.gready[gs]);
         mbar_arrive(&S.full[s]);
-        if (tid == 0) mbar_arrive(&S.afull[s]);
+        if (tid == 0) mbar_arrive_n(&S.afull[s], WNT);
       }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
@@ -831,12 +834,14 @@ __global__ void __launch_bounds__(WTHREADS, 1)
       }
     }
     __syncwarp();
-  } else if (warp == WTMA) {
-    // ============================ TMA issuer
-    // Walks the groups in order, counting every group's stages; those of
-    // contiguous groups are its own: wait for the stage, expect all its bytes,
-    // issue its tiles, and make all the producers' arrivals on full.
+  } else if (warp >= WTMA) {
+    // ============================ TMA issuers
+    // Walk the groups in order, counting every group's stages; those of
+    // contiguous groups are theirs: wait for the stage, expect the bytes of
+    // one's own tiles and issue them; the first lane also makes all the
+    // producers' arrivals on full.
     if (lane == 0) {
+      const bool home = warp == WTMA;
       uint32_t step = 0, group = 0;
       uint32_t mine[WNS] = {};
       long long pc_sfree = 0, pc_issue = 0;
@@ -854,7 +859,7 @@ __global__ void __launch_bounds__(WTHREADS, 1)
           continue;
         }
         const uint32_t a0 = Gm.a0, ng = Gm.ng, qf = Gm.qf, nbt = (Gm.ncols + WM - 1) / WM;
-        const uint32_t bytes = (ng + nbt) * 2u * A_CHUNK;  // 16 KB a 128-row tile at every precision
+        const uint32_t bytes = (home ? ng : nbt) * 2u * A_CHUNK;  // 16 KB a 128-row tile at every precision
         for (uint32_t kc = 0; kc < nkc; ++kc, ++step) {
           const uint32_t s = step % WNS;
           const long long cs0 = T.prof ? clock64() : 0;
@@ -864,10 +869,13 @@ __global__ void __launch_bounds__(WTHREADS, 1)
           const uint32_t sb = stage_base + s * STAGE_BYTES;
           const uint32_t ab = smem_u32(&S.afull[s]);
           mbar_expect_tx(ab, bytes);
-          home_tiles(sb, kc, a0, ng, ab);
+          if (home) {
+            home_tiles(sb, kc, a0, ng, ab);
+            mbar_arrive_n(&S.full[s], WNPROD);
+          }
           // the candidate rows [qf, qf + 128 nbt): rows past ncols are
           // fetched (or zero-filled past the last row) and never read
-          for (uint32_t b = 0; b < nbt; ++b) {
+          for (uint32_t b = 0; b < nbt && !home; ++b) {
             const int y = (int)(qf + b * WM);
             if (PREC == 0) {
               tma_tile_2d(sb + B_HI + b * A_CHUNK, map_ah, (int)(kc * WKC), y, ab);
@@ -876,7 +884,6 @@ __global__ void __launch_bounds__(WTHREADS, 1)
               tma_tile_2d(sb + S_B + b * S_ACHUNK, map_ah, (int)(kc * KST), y, ab);
             }
           }
-          mbar_arrive_n(&S.full[s], WNPROD);
           mine[s] = step + 1;
           if (T.prof) {
             pc_sfree += cs1 - cs0;
@@ -888,7 +895,7 @@ __global__ void __launch_bounds__(WTHREADS, 1)
         mbar_arrive(&S.gfree[gs]);
       }
       drain(mine);
-      if (T.prof) {
+      if (T.prof && home) {
         atomicAdd(&T.ctr->prof[0], (unsigned long long)pc_sfree);
         atomicAdd(&T.ctr->prof[9], (unsigned long long)pc_issue);
       }
