@@ -196,6 +196,8 @@ struct JoinParams {
   unsigned long long band0, band1;   // band decisions of band_list[band0 .. band1) (pair ring)
   uint32_t grid_cap;                 // pair ring: at most this many blocks (0: the persistent grid)
   unsigned long long claim_cap;      // pair ring: claim indices from this one on take no unit (0: no cap)
+  unsigned long long unit_work;      // CUDA-core units: average candidate points (0: unknown)
+  uint32_t claim_mask;               // CUDA-core units a claim, less one (set at the launch)
   // FP32 pre-decision of band pairs (null inv: every band pair goes to FP64):
   // rows xf32[inv[id]] (sorted FP32 rows, stride dpad32) filtered with the
   // FP32 filter's thresholds t_lo / t_hi before the FP64 predicate

@@ -1021,7 +1021,7 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
     }
   }
   uint32_t tots[3] = {0, 0, 0};
-  unsigned long long totc = 0;
+  unsigned long long totc = 0, simt_work = 0;
   uint32_t* nbr = nullptr;
   Unit* units = nullptr;
   Unit* units_tc = nullptr;
@@ -1038,6 +1038,7 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
     idx::EnumTotals ht{};
     d2h(h, &ht, tot_dev, sizeof ht);
     totc = ht.cand;
+    simt_work = ht.work[0];
     // MISTIC_TEST_WORKLIST_LIMIT=k lowers the limit (tests of this check)
     unsigned long long lim = 0xffffffffull - 1;
     if (const char* ev = getenv("MISTIC_TEST_WORKLIST_LIMIT")) lim = std::min(lim, strtoull(ev, nullptr, 10));
@@ -1122,6 +1123,7 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
   auto point_lists = [&]() {
     jp.units = units;
     jp.n_units = tots[1];
+    jp.unit_work = simt_work / std::max<uint32_t>(tots[1], 1u);
     jp.nbr = nbr;
     tp.units = units_tc;
     tp.n_units = tots[2];

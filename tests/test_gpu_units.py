@@ -51,3 +51,18 @@ def test_enumerations_find_every_pair(handle, n, d, k, eps):
     assert np.array_equal(r.pairs, ref), diff_pairs(r.pairs, ref)
     s = handle.selfjoin(x, k, eps, mode="fp64", csr="host", home_sample=0)
     assert s.pairs_ij == len(ref) and s.candidates == r.candidates
+
+
+@pytest.mark.parametrize("mode", ["fp32", "fp64"])
+@pytest.mark.parametrize("rows,cols", [(560, 561), (640, 641), (1001, 999)])
+def test_many_small_units(handle, mode, rows, cols):
+    """Unit lattices whose bins hold a point or two: unit counts on both sides
+    of where a warp begins to claim several units at a time.  At ε = 1.1 the
+    pairs are the lattice's edges."""
+    ids = np.arange(rows * cols, dtype=np.uint32).reshape(rows, cols)
+    x = np.stack(np.divmod(ids.ravel(), cols), axis=1).astype(np.float64)
+    edges = [(ids[:, :-1], ids[:, 1:]), (ids[:-1], ids[1:])]
+    ref = np.concatenate([np.stack([a.ravel(), b.ravel()], axis=1) for a, b in edges])
+    ref = ref[np.lexsort((ref[:, 1], ref[:, 0]))]
+    r = handle.selfjoin(x, 2, 1.1, mode=mode, pairs="host", sort_pairs=True)
+    assert np.array_equal(r.pairs, ref)
