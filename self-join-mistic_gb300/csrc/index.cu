@@ -422,7 +422,7 @@ __global__ void k_max_final(const double* __restrict__ part, uint32_t nparts, do
 }
 
 // ------------------------------------------------------------ neighbour enumeration
-// One thread per non-empty bin h.  Depth-first over the key fields: at
+// Up to 8 threads per non-empty bin h.  Depth-first over the key fields: at
 // level j the candidate field value is K_j - 1, K_j, K_j + 1; the bins whose
 // key starts with the chosen prefix form a contiguous sorted range, found by
 // two lower-bound searches inside the parent range.  The first p fields
@@ -517,34 +517,60 @@ __device__ __noinline__ void walk_deep(const uint64_t* __restrict__ bkey, uint64
   }
 }
 
+// Ranges of at most this many bins are read through instead of walked: the
+// reads do not depend on one another, a search's do.
+constexpr uint32_t ENUM_SCAN = 32;
+
+// leaf(a) for the bins a >= hb of [lo, hi) whose fields j .. k-1 are within
+// one of the home key's.
+template <class Leaf>
+__device__ __forceinline__ void scan_range(const uint64_t* __restrict__ bkey, uint64_t K, uint32_t hb,
+                                           const EnumParams& P, int j, uint32_t lo, uint32_t hi, Leaf& leaf) {
+#pragma unroll 1
+  for (uint32_t a = max(lo, hb); a < hi; ++a) {
+    bool ok = true;
+    if (j < P.k) {
+      const uint64_t Ka = bkey[a];
+      for (int q = j; q < P.k; ++q) {
+        const int df = key_field(Ka, P, q) - key_field(K, P, q);
+        ok = ok && df >= -1 && df <= 1;
+      }
+    }
+    if (ok) leaf(a);
+  }
+}
+
 // Depth-first walk of key fields j .. k-1 of home key K inside the sorted bin
-// range [lo, hi) whose keys share the prefix bits `base`: field values
-// K_j - 1, K_j, K_j + 1 in order, each narrowed by two lower-bound searches;
-// leaf(a) for every bin a >= hb, in ascending order.  The first R levels
-// keep their range and loop state in registers; deeper ones go to walk_deep.
+// range [lo, hi) whose keys share the prefix bits `base`: the range of field
+// values K_j - 1 .. K_j + 1, read through when it is short, else cut into its
+// three values; leaf(a) for every bin a >= hb, in ascending order.  The first
+// R levels keep their range and loop state in registers; deeper ones go to
+// walk_deep.
 template <int R, class Leaf>
 __device__ __forceinline__ void walk_levels(const uint64_t* __restrict__ bkey, uint64_t K, uint32_t hb,
                                             const EnumParams& P, int j, uint32_t lo, uint32_t hi, uint64_t base,
                                             Leaf& leaf) {
   const int sh = P.shift[j];
   const int kfj = key_field(K, P, j);
+  const int c0 = max(kfj - 1, 0), c1 = (int)min((long long)kfj + 1, (long long)P.maxkey[j]);
+  uint32_t a = lower_bound_u64(bkey, lo, hi, base | ((uint64_t)c0 << sh));
+  const uint32_t end = lower_bound_u64(bkey, a, hi, (base | ((uint64_t)c1 << sh)) + (1ull << sh));
+  if (end <= hb) return;
+  if (j == P.k - 1 || end - a <= ENUM_SCAN) {
+    scan_range(bkey, K, hb, P, j + 1, a, end, leaf);
+    return;
+  }
 #pragma unroll 1
-  for (int di = 0; di < 3; ++di) {
-    const int cv = kfj + di - 1;
-    if (cv < 0 || (long long)cv > (long long)P.maxkey[j]) continue;
+  for (int cv = c0; cv <= c1; ++cv) {
     const uint64_t lower = base | ((uint64_t)cv << sh);
-    const uint64_t upper = lower + (1ull << sh);
-    const uint32_t a = lower_bound_u64(bkey, lo, hi, lower);
-    const uint32_t b = lower_bound_u64(bkey, a, hi, upper);
-    if (a == b || b <= hb) continue;
-    if (j == P.k - 1) {
-      leaf(a);  // b == a + 1 and a >= hb
-      continue;
+    const uint32_t b = cv == c1 ? end : lower_bound_u64(bkey, a, end, lower + (1ull << sh));
+    if (a < b && b > hb) {
+      if constexpr (R > 1)
+        walk_levels<R - 1>(bkey, K, hb, P, j + 1, a, b, lower, leaf);
+      else
+        walk_deep(bkey, K, hb, P, j + 1, a, b, lower, leaf);
     }
-    if constexpr (R > 1)
-      walk_levels<R - 1>(bkey, K, hb, P, j + 1, a, b, lower, leaf);
-    else
-      walk_deep(bkey, K, hb, P, j + 1, a, b, lower, leaf);
+    a = b;
   }
 }
 
@@ -593,7 +619,7 @@ __device__ __forceinline__ uint32_t seg_chunks(const HomeSplit& s, uint32_t seg,
   return (uint32_t)min((unsigned long long)s.nch, (b + 1ull) * (seg / s.csz));
 }
 
-// Units of all nseg segments of a home bin.
+// Units of the first nseg segments of a home bin.
 __device__ __forceinline__ unsigned long long count_units(const EnumParams& P, const HomeSplit& s, uint32_t hb,
                                                           uint32_t seg, uint32_t nseg) {
   const uint32_t r = seg / s.csz;
@@ -604,7 +630,7 @@ __device__ __forceinline__ unsigned long long count_units(const EnumParams& P, c
   }
   unsigned long long u = 0;
   for (uint32_t c = 0; c < s.nch; ++c)
-    if (group_sampled(hb, c * s.csz / SAMPLE_GROUP, P.sample)) u += nseg - c / r;
+    if (c / r < nseg && group_sampled(hb, c * s.csz / SAMPLE_GROUP, P.sample)) u += nseg - c / r;
   return u;
 }
 
@@ -662,28 +688,44 @@ __device__ __forceinline__ void add_work(idx::EnumTotals* tot, unsigned long lon
   }
 }
 
+// P.lanes threads (a power of two within a warp) share a home bin when the
+// prefix table is used: each takes a run of the prefixes.  Pass 1 leaves each
+// one's first neighbour and first candidate rank within the bin in lane_off.
 template <bool FILL>
 __global__ void __launch_bounds__(128, 8) k_enum(const uint64_t* __restrict__ bkey, const uint32_t* __restrict__ bstart,
                        uint32_t m, EnumParams P, uint32_t* __restrict__ npts, uint32_t* __restrict__ nbr_cnt,
-                       idx::EnumTotals* __restrict__ tot, const uint32_t* __restrict__ nbr_off,
-                       const uint32_t* __restrict__ unit_off, const uint32_t* __restrict__ unit_off_tc,
-                       uint32_t* __restrict__ nbr, Unit* __restrict__ units_simt, Unit* __restrict__ units_tc) {
-  const uint32_t hb = blockIdx.x * blockDim.x + threadIdx.x;
+                       uint2* __restrict__ lane_off, idx::EnumTotals* __restrict__ tot,
+                       const uint32_t* __restrict__ nbr_off, const uint32_t* __restrict__ unit_off,
+                       const uint32_t* __restrict__ unit_off_tc, uint32_t* __restrict__ nbr,
+                       Unit* __restrict__ units_simt, Unit* __restrict__ units_tc) {
+  const unsigned long long gt = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t hb = (uint32_t)min((unsigned long long)m, gt / P.lanes), part = (uint32_t)gt & (P.lanes - 1);
   unsigned long long work = 0;
+  uint32_t cnt = 0, pts = 0;
   bool tc = false;
   if (hb < m) {
     const uint64_t K = bkey[hb];
     const uint32_t asz = bstart[hb + 1] - bstart[hb];
     const HomeSplit hsp = home_split(P, hb, asz);
     tc = hsp.tc;
-    uint32_t cnt = 0, pts = 0;
     const uint32_t n0 = FILL ? nbr_off[hb] : 0u;
     const uint32_t seg = FILL ? tot->seg[tc ? 1 : 0] : 0u;
     const uint32_t total = FILL ? npts[hb] : 0u;
     const uint32_t nseg = FILL ? (uint32_t)(((unsigned long long)total + seg - 1) / seg) : 0u;
     UnitWriter<false> uw{FILL ? (tc ? units_tc + unit_off_tc[hb] : units_simt + unit_off[hb]) : nullptr, hb, seg, nseg, 0};
     unsigned long long cut = seg;  // candidate rank of the next segment boundary
-    if (FILL) uw.begin(P, hsp, n0);
+    if (FILL) {
+      if (part == 0) {
+        uw.begin(P, hsp, n0);
+      } else {
+        const uint2 lo = lane_off[gt];
+        cnt = lo.x;
+        pts = lo.y;
+        uw.b = pts / seg;  // boundaries up to here belong to the threads before
+        uw.units += count_units(P, hsp, hb, seg, uw.b);
+        cut = (uw.b + 1ull) * seg;
+      }
+    }
 
     // Visits neighbour bin `a` (ascending, a >= hb): its points, and in pass
     // 2 the neighbour list and the segment boundaries that fall inside it.
@@ -702,23 +744,31 @@ __global__ void __launch_bounds__(128, 8) k_enum(const uint64_t* __restrict__ bk
     };
 
     if (P.k == 0) {
-      leaf(hb);  // no key fields: one bin holding every point
+      leaf(hb);  // no key fields: one bin holding every point (lanes is 1)
     } else if (P.p == 0) {
-      walk_levels<3>(bkey, K, hb, P, 0, 0u, m, 0ull, leaf);
+      walk_levels<3>(bkey, K, hb, P, 0, 0u, m, 0ull, leaf);  // lanes is 1
     } else {
-      // prefixes in ascending order: field j offset by digit j of c in base 3
-      // (field 0 most significant)
-      uint32_t n3 = 1;
-      for (int q = 0; q < P.p; ++q) n3 *= 3;
-      for (uint32_t cb = 0; cb < n3; ++cb) {
-        uint32_t rem = cb, pw = n3 / 3, idx = 0;
+      // prefixes in ascending order: field q < p - 1 offset by digit q of cb
+      // in base 3 (field 0 most significant).  The values of field p - 1
+      // adjoin in the table, so its three prefixes are one range.  The first
+      // half of the prefixes lies below the home bin's.
+      int n3 = 1;
+      for (int q = 0; q + 1 < P.p; ++q) n3 *= 3;
+      const int last = P.p - 1;
+      const int kl = key_field(K, P, last);
+      const int c0 = max(kl - 1, 0), c1 = (int)min((long long)kl + 1, (long long)P.maxkey[last]);
+      const int mid = n3 / 2, np = n3 - mid;
+      const int cb1 = mid + (int)(np * (part + 1) / P.lanes);
+      for (int cb = mid + (int)(np * part / P.lanes); cb < cb1; ++cb) {
+        int rem = cb, pw = n3 / 3;
+        uint32_t idx = 0;
         uint64_t pre = 0;
         bool ok = true;
-        for (int q = 0; q < P.p; ++q) {
-          const uint32_t t = rem / pw;
+        for (int q = 0; q < last; ++q) {
+          const int t = rem / pw;
           rem -= t * pw;
           pw /= 3;
-          const int cv = key_field(K, P, q) + (int)t - 1;
+          const int cv = key_field(K, P, q) + t - 1;
           if (cv < 0 || (uint32_t)cv > P.maxkey[q]) {
             ok = false;
             break;
@@ -727,22 +777,38 @@ __global__ void __launch_bounds__(128, 8) k_enum(const uint64_t* __restrict__ bk
           pre |= (uint64_t)cv << P.shift[q];
         }
         if (!ok) continue;
-        const uint32_t r0 = P.ptab[idx], r1 = P.ptab[idx + 1];
+        const uint32_t r0 = P.ptab[idx + c0], r1 = P.ptab[idx + c1 + 1];
         if (r0 == r1 || r1 <= hb) continue;
-        if (P.p == P.k) {  // every field fixed: the single bin r0 (>= hb)
-          leaf(r0);
+        if (P.p == P.k || r1 - r0 <= ENUM_SCAN) {
+          scan_range(bkey, K, hb, P, P.p, r0, r1, leaf);
           continue;
         }
-        walk_levels<3>(bkey, K, hb, P, P.p, r0, r1, pre, leaf);
+        for (int cv = c0; cv <= c1; ++cv) {
+          const uint32_t a = P.ptab[idx + cv], b = P.ptab[idx + cv + 1];
+          if (a < b && b > hb) walk_levels<3>(bkey, K, hb, P, P.p, a, b, pre | ((uint64_t)cv << P.shift[last]), leaf);
+        }
       }
     }
-    if (!FILL) {
-      nbr_cnt[hb] = cnt;
-      npts[hb] = pts;
-      work = (unsigned long long)hsp.nch_s * pts;
+    work = (unsigned long long)hsp.nch_s * pts;
+  }
+  if (!FILL) {
+    add_work(tot, work, tc);
+    uint32_t ce = cnt, pe = pts;  // inclusive sums over the bin's threads
+    for (uint32_t o = 1; o < P.lanes; o <<= 1) {
+      const uint32_t c = __shfl_up_sync(FULL_MASK, ce, o, P.lanes), p = __shfl_up_sync(FULL_MASK, pe, o, P.lanes);
+      if (part >= o) {
+        ce += c;
+        pe += p;
+      }
+    }
+    if (hb < m) {
+      if (P.lanes > 1) lane_off[gt] = make_uint2(ce - cnt, pe - pts);
+      if (part == P.lanes - 1) {
+        nbr_cnt[hb] = ce;
+        npts[hb] = pe;
+      }
     }
   }
-  if (!FILL) add_work(tot, work, tc);
 }
 
 // The same enumeration with a warp per home bin: the keys from the bin itself
@@ -989,22 +1055,44 @@ void prefix_table(mistic_handle_s* h, const uint64_t* bkey, uint32_t m, const En
   exclusive_scan<uint32_t>(h, ptab, ptab, (size_t)entries + 1, nullptr);
 }
 
-// A warp per bin reads every key whose field 0 lies near (m^2 work); a thread
-// per bin takes up to 3^k dependent steps whatever m is.  Both passes and the
-// scans, ms, warp / thread per bin: k = 2: 7,131 bins 0.060 / 0.091, 21,565
-// 0.100 / 0.097; k = 3: 87,584 bins 1.20 / 0.19; k = 6: 11,483 bins 0.30 /
-// 0.89, 28,343 1.04 / 0.93, 46,583 2.20 / 1.01; k = 8: 5,593 bins 0.23 / 5.68.
-bool enum_flat(uint32_t m, const EnumParams& P) { return m <= 4096u * (uint32_t)std::min(std::max(P.k, 1), 6); }
+// A warp per bin reads every key whose field 0 lies near (m^2 work); threads
+// that walk take up to 3^k dependent steps whatever m is.  Both passes and the
+// scans, ms, warp / threads per bin: k = 2: 7,131 bins 0.058 / 0.085, 14,921
+// 0.078 / 0.077, 21,555 0.099 / 0.087; k = 3: 8,952 bins 0.081 / 0.080, 17,832
+// 0.152 / 0.112; k = 4: 7,599 bins 0.090 / 0.105, 12,446 0.140 / 0.118; k = 6:
+// 7,824 bins 0.172 / 0.237, 10,061 0.248 / 0.247, 14,894 0.387 / 0.277; k = 8:
+// 9,867 bins 0.340 / 0.627, 16,761 0.708 / 0.815, 26,116 1.376 / 1.200.
+bool enum_flat(uint32_t m, const EnumParams& P) { return m <= (P.k > 6 ? 20480u : 10240u); }
+
+// Threads a bin: up to 8, while the device holds them about at once (152 SMs
+// x 1,024 threads); beyond that the extra searches cost more than the shorter
+// chains give.  ms at 1 / 2 / 4 / 8 threads: k = 6: 28,357 bins 0.725 / 0.514
+// / 0.403 / 0.359, 76,372 0.926 / 0.691 / 0.719 / 0.752, 136,090 1.061 / 1.042
+// / 1.166 / 1.289.  With three levels or more below the table the chains are
+// longer: k = 8: 129,896 bins 8.12 / 6.22 / 5.21 / 5.48, 321,117 12.6 / 10.7 /
+// 11.8 / 13.6.  Fewer than three table fields make too few prefixes to share.
+uint32_t enum_lanes(uint32_t m, const EnumParams& P) {
+  if (P.p < 3) return 1;
+  const unsigned long long most = P.k - P.p >= 3 ? 640u * 1024u : 256u * 1024u;
+  uint32_t l = 8;
+  while (l > 1 && (unsigned long long)m * l > most) l >>= 1;
+  return l;
+}
+
+static unsigned enum_grid(uint32_t m, const EnumParams& P) {
+  return (unsigned)(((unsigned long long)m * P.lanes + 127) / 128);
+}
 
 void enum_count(mistic_handle_s* h, const uint64_t* bkey, const uint32_t* bstart, uint32_t m, const EnumParams& P,
-                uint32_t* npts, uint32_t* nbr_cnt, uint32_t* unit_cnt, uint32_t* unit_cnt_tc, EnumTotals* tot) {
+                uint32_t* npts, uint32_t* nbr_cnt, uint2* lane_off, uint32_t* unit_cnt, uint32_t* unit_cnt_tc,
+                EnumTotals* tot) {
   MCK(cudaMemsetAsync(tot, 0, sizeof(EnumTotals), h->stream));
   if (enum_flat(m, P))
     k_enum_flat<false><<<(m + FLAT_WARPS - 1) / FLAT_WARPS, FLAT_WARPS * 32, 0, h->stream>>>(
         bkey, bstart, m, P, npts, nbr_cnt, tot, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
   else
-    k_enum<false><<<(m + 127) / 128, 128, 0, h->stream>>>(bkey, bstart, m, P, npts, nbr_cnt, tot, nullptr, nullptr,
-                                                          nullptr, nullptr, nullptr, nullptr);
+    k_enum<false><<<enum_grid(m, P), 128, 0, h->stream>>>(bkey, bstart, m, P, npts, nbr_cnt, lane_off, tot, nullptr,
+                                                          nullptr, nullptr, nullptr, nullptr, nullptr);
   launched(h, "enum_count");
   const unsigned nb = std::max(1u, std::min((m + 255) / 256, 4u * (unsigned)h->sms));
   k_unit_plan<<<nb, 256, 0, h->stream>>>(bstart, m, P, npts, nbr_cnt, unit_cnt, unit_cnt_tc, tot);
@@ -1013,16 +1101,16 @@ void enum_count(mistic_handle_s* h, const uint64_t* bkey, const uint32_t* bstart
 }
 
 void enum_fill(mistic_handle_s* h, const uint64_t* bkey, const uint32_t* bstart, uint32_t m, const EnumParams& P,
-               const uint32_t* npts, const uint32_t* nbr_off, const uint32_t* unit_off, const uint32_t* unit_off_tc,
-               const EnumTotals* tot, uint32_t* nbr, Unit* units, Unit* units_tc) {
+               const uint32_t* npts, const uint2* lane_off, const uint32_t* nbr_off, const uint32_t* unit_off,
+               const uint32_t* unit_off_tc, const EnumTotals* tot, uint32_t* nbr, Unit* units, Unit* units_tc) {
   uint32_t* np = const_cast<uint32_t*>(npts);
   EnumTotals* t = const_cast<EnumTotals*>(tot);
   if (enum_flat(m, P))
     k_enum_flat<true><<<(m + FLAT_WARPS - 1) / FLAT_WARPS, FLAT_WARPS * 32, 0, h->stream>>>(
         bkey, bstart, m, P, np, nullptr, t, nbr_off, unit_off, unit_off_tc, nbr, units, units_tc);
   else
-    k_enum<true><<<(m + 127) / 128, 128, 0, h->stream>>>(bkey, bstart, m, P, np, nullptr, t, nbr_off, unit_off,
-                                                         unit_off_tc, nbr, units, units_tc);
+    k_enum<true><<<enum_grid(m, P), 128, 0, h->stream>>>(bkey, bstart, m, P, np, nullptr, const_cast<uint2*>(lane_off),
+                                                         t, nbr_off, unit_off, unit_off_tc, nbr, units, units_tc);
   launched(h, "enum_fill");
 }
 

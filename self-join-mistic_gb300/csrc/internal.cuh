@@ -120,6 +120,7 @@ struct EnumParams {
   int p;
   uint32_t stride[MAX_K];
   const uint32_t* ptab;
+  uint32_t lanes;    // threads per bin of the thread-per-bin enumeration (a power of two up to 32)
 };
 
 // FP32 constants of a tensor-core join's per-column error bound (see
@@ -335,6 +336,8 @@ void prefix_table(mistic_handle_s*, const uint64_t* bkey, uint32_t m, const Enum
 // Whether m bins are enumerated by a warp per bin over the sorted keys (no
 // prefix table) rather than by a thread per bin.
 bool enum_flat(uint32_t m, const EnumParams&);
+// threads a bin the other enumeration takes (after the prefix table is chosen)
+uint32_t enum_lanes(uint32_t m, const EnumParams&);
 // Neighbour enumeration, first half: neighbours and units per home bin, as
 // exclusive prefix sums in nbr_cnt, unit_cnt and unit_cnt_tc, and the totals
 // (see EnumTotals); npts is scratch of m entries.
@@ -345,11 +348,12 @@ struct EnumTotals {
   uint32_t seg[2];              // segment lengths chosen
 };
 void enum_count(mistic_handle_s*, const uint64_t* bkey, const uint32_t* bstart, uint32_t m, const EnumParams&,
-                uint32_t* npts, uint32_t* nbr_cnt, uint32_t* unit_cnt, uint32_t* unit_cnt_tc, EnumTotals* tot);
+                uint32_t* npts, uint32_t* nbr_cnt, uint2* lane_off, uint32_t* unit_cnt, uint32_t* unit_cnt_tc,
+                EnumTotals* tot);
 // Second half: the neighbour list and the units.
 void enum_fill(mistic_handle_s*, const uint64_t* bkey, const uint32_t* bstart, uint32_t m, const EnumParams&,
-               const uint32_t* npts, const uint32_t* nbr_off, const uint32_t* unit_off, const uint32_t* unit_off_tc,
-               const EnumTotals* tot, uint32_t* nbr, Unit* units, Unit* units_tc);
+               const uint32_t* npts, const uint2* lane_off, const uint32_t* nbr_off, const uint32_t* unit_off,
+               const uint32_t* unit_off_tc, const EnumTotals* tot, uint32_t* nbr, Unit* units, Unit* units_tc);
 // points per log2 bin-size class (32 classes) into hist
 void bin_hist(mistic_handle_s*, const uint32_t* bstart, uint32_t m, unsigned long long* hist);
 }  // namespace idx

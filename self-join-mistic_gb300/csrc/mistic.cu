@@ -1020,6 +1020,7 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
       ep.ptab = ptab;
     }
   }
+  ep.lanes = idx::enum_lanes(m, ep);
   uint32_t tots[3] = {0, 0, 0};
   unsigned long long totc = 0, simt_work = 0;
   uint32_t* nbr = nullptr;
@@ -1032,7 +1033,9 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
     uint32_t* unit_cnt = abuf<uint32_t>(h, "unit_cnt", m + 1);
     uint32_t* unit_cnt_tc = abuf<uint32_t>(h, "unit_cnt_tc", m + 1);
     idx::EnumTotals* tot_dev = abuf<idx::EnumTotals>(h, "enum_tot", 1);
-    idx::enum_count(h, bkey, bstart, m, e, npts, nbr_cnt, unit_cnt, unit_cnt_tc, tot_dev);
+    // at most 640 K entries
+    uint2* lane_off = e.lanes > 1 ? abuf<uint2>(h, "enum_lane", (size_t)m * e.lanes) : nullptr;
+    idx::enum_count(h, bkey, bstart, m, e, npts, nbr_cnt, lane_off, unit_cnt, unit_cnt_tc, tot_dev);
     // 64-bit totals first: the work lists index neighbours and units with
     // 32-bit offsets, which a total of 2^32 or more would wrap
     idx::EnumTotals ht{};
@@ -1052,7 +1055,8 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
     nbr = abuf<uint32_t>(h, "nbr", (size_t)tots[0] + 1);
     units = abuf<Unit>(h, "units", (size_t)tots[1] + 1);
     units_tc = abuf<Unit>(h, "units_tc", (size_t)tots[2] + 1);
-    idx::enum_fill(h, bkey, bstart, m, e, npts, nbr_cnt, unit_cnt, unit_cnt_tc, tot_dev, nbr, units, units_tc);
+    idx::enum_fill(h, bkey, bstart, m, e, npts, lane_off, nbr_cnt, unit_cnt, unit_cnt_tc, tot_dev, nbr, units,
+                   units_tc);
   };
 
   // ---- join parameters

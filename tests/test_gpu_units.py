@@ -66,3 +66,25 @@ def test_many_small_units(handle, mode, rows, cols):
     ref = ref[np.lexsort((ref[:, 1], ref[:, 0]))]
     r = handle.selfjoin(x, 2, 1.1, mode=mode, pairs="host", sort_pairs=True)
     assert np.array_equal(r.pairs, ref)
+
+
+@pytest.mark.parametrize("n,d,k,eps", [(12000, 3, 3, 0.012), (24000, 4, 4, 0.04), (40000, 5, 5, 0.05),
+                                       (24000, 8, 8, 0.16), (36000, 6, 4, 0.05)])
+@pytest.mark.parametrize("clusters", [0, 5])
+def test_threads_sharing_a_walk(handle, n, d, k, eps, clusters):
+    """Bins beyond the warp-per-bin line, walked by 8, 4, 2 or one thread
+    each: uniform points, and a third of them in tight groups whose long lists
+    are cut into segments inside a thread's share.  The home samples add up to
+    no more than the whole."""
+    rng = np.random.default_rng(n + d + clusters)
+    x = rng.random((n, d))
+    g = n // 15
+    for c in range(clusters):
+        x[c * g:(c + 1) * g] = rng.random(d) + rng.random((g, d)) * eps
+    ref = O.brute_pairs(x, eps)
+    r = handle.selfjoin(x, k, eps, pairs="host", sort_pairs=True)
+    assert np.array_equal(r.pairs, ref), diff_pairs(r.pairs, ref)
+    s = handle.selfjoin(x, k, eps, pairs="host", sort_pairs=True, home_sample=3)
+    assert s.candidates < r.candidates
+    key = lambda p: p[:, 0].astype(np.uint64) << 32 | p[:, 1]
+    assert np.isin(key(s.pairs), key(ref)).all()
