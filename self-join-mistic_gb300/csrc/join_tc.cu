@@ -55,7 +55,7 @@ constexpr int TN = 128;          // candidate columns per tile (MMA N)
 constexpr int WIN = 256;         // neighbour bins per candidate window
 
 // ---------------------------------------------------------------- pipeline
-// One persistent CTA per SM: 8 producer warps, NEPI epilogue warps, 2 MMA warps.
+// One persistent CTA per SM: 8 producer warps, NEPI epilogue warps, 4 MMA warps.
 //   producers  K <= 32: 4 loader warps claim units, walk their neighbour bins
 //              and copy each tile's 128 candidate rows (raw FP32, cp.async)
 //              into a ring of RAW landing slots; 4 converter warps, a thread
@@ -68,10 +68,11 @@ constexpr int WIN = 256;         // neighbour bins per candidate window
 //              threads a row, the raw rows landing in the B stages
 //              themselves where no separate slots fit;
 //   MMA warps  one lane of each issues 3 * KP/16 tcgen05.mma per (tile, home
-//              chunk) into the next of NACC = 4 TMEM accumulators and commits,
-//              the two warps taking turns: at K = 32 a lane spends about 490
-//              cycles an accumulator issuing its MMAs and half as much again
-//              on waits, metadata and commits;
+//              chunk) into its own of the NACC = 4 TMEM accumulators and
+//              commits, the warps taking turns.  With two warps of two
+//              accumulators each, a warp that waited for one could not refill
+//              the other: 75.3 ms on the 5M x 18 join against 71.9, 1.54
+//              against 1.47 on its 250k;
 //   epilogue   groups of 4 warps, one per TMEM lane quarter, each group with
 //              its own accumulators: tcgen05.ld, sign-bit test (D' < 0 marks
 //              a candidate), home-bin rule by column range, sure accepts to
@@ -95,13 +96,13 @@ constexpr int NUNIT = 8;   // unit slots between them (at most RAW = 4 units hav
 // NEPI epilogue warps (a template parameter: 8 or 16) in groups of 4; the MMA
 // warps follow them.
 constexpr int EPI0 = NPW;  // first epilogue warp (a multiple of 4: warp % 4 is its lane quarter)
-constexpr int NMMA = 2;    // MMA warps
+constexpr int NMMA = 4;    // MMA warps
 __host__ __device__ constexpr int tc_threads(int nepi) { return (EPI0 + nepi + NMMA) * 32; }
 constexpr int NACC = 4;    // TMEM accumulators of 128 columns (512 per CTA, one CTA per SM)
 constexpr uint32_t FLAG_FIRST = 1, FLAG_LAST = 2, FLAG_END = 4;
 
 struct __align__(16) TileMeta {
-  uint32_t a0, na, flags, ng;  // ng: 128-row MMA tiles of this unit (1..G)
+  uint32_t a0, na, flags, ng;  // ng: 128-row MMA tiles of this unit (1..G); the MMA warps read these four as one
   uint32_t inst;               // instance of the unit (fused batch joins; else 0)
   uint32_t ncols;
   uint32_t hcr, hq;  // columns [hcr & 255, hcr >> 8) hold home-bin rows, the first at sorted position hq
@@ -126,7 +127,11 @@ struct __align__(16) TcAcc {
 
 template <int NS, int G, int RAW>
 struct TcShared2 {
-  static constexpr int NM = NS;  // metadata slots
+  // Metadata slots.  Eight where they are apart from the stages: a slot is
+  // held until the epilogue is done with its tile, and with four, tiles of one
+  // home chunk could not be converted ahead of the four accumulators (250k x
+  // 18 1.47 -> 1.44 ms).
+  static constexpr int NM = RAW == 4 ? 8 : NS;
   __align__(16) float cadd_a[128];  // -c   (A rows: x - c)
   __align__(16) float cadd_b[128];  // 2c   (B rows: -2 (x - c))
   uint32_t w_home;  // (window generation << 8) | index of the home bin in the window
@@ -984,14 +989,14 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
   } else if (warp >= MMA_WARP) {
     // ============================ MMA issuers
     // B tiles come in stage order; each is multiplied with the unit's ng home
-    // chunks into a TMEM accumulator (MMA tile counter mt), warp w of the two
-    // issuing every mt = w mod 2 into accumulators w and w + 2 in turn.
-    const uint32_t me = (uint32_t)(warp - MMA_WARP);
+    // chunks into a TMEM accumulator (MMA tile counter mt), warp w issuing
+    // every mt = w mod NMMA into accumulator w.
+    const uint32_t me = (uint32_t)(warp - MMA_WARP), b = me;
+    static_assert(NMMA == NACC, "an accumulator a warp");
     if (lane == 0) {
       const uint64_t desc_a = chunk_desc<KP>(smem_u32(Ahi)), desc_b = chunk_desc<KP>(smem_u32(Bhi));
       uint32_t tile = 0, mt = 0, unit_k = 0;
-      uint32_t use[2] = {0, 0}, nxt = 0;  // uses of accumulators me, me + 2 so far; the one to take next
-      int last_b = -1;
+      uint32_t use = 0;  // uses of accumulator me so far
       uint32_t last_par = 0;
       long long mw_full = 0, mw_dfree = 0;
       const long long m_start = T.prof ? clock64() : 0;
@@ -1001,16 +1006,14 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
         const bool fok = wait_or_abort(&S.full[st], (tile / NS) & 1, abort_flag, T.wait_limit);
         if (T.prof) mw_full += clock64() - c0;
         if (!fok) break;
-        const uint32_t flags = S.meta[ms].flags;
-        const uint32_t ng = S.meta[ms].ng;
+        const uint4 m4 = *reinterpret_cast<const uint4*>(&S.meta[ms]);
+        const uint32_t flags = m4.z, ng = m4.w;
         if (flags & FLAG_END) {
-          // wake every epilogue group on its next accumulator, but only once
-          // the group has taken that accumulator's previous use: an arrival
+          // wake the epilogue group on its next accumulator, but only once
+          // the group has taken the accumulator's previous use: an arrival
           // before that would complete a second phase of dfull[b] under a
           // warp still waiting for the first (parity aliasing)
-          for (uint32_t j = 0; j < 2; ++j) {
-            const uint32_t b = me + 2 * j;
-            if (!wait_or_abort(&S.dfree[b], ((j ? use[1] : use[0]) & 1) ^ 1, abort_flag, T.wait_limit)) break;
+          if (wait_or_abort(&S.dfree[b], (use & 1) ^ 1, abort_flag, T.wait_limit)) {
             S.acc[b].end = 1;
             mbar_arrive_n(&S.dfull[b], 2);
           }
@@ -1022,22 +1025,14 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
         // descriptors differ from the buffers' first ones by address / 16 alone
         const uint64_t dbh = desc_b + st * (OPB * 2 / 16), dbl = dbh + NS * (OPB * 2 / 16);
         constexpr uint32_t idesc = umma_idesc(TM, TN);
-        for (uint32_t g = 0; g < ng && ok; ++g) {
-          if (mt % NMMA != me) {
-            ++mt;
-            continue;
-          }
+        for (uint32_t g = (me - mt) % NMMA; g < ng; g += NMMA) {
           const long long c1 = T.prof ? clock64() : 0;
-          const uint32_t j = nxt, par = (j ? use[1] : use[0]) & 1, b = me + 2 * j;
+          const uint32_t par = use & 1;
           ok = wait_or_abort(&S.dfree[b], par ^ 1, abort_flag, T.wait_limit);
           if (T.prof) mw_dfree += clock64() - c1;
           if (!ok) break;
-          nxt = j ^ 1;
-          if (j) ++use[1]; else ++use[0];
-          if (T.stall_test) {  // failure-detection test: never signal, let the waits run out
-            ++mt;
-            continue;
-          }
+          ++use;
+          if (T.stall_test) continue;  // failure-detection test: never signal, let the waits run out
           asm volatile("tcgen05.fence::after_thread_sync;");
           S.acc[b] = TcAcc{ms, g, 0u};
           mbar_arrive(&S.dfull[b]);  // releases the metadata; the commit below completes the phase
@@ -1051,11 +1046,10 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
             mma_bf16(dt, dal + o, dbh + o, idesc, 1u);
           }
           tc_commit(&S.dfull[b]);
-          last_b = (int)b;
           last_par = par;
-          ++mt;
         }
         if (!ok) break;
+        mt += ng;
         if (!T.stall_test) tc_commit(&S.bfree[st]);
         if ((flags & FLAG_LAST) && !T.stall_test) {
           tc_commit(&S.afree);
@@ -1067,13 +1061,13 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
         atomicAdd(&T.ctr->prof[2], (unsigned long long)mw_full);
         atomicAdd(&T.ctr->prof[3], (unsigned long long)mw_dfree);
         atomicAdd(&T.ctr->prof[4], (unsigned long long)(clock64() - m_start));
-        atomicAdd(&T.ctr->prof[12], (unsigned long long)mt);
+        if (me == 0) atomicAdd(&T.ctr->prof[12], (unsigned long long)mt);
       }
       // an aborting CTA may still have MMAs in flight: wait (bounded) for the
       // last committed tile, MMAs complete in issue order
-      if (*abort_flag && last_b >= 0) {
+      if (*abort_flag && use > 0 && !T.stall_test) {
         volatile uint32_t no_abort = 0;
-        wait_or_abort(&S.dfull[last_b], last_par, &no_abort, T.wait_limit);
+        wait_or_abort(&S.dfull[b], last_par, &no_abort, T.wait_limit);
       }
     }
     __syncwarp();
@@ -1125,6 +1119,13 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
           uint32_t v[32];
           tmem_ld32_nowait(tbase + b * TN + ((quarter * 32u) << 16) + c0, v);
           tmem_wait();
+          // with the last block in registers the accumulator can be refilled
+          // (5M x 18 77.0 -> 75.3 ms, 100k x 18 1.55 -> 1.47)
+          if (c0 + 32 >= M.ncols) {
+            asm volatile("tcgen05.fence::before_thread_sync;");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&S.dfree[b]);
+          }
           // D' < 0 marks a candidate.  Three blocks of four hold none: a tree
           // of three-input ORs over the signs (16 operations) finds those;
           // extracting the 32 sign bits takes a funnel shift each, on a pipe
@@ -1201,10 +1202,9 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
             emit(bs, m & ~acc_bits, &P.ctr->band_n, P.band_list, P.band_cap, nullptr, rcb);
         }
       }
-      asm volatile("tcgen05.fence::before_thread_sync;");
       __syncwarp();
       if (lane == 0) {
-        mbar_arrive(&S.dfree[b]);
+        if (row0 >= M.na) mbar_arrive(&S.dfree[b]);
         mbar_arrive_n(&S.mfree[A.ms], 12u / M.ng);  // the tile served one of its home chunks
       }
     }
