@@ -132,7 +132,7 @@ struct TcBound {
   float uR2;               // 2uR (global centring error)
   float u1;                // u(1+u)
   float Dp;                // 1.1 sqrt(eps2)
-  float cap;               // 0.1 eps2: larger bounds re-decide the whole column in FP64
+  float cap;               // 0.1 eps2: up to here T <= 1.2 eps2 (column_threshold)
   float margin;            // small positive slack that makes D' >= 0 a strict reject
 };
 

@@ -25,8 +25,8 @@
 //   - tensor-core FP32 accumulation: taken as <= 2^-19 per MMA instruction
 //     relative to the sum of |products| (a generous allowance),
 //   - FP32 norms (g_d), the FP32 centring (2uR + u(|a'|+|q'|)),
-// with sum_k |A_k||B_k| <= (|a'| + |q'|)^2.  Rows whose bound exceeds
-// 0.1 eps2 are re-decided entirely in FP64 (T_lo = -1, T_hi = inf).
+// with sum_k |A_k||B_k| <= (|a'| + |q'|)^2.  Columns whose bound
+// exceeds 16 eps2 are re-decided entirely in FP64 (T_lo = -1, T_hi = inf).
 //
 // Data movement: operands are converted from the sorted FP32 rows into the
 // K-major layouts of chunk_off (tc_common.cuh), elected threads issue the MMAs

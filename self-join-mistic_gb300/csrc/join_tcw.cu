@@ -45,7 +45,7 @@
 // FP32 centring), plus the FP32 epilogue arithmetic (accounted for in
 // TcParams.kappa by the host): D' <= -dlt(n) accepts, D' < 0 otherwise goes
 // to the band list, whose pairs are re-decided with the reference FP64
-// predicate.  Columns whose bound exceeds 0.1 eps2 are re-decided entirely
+// predicate.  Columns whose bound exceeds 16 eps2 are re-decided entirely
 // in FP64.
 #include <cuda.h>
 #include <cudaTypedefs.h>

@@ -86,3 +86,21 @@ def test_pairs_around_the_band_medium_rows_on_the_k_chunked_kernel(handle, monke
     r = handle.selfjoin(x, 2, 1.0, mode="bf16", rp="user", rp_user=rps, pairs="host", sort_pairs=True)
     assert r.n_units_tc > 0 and r.tc_tiles > 0
     assert np.array_equal(r.pairs, ref), diff_pairs(r.pairs, ref)
+
+
+@pytest.mark.parametrize("d,prec,rho_max", [(18, "auto", 45.0), (18, "auto", 120.0), (18, "auto", 300.0),
+                                            (90, "auto", 100.0), (384, "tf32", 40.0), (384, "auto", 100.0)])
+def test_columns_with_wide_bounds(handle, monkeypatch, d, prec, rho_max):
+    """Bounds from a tenth of eps^2 to beyond 16 eps^2 (the largest radius of
+    the first kernel), where a column is left to FP64 whole: the pair sets
+    stay the oracle's, and up to there only pairs near the threshold are."""
+    monkeypatch.setenv("MISTIC_TC_MIN_BIN", "1")
+    monkeypatch.setenv("MISTIC_TC_WIDE", "0")
+    x, rps = shell_case(d, 1500, rho_max, seed=d * 1000 + int(rho_max))
+    ref = O.brute_pairs(x, 1.0)
+    r = handle.selfjoin(x, 2, 1.0, mode="tf32" if prec == "tf32" else "bf16", rp="user", rp_user=rps,
+                        pairs="host", sort_pairs=True)
+    assert r.n_units_tc > 0 and r.tc_tiles > 0
+    assert np.array_equal(r.pairs, ref), diff_pairs(r.pairs, ref)
+    if rho_max < 300.0:
+        assert r.band_pairs < r.candidates // 10
