@@ -146,7 +146,8 @@ struct TcShared2 {
   unsigned long long unit;
   uint32_t w_total, w_pos, seg_next, w_nb;
   uint32_t ra2max;  // float bits, non-negative
-  float cadd[2][2][RAW == 4 ? 32 : 1];  // K <= 32: [unit parity][A, B] as cadd_a, cadd_b
+  // K <= 32: [unit parity][A, B] as cadd_a, cadd_b, then the columns d and d + 1 (conv_row) and zeros
+  __align__(16) float cadd[2][2][RAW == 4 ? 32 : 4];
   uint32_t ra2[4];                      // K <= 32: largest |a|^2 by unit mod 4, float bits
   TcUnit units[RAW == 4 ? NUNIT : 1];
   TcSlot slot[RAW == 4 ? RAW : 1];
@@ -292,13 +293,16 @@ __device__ __forceinline__ void load_row(__nv_bfloat16* hi, __nv_bfloat16* lo, u
   }
 }
 
-// Converts row r, its 8-float blocks given by block(kb, x), into the bf16
-// hi/lo operand row (hi, lo), K blocks in order, with placeholders pd, pd1 in
-// the augmented columns d and d + 1; returns the row norm |x - c|^2 (times
-// scale^2).
+// Converts row r, its 8-float blocks given by block(kb, x) (zeros beyond
+// column d - 1), into the bf16 hi/lo operand row (hi, lo), K blocks in order;
+// returns the row norm |x - c|^2 (times scale^2).  cadd holds the constants of
+// the augmented columns d and d + 1 after the data's, so that every column is
+// one FMA: with a select by column instead, and cadd read a word at a time,
+// the converters were the slowest role of joins with one home chunk a unit
+// (5M x 18 69.0 -> 66.0 ms of tensor-core time, 100k x 18 1.45 -> 1.41).
 template <int KP, class Block>
 __device__ __forceinline__ float conv_row(Block block, __nv_bfloat16* hi, __nv_bfloat16* lo, uint32_t r,
-                                          const float* cadd, float scale, uint32_t d, float pd, float pd1) {
+                                          const float* cadd, float scale, uint32_t d) {
   float acc = 0.f;
 #pragma unroll
   for (int kb = 0; kb < KP / 8; ++kb) {
@@ -306,27 +310,12 @@ __device__ __forceinline__ float conv_row(Block block, __nv_bfloat16* hi, __nv_b
     if (k0 >= d + 2) break;  // zero blocks (cleared at the start)
     float x[8], v[8];
     block(kb, x);
-    if (k0 + 8 <= d) {
+    const float4 c0 = *reinterpret_cast<const float4*>(cadd + k0), c1 = *reinterpret_cast<const float4*>(cadd + k0 + 4);
+    const float c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        v[i] = fmaf(x[i], scale, cadd[k0 + i]);
-        acc = fmaf(v[i], v[i], acc);
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const uint32_t k = k0 + i;
-        float t = 0.f;
-        if (k < d) {
-          t = fmaf(x[i], scale, cadd[k]);
-          acc = fmaf(t, t, acc);
-        } else if (k == d) {
-          t = pd;
-        } else if (k == d + 1) {
-          t = pd1;
-        }
-        v[i] = t;
-      }
+    for (int i = 0; i < 8; ++i) {
+      v[i] = fmaf(x[i], scale, c[i]);
+      if (k0 + i < d) acc = fmaf(v[i], v[i], acc);
     }
     store_split(hi, lo, off, v);
   }
@@ -552,7 +541,7 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
       unsigned long long n_tiles = 0, n_cells = 0;
       uint32_t a0 = 0, na = 0, ng = 0, inst = 0;
       TcBound tb = T.b;
-      float ra2max = 0.f;
+      float ra = 0.f;  // bound of the unit's largest |a|
       long long pw_sfree = 0, pw_raw = 0;
       const long long p_start = T.prof ? clock64() : 0;
       for (uint32_t tile = 0;; ++tile) {
@@ -583,10 +572,10 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
           a0 = W.a0, na = W.na, ng = W.ng, inst = W.inst;
           tb = W.tb;
           float* ca = S.cadd[useq & 1][0];
-          if (c < P.dpad) {
-            const float x = X[(size_t)a0 * P.dpad + c];
-            ca[c] = -x;
-            S.cadd[useq & 1][1][c] = 2.f * x;
+          if (c < KP) {
+            const float x = c < P.d ? X[(size_t)a0 * P.dpad + c] : 0.f;
+            ca[c] = c == P.d + 1 ? 1.f : -x;
+            S.cadd[useq & 1][1][c] = c == P.d ? 1.f : 2.f * x;
           }
           if (c == 0) S.ra2[(useq + 2) & 3] = 0;  // last read two units ago
           mbar_arrive(&S.ubar);
@@ -606,7 +595,7 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
                 x[4] = f[2 * kb + 1].x, x[5] = f[2 * kb + 1].y, x[6] = f[2 * kb + 1].z, x[7] = f[2 * kb + 1].w;
               };
               __nv_bfloat16 *ah = Ahi + g * OPB, *al = Alo + g * OPB;
-              const float nrm = conv_row<KP>(block, ah, al, c, ca, 1.f, P.d, 0.f, 1.f);
+              const float nrm = conv_row<KP>(block, ah, al, c, ca, 1.f, P.d);
               patch_col<KP>(ah, al, c, P.d, nrm);
               m = fmaxf(m, nrm);
             }
@@ -618,7 +607,7 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
           mbar_arrive(&S.afull);
           mbar_arrive(&S.ubar);
           if (!__all_sync(FULL_MASK, wait_or_abort(&S.ubar, 1, abort_flag, T.wait_limit))) break;
-          ra2max = __uint_as_float(*(volatile uint32_t*)&S.ra2[useq & 3]);
+          ra = norm_bound(tb, __uint_as_float(*(volatile uint32_t*)&S.ra2[useq & 3]));
           ++useq;
         }
         __nv_bfloat16 *bh = Bhi + st * OPB, *bl = Blo + st * OPB;
@@ -629,9 +618,9 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
           };
           S.qid[ms][c] = S.rid[rs][c];
           const float nq2 =
-              conv_row<KP>(block, bh, bl, c, S.cadd[(useq - 1) & 1][1], -2.f, P.d, 1.f, 0.f) * 0.25f;
+              conv_row<KP>(block, bh, bl, c, S.cadd[(useq - 1) & 1][1], -2.f, P.d) * 0.25f;
           float tcol = 0.f, dl = 0.f;
-          if (!column_threshold(tb, ra2max, nq2, &tcol, &dl)) {
+          if (!column_threshold(tb, ra, nq2, &tcol, &dl)) {
             tcol = 1e30f;   // every row of this column becomes a candidate ...
             dl = INFINITY;  // ... and none is accepted without the FP64 check
           }
@@ -933,7 +922,7 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
         const float part = conv_pass1<KP>(sh, sl, bh, bl, prow, half, ok, S.cadd_b, -2.f, P.d, 1.f, 0.f);
         const float nq2 = row_norm(part) * 0.25f;
         float tcol = 0.f, dl = 0.f;
-        if (ok && !column_threshold(tb, ra2max, nq2, &tcol, &dl)) {
+        if (ok && !column_threshold(tb, norm_bound(tb, ra2max), nq2, &tcol, &dl)) {
           tcol = 1e30f;   // every row of this column becomes a candidate ...
           dl = INFINITY;  // ... and none is accepted without the FP64 check
         }

@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(WTHREADS, 1)
           qid = P.ids[q];
           const float nq2 = T.xn[q];
           float tcol;
-          if (column_threshold(T.b, ra2max, nq2, &tcol, &dl)) {
+          if (column_threshold(T.b, norm_bound(T.b, ra2max), nq2, &tcol, &dl)) {
             hqv = nq2 - tcol;
           } else {
             hqv = -1e30f;   // every row of this column becomes a candidate ...

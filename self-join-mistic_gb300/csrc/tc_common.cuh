@@ -170,9 +170,9 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 }
 
 // Per-column threshold T(n) and accept distance dlt(n) of the tensor-core
-// filter, from the unit's largest |a|^2 and this column's |q|^2 (FP32,
-// rounded outward).  Returns false when the bound is too wide to be worth a
-// threshold (the column is then re-decided entirely in FP64).
+// filter, from the unit's largest |a| (norm_bound of |a|^2) and this column's
+// |q|^2 (FP32, rounded outward).  Returns false when the bound is too wide to
+// be worth a threshold (the column is then re-decided entirely in FP64).
 //
 // E = kappa (rs^2 + t) + delta (2 Dp + delta), rs = |a'| + |q'|, bounds
 // |D - s64| for pairs at distance x <= Dp = 1.1 eps when T <= t, T being part
@@ -185,9 +185,10 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 // eps2.  Of the 3.2e8 pairs that a heavy-tailed 5M x 18 join left to the FP64
 // predicate, 3.0e8 were whole columns beyond the first of the two (0.2 % of
 // its cells).
-__device__ __forceinline__ bool column_threshold(const TcBound& T, float ra2max, float nq2, float* tcol,
-                                                 float* dlt) {
-  const float ra = sqrtf(ra2max * T.ginf), rq = sqrtf(nq2 * T.ginf);
+__device__ __forceinline__ float norm_bound(const TcBound& T, float n2) { return sqrtf(n2 * T.ginf); }
+
+__device__ __forceinline__ bool column_threshold(const TcBound& T, float ra, float nq2, float* tcol, float* dlt) {
+  const float rq = norm_bound(T, nq2);
   const float rs = ra + rq;
   const float delta = T.uR2 + T.u1 * rs;
   float E = (T.kappa * (rs * rs + 1.2f * T.eps2_hi) + delta * (2.f * T.Dp + delta)) * 1.001f;
