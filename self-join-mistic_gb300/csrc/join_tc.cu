@@ -1217,8 +1217,8 @@ template <int KP>
 struct TcShape {
   static constexpr int G = KP <= 32 ? 4 : (KP <= 64 ? 2 : 1);
   static constexpr int NS = KP <= 32 ? 4 : (KP <= 96 ? 3 : 2);
-  // separate landing slots where they fit: four for K <= 32 (pair mode, two
-  // pairs of tiles in flight), three for K = 48
+  // separate landing slots where they fit: four for K <= 32 (tiles on their
+  // way to the converters), three for K = 48
   static constexpr int RAW = KP <= 32 ? 4 : (KP <= 48 ? 3 : 0);
   // short rows: many tiles, pairs and hits per converted row -> more epilogue
   // warps (16: 72 registers a thread); long rows: 8 (96 registers)

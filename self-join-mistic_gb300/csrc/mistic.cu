@@ -414,8 +414,9 @@ uint32_t tc_min_bin(uint32_t d, bool wide) {
   // long rows (K-chunked kernel): every bin.  Even a one-row bin is joined
   // faster on the tensor cores (a 128-row tile at ~1/128 use) than by the
   // FP32 CUDA-core kernel, whose units of a small home bin against a very
-  // large neighbour bin (one segment holds a whole bin) run on single warps:
-  // on the 5M x 384 workload such units took 2.1 s of a 14 s join at T = 8.
+  // large neighbour bin run on few warps:
+  // on the 5M x 384 workload such units took 2.1 s of a 14 s join at T = 8,
+  // when a segment still held a whole bin.
   if (wide) return 1;
   return (uint32_t)std::min(96.0, std::max(1.0, std::floor(16000.0 / ((double)d * d))));
 }

@@ -12,11 +12,13 @@
 // about four times; the 8-bit radix sort of the packed pairs it replaces
 // moved it three times per digit over 5 to 8 digits, most of them needed only
 // to tell rows apart.  Sorted lists, before and after: 1.53e8 pairs of 5M rows
-// 17.6 -> 5.8 ms, 1.7e7 pairs of 2M rows 1.90 -> 0.46 ms; the table of 1.6e5
+// 17.6 -> 4.6 ms, 1.7e7 pairs of 2M rows 1.90 -> 0.46 ms; the table of 1.6e5
 // pairs of 20,011 rows 0.26 -> 0.10 ms.
 //
 // Bounds: the counting and placing passes by one atomic and one scattered
 // 4-byte access an entry, the row sort by HBM.
+#include <type_traits>
+
 #include "internal.cuh"
 
 namespace mistic {
@@ -25,7 +27,7 @@ namespace {
 constexpr int RW_THREADS = 256;
 constexpr int RW_ITEMS = 4;                  // pairs a thread has in flight
 constexpr uint32_t ROW_REG_MAX = 256;        // rows sorted in a warp's registers
-constexpr uint32_t ROW_SMEM_MAX = 8192;      // rows sorted in shared memory
+constexpr uint32_t ROW_BLOCK_MAX = 8192;     // rows sorted in a block's registers
 constexpr int RL_THREADS = 256;              // block of the long-row kernel
 constexpr int RL_BINS = 256;
 
@@ -119,34 +121,66 @@ __device__ __forceinline__ void put(const RowOut& R, size_t e, uint32_t i, uint3
     R.pairs[e] = ((unsigned long long)(j - r0) << 32) | (i - r0);
 }
 
-// Ascending bitonic sort of 32 E values, value idx = 32 e + lane in v[e].
+// The steps j = j0, j0 / 2 .. 1 of a bitonic merge of length k inside a warp;
+// value idx = base + 32 e + lane is in v[e], base a multiple of 32 E.
 template <int E>
-__device__ __forceinline__ void warp_sort(uint32_t (&v)[E]) {
+__device__ __forceinline__ void warp_merge(uint32_t (&v)[E], uint32_t base, int k, int j0) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
-  for (int k = 2; k <= 32 * E; k <<= 1) {
+  for (int j = 16 * E; j > 0; j >>= 1) {
+    if (j > j0) continue;
+    if (j >= 32) {
 #pragma unroll
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      if (j >= 32) {
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-          const int f = e ^ (j >> 5);
-          if (f > e) {
-            const bool up = ((32 * e) & k) == 0;  // k > j >= 32: the direction depends on e alone
-            const uint32_t a = min(v[e], v[f]), b = max(v[e], v[f]);
-            v[e] = up ? a : b;
-            v[f] = up ? b : a;
-          }
-        }
-      } else {
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-          const uint32_t o = __shfl_xor_sync(FULL_MASK, v[e], j);
-          const bool up = ((32 * e + lane) & k) == 0, low = (lane & j) == 0;
-          v[e] = (up == low) ? min(v[e], o) : max(v[e], o);
+      for (int e = 0; e < E; ++e) {
+        const int f = e ^ (j >> 5);
+        if (f > e) {
+          const bool up = ((base + 32 * e) & k) == 0;  // k > j >= 32: the lane has no say in the direction
+          const uint32_t a = min(v[e], v[f]), b = max(v[e], v[f]);
+          v[e] = up ? a : b;
+          v[f] = up ? b : a;
         }
       }
+    } else {
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const uint32_t o = __shfl_xor_sync(FULL_MASK, v[e], j);
+        const bool up = ((base + 32 * e + lane) & k) == 0, low = (lane & j) == 0;
+        v[e] = (up == low) ? min(v[e], o) : max(v[e], o);
+      }
     }
+  }
+}
+
+// Bitonic sort of the warp's 32 E values: ascending, or (base & 32 E) descending.
+template <int E>
+__device__ __forceinline__ void warp_sort(uint32_t (&v)[E], uint32_t base = 0) {
+#pragma unroll
+  for (int k = 2; k <= 32 * E; k <<= 1) warp_merge<E>(v, base, k, k >> 1);
+}
+
+// Ascending sort of a block's 32 E RL_THREADS / 32 values, warp w's from 32 E w
+// on: only the steps between warps go through shared memory (sv), 6 of the 45
+// to 91.
+template <int E>
+__device__ __forceinline__ void block_sort(uint32_t (&v)[E], uint32_t* sv) {
+  const uint32_t lane = threadIdx.x & 31, base = (threadIdx.x >> 5) * 32 * E;
+  warp_sort<E>(v, base);
+#pragma unroll 1
+  for (uint32_t k = 64 * E; k <= RL_THREADS * E; k <<= 1) {
+#pragma unroll 1
+    for (uint32_t j = k >> 1; j >= 32 * E; j >>= 1) {
+      __syncthreads();
+#pragma unroll
+      for (int e = 0; e < E; ++e) sv[base + 32 * e + lane] = v[e];
+      __syncthreads();
+      const bool keep_min = ((base & k) == 0) == ((base & j) == 0);
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const uint32_t o = sv[(base + 32 * e + lane) ^ j];
+        v[e] = keep_min ? min(v[e], o) : max(v[e], o);
+      }
+    }
+    warp_merge<E>(v, base, (int)k, 16 * E);
   }
 }
 
@@ -232,11 +266,13 @@ __global__ void __launch_bounds__(RW_THREADS) k_row_sort(const RowOut R) {
 }
 
 // Rows above ROW_REG_MAX entries, a block a row, claimed from the list.  Up
-// to ROW_SMEM_MAX entries are sorted in shared memory; longer rows by a
+// to ROW_BLOCK_MAX entries are sorted in the block's registers (in shared
+// memory, a barrier a step, these rows took 2.0 ms of a 5M x 18 join's sorted
+// list; now 1.0); longer rows by a
 // stable 8-bit radix sort through global memory, between the unsorted ids and
 // the row's own place in the output (which is at least as large).
-__global__ void __launch_bounds__(RL_THREADS) k_row_sort_long(const RowOut R) {
-  extern __shared__ uint32_t sv[];  // ROW_SMEM_MAX
+__global__ void __launch_bounds__(RL_THREADS, 4) k_row_sort_long(const RowOut R) {
+  extern __shared__ uint32_t sv[];  // ROW_BLOCK_MAX
   __shared__ uint32_t s_claim, wcnt[RL_THREADS / 32][RL_BINS], ws[RL_THREADS / 32], gbase[RL_BINS];
   const uint32_t total = R.long_n[0];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -248,24 +284,28 @@ __global__ void __launch_bounds__(RL_THREADS) k_row_sort_long(const RowOut R) {
     const uint32_t i = R.long_rows[s_claim], r0 = row_base(R, i);
     const size_t b = row_begin(R, i);
     const uint32_t len = (uint32_t)(row_begin(R, (size_t)i + 1) - b);
-    if (len <= ROW_SMEM_MAX) {
-      uint32_t N = 512;
-      while (N < len) N <<= 1;
-      for (uint32_t t = tid; t < N; t += RL_THREADS) sv[t] = t < len ? R.ids[b + t] : 0xffffffffu;
-      for (uint32_t k = 2; k <= N; k <<= 1)
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-          __syncthreads();
-          for (uint32_t t = tid; t < N / 2; t += RL_THREADS) {
-            const uint32_t x = 2 * t - (t & (j - 1)), y = x + j;  // bit j of x is clear
-            const uint32_t p = sv[x], q = sv[y];
-            if ((p > q) == ((x & k) == 0)) {
-              sv[x] = q;
-              sv[y] = p;
-            }
-          }
-        }
-      __syncthreads();
-      for (uint32_t t = tid; t < len; t += RL_THREADS) put(R, b + t, i, sv[t], r0);
+    if (len <= ROW_BLOCK_MAX) {
+      auto row = [&](auto e_) {
+        constexpr int E = decltype(e_)::value;
+        uint32_t v[E];
+        const uint32_t t0 = w * 32 * E + lane;
+#pragma unroll
+        for (int e = 0; e < E; ++e) v[e] = t0 + 32 * e < len ? R.ids[b + t0 + 32 * e] : 0xffffffffu;
+        block_sort<E>(v, sv);
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+          if (t0 + 32 * e < len) put(R, b + t0 + 32 * e, i, v[e], r0);
+      };
+      if (len <= 2 * RL_THREADS)
+        row(std::integral_constant<int, 2>());
+      else if (len <= 4 * RL_THREADS)
+        row(std::integral_constant<int, 4>());
+      else if (len <= 8 * RL_THREADS)
+        row(std::integral_constant<int, 8>());
+      else if (len <= 16 * RL_THREADS)
+        row(std::integral_constant<int, 16>());
+      else
+        row(std::integral_constant<int, 32>());
       continue;
     }
     uint32_t* src = R.ids + b;
@@ -365,7 +405,7 @@ static void sort_rows(mistic_handle_s* h, const unsigned long long* in, size_t n
   k_row_sort<<<(unsigned)((n + per_block - 1) / per_block), RW_THREADS, 0, h->stream>>>(R);
   launched(h, "row_sort");
   k_row_sort_long<<<(unsigned)std::min<size_t>((size_t)h->sms * 4, max_long), RL_THREADS,
-                    ROW_SMEM_MAX * sizeof(uint32_t), h->stream>>>(R);
+                    ROW_BLOCK_MAX * sizeof(uint32_t), h->stream>>>(R);
   launched(h, "row_sort_long");
 }
 
