@@ -403,9 +403,9 @@ int bit_length(uint64_t v) {
 // it, for tuning).  A tensor-core tile costs about the same per candidate row
 // whatever its number of home rows, a CUDA-core unit costs d FMAs per cell,
 // so small bins go to the CUDA cores.  Measured on GB300 (whole join, ms):
-//   5M x 18:        T = 24: 105.7, 32: 104.1, 44: 103.4, 66: 104.7, 89: 108.0
-//   250,007 x 18:   T = 24: 2.81, 32: 2.79, 44: 2.78, 66: 2.81, 89: 2.92
-//   100,000 x 18:   T = 24: 1.98, 32: 1.99, 44: 1.99, 66: 2.01, 89: 2.05
+//   5M x 18:        T = 16: 92.3, 24: 89.4, 32: 88.1, 40: 87.8, 49: 88.1, 66: 89.5
+//   250,007 x 18:   T = 16: 2.79, 24: 2.66, 32: 2.64, 40: 2.61, 49: 2.64, 66: 2.67
+//   100,000 x 18:   T = 16: 1.65, 24: 1.62, 32: 1.62, 40: 1.62, 49: 1.63, 66: 1.65
 //   515k x 90 (short-row kernel): T = 1: 259.9, 2: 261.9, 4: 261.9, 8: 263.3
 // hence 16000 / d^2, clamped to [1, 96].
 uint32_t tc_min_bin(uint32_t d, bool wide) {
