@@ -133,6 +133,7 @@ struct TcBound {
   float u1;                // u(1+u)
   float Dp;                // 1.1 sqrt(eps2)
   float cap;               // 0.1 eps2: up to here T <= 1.2 eps2 (column_threshold)
+  float cap2;              // 16 eps2 (no more than keeps T finite): up to here T <= 17.2 eps2
   float margin;            // small positive slack that makes D' >= 0 a strict reject
 };
 

@@ -1102,6 +1102,7 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
     tp.b.u1 = (float)(u * (1.0 + u) * 1.0001);
     tp.b.Dp = (float)(1.1 * sqrt(eps2));
     tp.b.cap = (float)(0.1 * eps2);
+    tp.b.cap2 = (float)std::max(0.1 * eps2, std::min(16.0 * eps2, 1e36));
     tp.b.margin = (float)(1e-6 * eps2);
     // MISTIC_TEST_TC_STALL=1 is the failure-detection test: the MMA warp
     // signals nothing, every bounded wait runs out after a short limit, the

@@ -169,6 +169,9 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 
+// Bound of a row norm from its FP32 square.
+__device__ __forceinline__ float norm_bound(const TcBound& T, float n2) { return sqrtf(n2 * T.ginf); }
+
 // Per-column threshold T(n) and accept distance dlt(n) of the tensor-core
 // filter, from the unit's largest |a| (norm_bound of |a|^2) and this column's
 // |q|^2 (FP32, rounded outward).  Returns false when the bound is too wide to
@@ -181,12 +184,10 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 // at most delta, so if delta <= Dp then D >= (Dp - delta)^2 - kappa (rs^2 + t)
 // >= Dp^2 - E > eps2_lo - E, and if delta > Dp then E > 3 Dp^2 + kappa (rs^2 +
 // t) while D >= -kappa (rs^2 + t).  Hence E may be any size as long as t
-// covers T: 1.2 eps2 up to E = cap = 0.1 eps2, and 17.2 eps2 up to E = 16
-// eps2.  Of the 3.2e8 pairs that a heavy-tailed 5M x 18 join left to the FP64
+// covers T: 1.2 eps2 up to E = cap = 0.1 eps2, and 17.2 eps2 up to E = cap2 =
+// 16 eps2.  Of the 3.2e8 pairs that a heavy-tailed 5M x 18 join left to the FP64
 // predicate, 3.0e8 were whole columns beyond the first of the two (0.2 % of
 // its cells).
-__device__ __forceinline__ float norm_bound(const TcBound& T, float n2) { return sqrtf(n2 * T.ginf); }
-
 __device__ __forceinline__ bool column_threshold(const TcBound& T, float ra, float nq2, float* tcol, float* dlt) {
   const float rq = norm_bound(T, nq2);
   const float rs = ra + rq;
@@ -195,7 +196,7 @@ __device__ __forceinline__ bool column_threshold(const TcBound& T, float ra, flo
   // (a select, not a branch: the join of 100k x 18 uniform points, which has
   // no such column, is 0.7 % slower with one)
   E = E <= T.cap ? E : fmaf(T.kappa * 16.1f, T.eps2_hi, E);
-  if (!(E <= 160.f * T.cap)) return false;
+  if (!(E <= T.cap2)) return false;
   float t = T.eps2_hi + E + T.margin;
   t += fabsf(t) * 1e-6f;
   float dl = (T.eps2_hi - T.eps2_lo) + 2.f * E + T.margin;
