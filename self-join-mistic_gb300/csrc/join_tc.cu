@@ -82,13 +82,19 @@ constexpr int WIN = 256;         // neighbour bins per candidate window
 //   rawfree[r] converters -> loaders    (4 arrivals: slot read)
 //   ubar       converters among themselves, twice a unit (128 arrivals)
 //   full[s]    producers  -> MMA        (128 arrivals, or NPROD)
-//   bfree[s]   MMA        -> converters (a tcgen05.commit by each MMA warp: stage s read)
-//   mfree[m]   epilogue   -> producers  (metadata slot m, and with it the stage of K >= 48; 48 arrivals: 12 / home
-//                                        chunks by each of a group's 4 warps)
+//   bfree[s]   MMA        -> producers  (a tcgen05.commit by each MMA warp, whether or not the tile holds work
+//                                        for it: stage s read, full[s] and the tile's metadata seen)
+//   mfree[m]   epilogue   -> producers  (metadata slot m drained; 48 arrivals: 12 / home chunks by each of a
+//                                        group's 4 warps)
 //   dfull[b]   MMA        -> epilogue   (tcgen05.commit, + 1 for the accumulator's metadata)
 //   dfree[b]   epilogue   -> MMA        (4 arrivals; accumulator b reusable)
 //   afull      producers  -> MMA        (128 arrivals, or NPROD, per unit: A written)
 //   afree      MMA        -> producers  (a tcgen05.commit by each MMA warp after a unit's last tile)
+// A stage and its metadata slot are written again after both bfree and mfree.
+// mfree alone says only that the warps which own a home chunk of the tile have
+// issued it: a warp that owns none may not have waited on full[s] yet, and a
+// second completion of full[s] would leave it on the wrong phase, or reading
+// the wrong tile's metadata.
 constexpr int NPW = 8;     // producer warps: two threads per operand row
 constexpr int NPROD = NPW * 32;
 constexpr int NLOAD = 128; // K <= 32: threads of the loader warps, and of the converter warps after them
@@ -678,10 +684,16 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
     // before t
     constexpr uint32_t LA = RAW > 0 ? RAW : (NS - 1 < 3 ? NS - 1 : 3);
     const long long p_start = T.prof ? clock64() : 0;
-    auto end_marker = [&]() {  // last tile slot: tells the MMA warp and the epilogue to stop
+    // bounded wait until stage k % NS may take tile k (bfree and mfree, see the barrier table)
+    auto stage_free = [&](uint32_t k) -> bool {
+      const uint32_t st = k % NS, par = ((k / NS) & 1) ^ 1;
+      return wait_or_abort(&S.mfree[st], par, abort_flag, T.wait_limit) &&
+             wait_or_abort(&S.bfree[st], par, abort_flag, T.wait_limit);
+    };
+    auto end_marker = [&]() {  // last tile slot: tells the MMA warps and the epilogue to stop
       const uint32_t st = tile % NS;
       if (tid == 0) {
-        wait_or_abort(&S.mfree[st], ((tile / NS) & 1) ^ 1, abort_flag, T.wait_limit);
+        stage_free(tile);
         S.meta[st].flags = FLAG_END;
       }
       prod_sync();
@@ -837,7 +849,7 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
           const uint32_t sl = pf++ & 1;
           if (tid == 0) {
             const long long c0 = T.prof ? clock64() : 0;
-            S.pflag[sl] = wait_or_abort(&S.mfree[st], ((issued / NS) & 1) ^ 1, abort_flag, T.wait_limit) ? 1u : 0u;
+            S.pflag[sl] = stage_free(issued) ? 1u : 0u;
             if (T.prof) pw_sfree += clock64() - c0;
           }
           prod_sync();
@@ -906,7 +918,7 @@ __global__ void __launch_bounds__(tc_threads(NEPI), 1) k_join_tc(const JoinParam
           const long long cb0 = T.prof ? clock64() : 0;
           if (tid == 0) {
             const long long c0 = T.prof ? clock64() : 0;
-            S.pflag[fl] = wait_or_abort(&S.mfree[st], ((tile / NS) & 1) ^ 1, abort_flag, T.wait_limit) ? 1u : 0u;
+            S.pflag[fl] = stage_free(tile) ? 1u : 0u;
             if (T.prof) pw_sfree += clock64() - c0;
           }
           prod_sync();
