@@ -905,6 +905,16 @@ __global__ void k_unit_plan(const uint32_t* __restrict__ bstart, uint32_t m, Enu
       const unsigned long long fair = (tot->work[c] / P.want_units[c] + 127) & ~127ull;
       seg[c] = (uint32_t)min((unsigned long long)P.seg_max[c], max((unsigned long long)P.seg_min[c], fair));
     }
+    // A bin of n points holds n^2 / (2 chunk seg) units, so a few very large
+    // bins would run past the work lists' 32-bit offsets, and long before that
+    // take gigabytes at 24 bytes a unit: 4,096-point segments of 12M points in
+    // one bin are 4.4e9 units at chunks of 4.  work / seg + one a chunk bounds
+    // the units of a class.
+    if (P.max_units) {
+      unsigned long long len = min(tot->work[c] / P.max_units + 1, 1ull << 30);
+      if (P.seg_to_bin) len = min(len, (unsigned long long)tot->max_bin);
+      seg[c] = (uint32_t)max((unsigned long long)seg[c], len);
+    }
     const uint32_t csz = c ? P.tc_chunk : P.chunk;  // a multiple of the home chunk (seg_chunks)
     seg[c] = (seg[c] + csz - 1) / csz * csz;
   }
@@ -936,6 +946,15 @@ __global__ void k_unit_plan(const uint32_t* __restrict__ bstart, uint32_t m, Enu
     for (int k = 0; k < 3; ++k)
       if (s[k + 1]) atomicAdd(&tot->n[k], s[k + 1]);
   }
+}
+
+// Points of the largest bin into *out (zero before).
+__global__ void k_max_bin(const uint32_t* __restrict__ bstart, uint32_t m, uint32_t* __restrict__ out) {
+  uint32_t v = 0;
+  for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < m; b += gridDim.x * blockDim.x)
+    v = max(v, bstart[b + 1] - bstart[b]);
+  v = __reduce_max_sync(FULL_MASK, v);
+  if ((threadIdx.x & 31) == 0 && v) atomicMax(out, v);
 }
 
 // Bins per prefix of the enumeration table: cnt[v] += 1 for each bin whose
@@ -1095,6 +1114,10 @@ void enum_count(mistic_handle_s* h, const uint64_t* bkey, const uint32_t* bstart
                                                           nullptr, nullptr, nullptr, nullptr, nullptr);
   launched(h, "enum_count");
   const unsigned nb = std::max(1u, std::min((m + 255) / 256, 4u * (unsigned)h->sms));
+  if (P.seg_to_bin) {
+    k_max_bin<<<nb, 256, 0, h->stream>>>(bstart, m, &tot->max_bin);
+    launched(h, "max_bin");
+  }
   k_unit_plan<<<nb, 256, 0, h->stream>>>(bstart, m, P, npts, nbr_cnt, unit_cnt, unit_cnt_tc, tot);
   launched(h, "unit_plan");
   exclusive_scan3(h, nbr_cnt, unit_cnt, unit_cnt_tc, m);

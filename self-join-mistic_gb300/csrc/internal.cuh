@@ -111,6 +111,10 @@ struct EnumParams {
   // and the number of units that small joins shorten their segments for (0:
   // always the longest), for CUDA-core [0] and tensor-core [1] units
   uint32_t seg_max[2], seg_min[2], want_units[2];
+  // beyond about this many units of a class, segments grow past seg_max (0:
+  // no limit); with seg_to_bin up to the largest bin's size only
+  uint32_t max_units;
+  int seg_to_bin;
   uint32_t chunk;    // home points per CUDA-core unit
   uint32_t tc_min;   // home bins with at least this many points get tensor-core units (0: none)
   uint32_t tc_chunk; // home points per tensor-core unit
@@ -347,6 +351,7 @@ struct EnumTotals {
   unsigned long long n[3];      // neighbour bins, CUDA-core units, tensor-core units
   unsigned long long work[2];   // sum over home chunks of their candidate points, by unit class
   uint32_t seg[2];              // segment lengths chosen
+  uint32_t max_bin;             // points of the largest bin (EnumParams.seg_to_bin only)
 };
 void enum_count(mistic_handle_s*, const uint64_t* bkey, const uint32_t* bstart, uint32_t m, const EnumParams&,
                 uint32_t* npts, uint32_t* nbr_cnt, uint2* lane_off, uint32_t* unit_cnt, uint32_t* unit_cnt_tc,

@@ -998,6 +998,17 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
     ep.want_units[0] = (ex ? 16u : 128u) * (uint32_t)h->sms;
     ep.want_units[1] = (ex ? 1u : 6u) * (uint32_t)h->sms;
   }
+  // MISTIC_TEST_WORKLIST_LIMIT=k lowers the limit on the work lists' lengths
+  // (tests of its check and of the segments that grow to keep below it)
+  unsigned long long worklist_limit = 0xffffffffull - 1;
+  if (const char* ev = getenv("MISTIC_TEST_WORKLIST_LIMIT"))
+    worklist_limit = std::min(worklist_limit, strtoull(ev, nullptr, 10));
+  // 2^25 units are 0.8 GB, 6,900 a resident warp of the CUDA-core join: more
+  // of them balance nothing better.  The pair ring needs a unit's pairs to fit
+  // it, so there no segment grows beyond the largest bin (what a unit holds at
+  // least when bins are not cut).
+  ep.max_units = (uint32_t)std::max(1ull, std::min(1ull << 25, worklist_limit / 2));
+  ep.seg_to_bin = o.ring_capacity != 0;
   ep.sample = o.home_sample;
   ep.tc_min = use_tc ? tc_min_bin(d, wide) : 0u;
   ep.tc_chunk = use_tc ? (wide ? 256u : join::tc_rows(d)) : 128;
@@ -1043,11 +1054,8 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
     d2h(h, &ht, tot_dev, sizeof ht);
     totc = ht.cand;
     simt_work = ht.work[0];
-    // MISTIC_TEST_WORKLIST_LIMIT=k lowers the limit (tests of this check)
-    unsigned long long lim = 0xffffffffull - 1;
-    if (const char* ev = getenv("MISTIC_TEST_WORKLIST_LIMIT")) lim = std::min(lim, strtoull(ev, nullptr, 10));
     for (int i = 0; i < 3; ++i) {
-      if (ht.n[i] > lim)
+      if (ht.n[i] > worklist_limit)
         throw Error(MISTIC_ERR_TOO_LARGE,
                     "neighbour-bin or work-unit list beyond the 32-bit offsets of the join work lists "
                     "(raise eps resolution: more reference points, or split the input)");
