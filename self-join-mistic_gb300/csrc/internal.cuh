@@ -45,7 +45,9 @@ struct Arena {
   };
   std::map<std::string, Buf> bufs;
   cudaStream_t stream = nullptr;  // work using the buffers; drained before a regrow
+  size_t growth_left = SIZE_MAX;  // bytes this call may still add (tests of exhausted device memory)
   void* get(const std::string& name, size_t bytes);
+  bool may_grow(size_t bytes) const { return bytes <= growth_left; }
   void release_all();
 };
 

@@ -68,14 +68,15 @@ void* Arena::get(const std::string& name, size_t bytes) {
     b.p = nullptr;
     b.bytes = 0;
     size_t want = bytes + bytes / 8;  // head-room against regrowth
-    cudaError_t e = cudaMalloc(&b.p, want);
-    if (e != cudaSuccess) {
+    cudaError_t e = may_grow(want) ? cudaMalloc(&b.p, want) : cudaErrorMemoryAllocation;
+    if (e != cudaSuccess && may_grow(bytes)) {
       cudaGetLastError();
       e = cudaMalloc(&b.p, bytes);
       want = bytes;
     }
     if (e != cudaSuccess) throw_cuda(e, ("cudaMalloc " + name).c_str(), __FILE__, __LINE__);
     b.bytes = want;
+    if (growth_left != SIZE_MAX) growth_left -= want;
   }
   return b.p;
 }
@@ -224,6 +225,15 @@ struct PinnedHold {
     p = nullptr;
   }
   ~PinnedHold() { reset(); }
+};
+
+// A device block owned by a call until it is handed to the result; an error
+// that unwinds the call frees it.
+struct DeviceHold {
+  void* p = nullptr;
+  ~DeviceHold() {
+    if (p) cudaFree(p);
+  }
 };
 
 template <class T>
@@ -737,6 +747,10 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
   if (!r) throw Error(MISTIC_ERR_INVALID_ARG, "null result");
   memset(r, 0, sizeof(*r));
   check_handle(h);
+  // MISTIC_TEST_DEVICE_GROWTH=k: the call may take k more bytes of device
+  // memory than the handle holds (tests of exhausted device memory)
+  const char* growth = getenv("MISTIC_TEST_DEVICE_GROWTH");
+  h->arena.growth_left = growth && *growth ? (size_t)strtoull(growth, nullptr, 10) : SIZE_MAX;
   if (dt != MISTIC_F64 && dt != MISTIC_F32) throw Error(MISTIC_ERR_INVALID_ARG, "unknown dtype");
   if (d == 0) throw Error(MISTIC_ERR_INVALID_ARG, "d must be >= 1");
   if (d > MAX_D) throw Error(MISTIC_ERR_TOO_LARGE, "d above the supported maximum (4096)");
@@ -1636,25 +1650,28 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
     // buffer stays with the handle at the size this data needed, where a
     // handed-over one would be sized afresh by the next call, and the join
     // run twice whenever a point has more than 16 pairs on average.
-    unsigned long long* out = pbuf;
+    DeviceHold own;
     if (o.pairs == MISTIC_PAIRS_DEVICE && !caller_buf) {
-      void* dp = nullptr;
-      if (cudaMalloc(&dp, std::max<size_t>(8, stored * 8)) == cudaSuccess)
-        out = (unsigned long long*)dp;
-      else
+      const size_t bytes = std::max<size_t>(8, stored * 8);
+      if (!h->arena.may_grow(bytes) || cudaMalloc(&own.p, bytes) != cudaSuccess) {
         cudaGetLastError();  // no room for both: the join's buffer goes to the result
+        own.p = nullptr;
+      } else if (h->arena.growth_left != SIZE_MAX) {
+        h->arena.growth_left -= bytes;
+      }
     }
-    // the result's from here on: freed with it if the call fails
-    if (out != pbuf) {
-      r->pairs = (uint32_t*)out;
-      r->pairs_on_device = 1;
-      r->_owner = (void*)out;
-    }
+    unsigned long long* out = own.p ? (unsigned long long*)own.p : pbuf;
     if (o.sort_pairs && stored > 1)
       sort_pairs_ij(h, pbuf, out, stored, n, nullptr, 0);
     else
       pairs_to_ij(h, pbuf, out, stored);
     r->pairs_len = stored;
+    if (own.p) {
+      r->pairs = (uint32_t*)own.p;
+      r->pairs_on_device = 1;
+      r->_owner = own.p;
+      own.p = nullptr;
+    }
     if (o.pairs == MISTIC_PAIRS_HOST) {
       uint32_t* hp = (uint32_t*)pinned_cache().acquire(std::max<size_t>(1, stored * 8));
       if (!hp) hp = (uint32_t*)malloc(std::max<size_t>(1, stored * 8));
