@@ -309,7 +309,11 @@ size_t scan_partials_count(size_t n);
 // (0/1) holds the result.
 int radix_sort_u64(mistic_handle_s* h, uint64_t* keys[2], uint32_t* vals[2], size_t n, int bits);
 
-// ---- rows.cu: np packed pairs (i << 32 | j, i < j < n), sorted by (i, j) and
+// ---- rows.cu
+// Takes the buffers that sorting np pairs of n rows needs (csr: building the
+// neighbour table) into the arena; the functions below then allocate nothing.
+void reserve_row_sort(mistic_handle_s* h, size_t np, size_t n, bool csr);
+// np packed pairs (i << 32 | j, i < j < n), sorted by (i, j) and
 // stored in memory order (i, j) in out (which may be pairs); in a fused batch
 // (row0 of n_inst instances) with ids relative to their instance.
 void sort_pairs_ij(mistic_handle_s* h, const unsigned long long* pairs, unsigned long long* out, size_t np, size_t n,

@@ -1650,18 +1650,21 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
     // buffer stays with the handle at the size this data needed, where a
     // handed-over one would be sized afresh by the next call, and the join
     // run twice whenever a point has more than 16 pairs on average.
+    // The block is a luxury (24 bytes a pair with the sort's scratch, 16 in
+    // place): it is taken after the scratch, and where it does not fit the list
+    // is sorted in the join's buffer, which then goes to the result.
+    const bool sorting = o.sort_pairs && stored > 1;
+    if (sorting) reserve_row_sort(h, stored, n, false);
     DeviceHold own;
     if (o.pairs == MISTIC_PAIRS_DEVICE && !caller_buf) {
       const size_t bytes = std::max<size_t>(8, stored * 8);
       if (!h->arena.may_grow(bytes) || cudaMalloc(&own.p, bytes) != cudaSuccess) {
-        cudaGetLastError();  // no room for both: the join's buffer goes to the result
+        cudaGetLastError();
         own.p = nullptr;
-      } else if (h->arena.growth_left != SIZE_MAX) {
-        h->arena.growth_left -= bytes;
       }
     }
     unsigned long long* out = own.p ? (unsigned long long*)own.p : pbuf;
-    if (o.sort_pairs && stored > 1)
+    if (sorting)
       sort_pairs_ij(h, pbuf, out, stored, n, nullptr, 0);
     else
       pairs_to_ij(h, pbuf, out, stored);

@@ -363,16 +363,33 @@ __global__ void __launch_bounds__(RL_THREADS, 4) k_row_sort_long(const RowOut R)
 
 }  // namespace
 
-static void sort_rows(mistic_handle_s* h, const unsigned long long* in, size_t np, size_t n, RowOut R) {
+namespace {
+struct RowScratch {
+  uint32_t *off, *rank, *ids, *lrows;
+  size_t max_long;  // at most this many rows can hold more than ROW_REG_MAX entries
+};
+
+RowScratch row_scratch(mistic_handle_s* h, size_t np, size_t n, bool both) {
   // 32-bit offsets and ranks
   if (np > 0xffffffffull) throw Error(MISTIC_ERR_TOO_LARGE, "sorting supports < 2^32 pairs");
+  const size_t dir = (both ? 2 : 1) * np, entries = dir + (both ? n : 0);
+  RowScratch s;
+  s.max_long = entries / ROW_REG_MAX + 1;
+  s.off = (uint32_t*)h->arena.get("row_off", (n + 1) * sizeof(uint32_t));
+  s.rank = (uint32_t*)h->arena.get("row_rank", dir * sizeof(uint32_t));
+  s.ids = (uint32_t*)h->arena.get("row_ids", entries * sizeof(uint32_t));
+  s.lrows = (uint32_t*)h->arena.get("row_long", (s.max_long + 2) * sizeof(uint32_t));
+  return s;
+}
+}  // namespace
+
+void reserve_row_sort(mistic_handle_s* h, size_t np, size_t n, bool csr) { row_scratch(h, np, n, csr); }
+
+static void sort_rows(mistic_handle_s* h, const unsigned long long* in, size_t np, size_t n, RowOut R) {
   const bool both = R.csr != 0;
-  uint32_t* off = (uint32_t*)h->arena.get("row_off", (n + 1) * sizeof(uint32_t));
-  uint32_t* rank = (uint32_t*)h->arena.get("row_rank", (both ? 2 : 1) * np * sizeof(uint32_t));
-  uint32_t* ids = (uint32_t*)h->arena.get("row_ids", ((both ? 2 : 1) * np + (both ? n : 0)) * sizeof(uint32_t));
-  // at most this many rows can hold more than ROW_REG_MAX entries
-  const size_t max_long = ((both ? 2 : 1) * np + (both ? n : 0)) / ROW_REG_MAX + 1;
-  uint32_t* lrows = (uint32_t*)h->arena.get("row_long", (max_long + 2) * sizeof(uint32_t));
+  const RowScratch sc = row_scratch(h, np, n, both);
+  uint32_t *off = sc.off, *rank = sc.rank, *ids = sc.ids, *lrows = sc.lrows;
+  const size_t max_long = sc.max_long;
   MCK(cudaMemsetAsync(off, 0, (n + 1) * sizeof(uint32_t), h->stream));
   MCK(cudaMemsetAsync(lrows, 0, 2 * sizeof(uint32_t), h->stream));
   const size_t tile = RW_THREADS * RW_ITEMS;

@@ -5,7 +5,9 @@ the join's buffer.
   buffer is sized by the first call and stays with the handle).
 - Where device memory ends during the sort and the call fails, nothing is left
   in its result, and the handle works on.  MISTIC_TEST_DEVICE_GROWTH sets the
-  bytes a call may add to what its handle holds."""
+  bytes a call may add to what its handle holds.
+- Where it ends between the sort's scratch and that block, the list is sorted
+  in the join's buffer: 16 bytes a pair instead of 24."""
 import ctypes
 
 import numpy as np
@@ -75,4 +77,18 @@ def test_a_failed_call_leaves_nothing(monkeypatch, room):
         monkeypatch.delenv("MISTIC_TEST_DEVICE_GROWTH")
         st, r = _device_list(h, x, eps, True)
         assert st == L.OK and np.array_equal(_host(r), ref)
+        h.lib.mistic_result_free(ctypes.byref(r))
+
+
+def test_sorted_in_place_without_room_for_a_block(monkeypatch):
+    x, eps = _points()
+    ref = O.brute_pairs(x, eps)
+    with mistic.Handle(0) as h:
+        st, r = _device_list(h, x, eps, False)  # sizes every buffer of the join
+        assert st == L.OK
+        h.lib.mistic_result_free(ctypes.byref(r))
+        monkeypatch.setenv("MISTIC_TEST_DEVICE_GROWTH", str(10 * len(ref)))
+        st, r = _device_list(h, x, eps, True)
+        assert st == L.OK and r.pairs_on_device
+        assert np.array_equal(_host(r), ref)
         h.lib.mistic_result_free(ctypes.byref(r))
