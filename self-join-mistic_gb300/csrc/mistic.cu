@@ -987,7 +987,11 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
   // 0.2 ms of launches and read-backs, at 168,656 x 90 about 13 against 5.5 ms.
   const bool wide = use_tc && (tf32_mode || join::tc_kp(d) > 128 ||
                                ((!ex || n >= 16384) && tcw_for_medium_rows(d, eps2, R)));
-  const int prec = wide ? tc_precision(o.mode, d, eps2, R) : 0;
+  // Rows that the short-row kernel would take with split operands (31 and 32
+  // columns, medium rows of a batch) keep them here: the kernel is chosen for
+  // its speed, and single bf16 would halve their operands' bits with it.
+  const bool keep_split = !tf32_mode && join::tc_kp(d) <= 128 && (ex || d <= 32);
+  const int prec = wide && !keep_split ? tc_precision(o.mode, d, eps2, R) : 0;
   r->mode_used = fp64 ? MISTIC_MODE_FP64
                       : (use_tc ? (tf32_mode ? MISTIC_MODE_TF32 : MISTIC_MODE_BF16) : MISTIC_MODE_FP32);
   clk.mark();  // 5
