@@ -30,6 +30,7 @@ constexpr uint32_t ROW_REG_MAX = 256;        // rows sorted in a warp's register
 constexpr uint32_t ROW_BLOCK_MAX = 8192;     // rows sorted in a block's registers
 constexpr int RL_THREADS = 256;              // block of the long-row kernel
 constexpr int RL_BINS = 256;
+constexpr int RL_ITEMS = 8;                  // entries a thread ranks between barriers of its radix sort
 
 // BOTH: an entry in either row of the pair (the neighbour table); else one in
 // row i (the pair list).
@@ -88,6 +89,7 @@ struct RowOut {
   const uint32_t* off;         // n + 1
   size_t n;
   uint32_t* ids;               // entries, row by row, unsorted
+  uint32_t* rank;              // their ranks, no longer needed: scratch, row i's from off[i] on
   int csr;                     // rows hold their own id too (start at off[i] + i)
   unsigned long long* pairs;   // pair list: entry e as (i, j) in memory order
   uint32_t* nbrs;              // neighbour table: ids
@@ -265,12 +267,55 @@ __global__ void __launch_bounds__(RW_THREADS) k_row_sort(const RowOut R) {
   }
 }
 
+// A row whose ids, all different, fill a bitmap of n bits: the bits are set,
+// then written out in order behind a running count.
+__device__ __forceinline__ void sort_by_bitmap(const RowOut& R, size_t b, uint32_t len, uint32_t i, uint32_t r0,
+                                            uint32_t* ws) {
+  const uint32_t words = (uint32_t)((R.n + 31) / 32);
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  uint32_t* bm = R.rank + R.off[i];
+  for (uint32_t t = tid; t < words; t += RL_THREADS) bm[t] = 0u;
+  __syncthreads();
+#pragma unroll 8
+  for (uint32_t t = tid; t < len; t += RL_THREADS) {
+    const uint32_t v = R.ids[b + t];
+    atomicOr(&bm[v >> 5], 1u << (v & 31));
+  }
+  __syncthreads();
+  uint32_t base = 0;  // entries written before this step's words
+  for (uint32_t t0 = 0; t0 < words; t0 += RL_THREADS) {
+    uint32_t m = t0 + tid < words ? __ldcg(&bm[t0 + tid]) : 0u;
+    uint32_t incl = __popc(m);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(FULL_MASK, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) ws[w] = incl;
+    __syncthreads();
+    uint32_t pos = base + incl - __popc(m), total = 0;
+    for (int q = 0; q < RL_THREADS / 32; ++q) {
+      pos += q < w ? ws[q] : 0u;
+      total += ws[q];
+    }
+    for (; m; m &= m - 1) put(R, b + pos++, i, 32u * (t0 + tid) + __ffs(m) - 1, r0);
+    base += total;
+    __syncthreads();
+  }
+}
+
 // Rows above ROW_REG_MAX entries, a block a row, claimed from the list.  Up
 // to ROW_BLOCK_MAX entries are sorted in the block's registers (in shared
 // memory, a barrier a step, these rows took 2.0 ms of a 5M x 18 join's sorted
-// list; now 1.0); longer rows by a
+// list; now 1.0).  Longer rows: by a bitmap of the n ids in the place of the
+// row's ranks where that is large enough (n / 32 entries); shorter ones by a
 // stable 8-bit radix sort through global memory, between the unsorted ids and
 // the row's own place in the output (which is at least as large).
+// One block sorts a row however long, so a lone row of nearly n entries (a point
+// amid all others) ends the pass: of 50,000, 200,000 and 1M rows (90 columns,
+// joins of 0.4, 5.8 and 143 ms) 0.16, 0.58 and 2.4 ms for the whole sorted list;
+// 0.69, 2.7 and 13.6 by a radix sort that ranked an entry a thread.  Where all
+// rows are long: 40,000 near duplicates, 8e8 pairs, 37 -> 17.5 ms.
 __global__ void __launch_bounds__(RL_THREADS, 4) k_row_sort_long(const RowOut R) {
   extern __shared__ uint32_t sv[];  // ROW_BLOCK_MAX
   __shared__ uint32_t s_claim, wcnt[RL_THREADS / 32][RL_BINS], ws[RL_THREADS / 32], gbase[RL_BINS];
@@ -308,6 +353,10 @@ __global__ void __launch_bounds__(RL_THREADS, 4) k_row_sort_long(const RowOut R)
         row(std::integral_constant<int, 32>());
       continue;
     }
+    if (R.off[i + 1] - R.off[i] >= (R.n + 31) / 32) {
+      sort_by_bitmap(R, b, len, i, r0, ws);
+      continue;
+    }
     uint32_t* src = R.ids + b;
     uint32_t* dst = R.csr ? R.nbrs + b : reinterpret_cast<uint32_t*>(R.pairs + b);
     for (int shift = 0; shift < 32; shift += 8) {
@@ -327,28 +376,40 @@ __global__ void __launch_bounds__(RL_THREADS, 4) k_row_sort_long(const RowOut R)
       uint32_t pre = 0;
       for (int q = 0; q < w; ++q) pre += ws[q];
       gbase[tid] = pre + x - c;
-      // tiles of RL_THREADS entries in order: rank among equal digits before
-      // it in the warp, in the warps before it, then in the tiles before it
-      for (uint32_t t0 = 0; t0 < len; t0 += RL_THREADS) {
+      // tiles of RL_THREADS x RL_ITEMS entries in order, each warp a run of
+      // them: rank among equal digits before it in the warp's run, in the warps
+      // before it, then in the tiles before it
+      for (uint32_t t0 = 0; t0 < len; t0 += RL_THREADS * RL_ITEMS) {
         for (int q = 0; q < RL_THREADS / 32; ++q) wcnt[q][tid] = 0;
         __syncthreads();
-        const uint32_t t = t0 + tid;
-        const bool ok = t < len;
-        const uint32_t v = ok ? src[t] : 0u;
-        const uint32_t dg = ok ? (v >> shift) & 255u : RL_BINS + lane;
-        const uint32_t peers = __match_any_sync(FULL_MASK, dg);
-        const uint32_t lt = __popc(peers & ((1u << lane) - 1u));
-        if (ok && lt == 0) wcnt[w][dg] = __popc(peers);
-        __syncthreads();
-        if (ok) {
-          uint32_t pos = gbase[dg] + lt;
-          for (int q = 0; q < w; ++q) pos += wcnt[q][dg];
-          dst[pos] = v;
+        const uint32_t tw = t0 + w * 32 * RL_ITEMS + lane;
+        uint32_t v[RL_ITEMS], rk[RL_ITEMS];
+#pragma unroll
+        for (int r = 0; r < RL_ITEMS; ++r) v[r] = tw + 32 * r < len ? src[tw + 32 * r] : 0u;
+#pragma unroll
+        for (int r = 0; r < RL_ITEMS; ++r) {
+          const bool ok = tw + 32 * r < len;
+          const uint32_t dg = ok ? (v[r] >> shift) & 255u : RL_BINS + lane;
+          const uint32_t peers = __match_any_sync(FULL_MASK, dg);
+          const uint32_t lt = __popc(peers & ((1u << lane) - 1u));
+          const uint32_t before = ok ? wcnt[w][dg] : 0u;
+          __syncwarp();
+          if (ok && lt == 0) wcnt[w][dg] = before + __popc(peers);
+          __syncwarp();
+          rk[r] = before + lt;
         }
         __syncthreads();
-        uint32_t add = 0;
-        for (int q = 0; q < RL_THREADS / 32; ++q) add += wcnt[q][tid];
-        gbase[tid] += add;
+        uint32_t run = gbase[tid];
+        for (int q = 0; q < RL_THREADS / 32; ++q) {
+          const uint32_t c = wcnt[q][tid];
+          wcnt[q][tid] = run;
+          run += c;
+        }
+        gbase[tid] = run;
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < RL_ITEMS; ++r)
+          if (tw + 32 * r < len) dst[wcnt[w][(v[r] >> shift) & 255u] + rk[r]] = v[r];
         __syncthreads();
       }
       uint32_t* sw = src;
@@ -412,6 +473,7 @@ static void sort_rows(mistic_handle_s* h, const unsigned long long* in, size_t n
   R.off = off;
   R.n = n;
   R.ids = ids;
+  R.rank = rank;
   R.long_n = lrows;
   R.long_rows = lrows + 2;
   // 32 rows a warp, fewer while that leaves the SMs without 16 warps each
