@@ -585,8 +585,8 @@ __device__ __forceinline__ float sq4(float4 x, float4 y, float s) {
 }
 
 __global__ void __launch_bounds__(256) k_band_check(const JoinParams P) {
-  // ring mode: the slice [band0, band1) of the band list, entries of deferred
-  // units skipped, accepted pairs written with their unit's tag (the slice
+  // ring mode: the slice [band0, band1) of the band list, slots without an
+  // entry and entries of deferred units skipped, accepted pairs written with their unit's tag (the slice
   // is sized to fit the ring); otherwise the whole list
   const unsigned long long n =
       P.ring ? P.band1 : min(*(volatile unsigned long long*)&P.ctr->band_n, P.band_cap);
@@ -602,7 +602,8 @@ __global__ void __launch_bounds__(256) k_band_check(const JoinParams P) {
     uint32_t tag = 0;
     if (i < n && P.ring) {
       tag = P.band_tags[i];
-      if (P.deferred[tag]) e = ~0ull;  // that unit runs again: its band entries come again
+      // a slot that holds nothing, or a unit that runs again (its band entries come again)
+      if (tag == RING_INVALID || P.deferred[tag]) e = ~0ull;
     }
     const bool coop = !P.insts && P.inv && P.dpad32 >= BAND_COOP_MIN;  // launch-uniform
     float s_coop = 0.f;
