@@ -571,8 +571,12 @@ k_join_f64(const JoinParams P) {
 // FP32 pre-decision of long rows: with a lane reading both rows of its pair on
 // its own, every 32-byte sector was fetched twice; 8 lanes now share a pair's
 // rows, 4 pairs of the warp at a time (1M x 384, 4.2e7 band pairs: 22.9 ->
-// 7.0 ms).  Rows below 32 columns stay with one lane.
-constexpr uint32_t BAND_COOP_MIN = 32;
+// 7.0 ms).  The sharing costs about the same whatever the rows, so rows below
+// 96 columns stay with one lane; 3.3e7 band pairs of repeated points, one lane /
+// shared, ms: 40 columns 0.87 / 1.82, 57 1.02 / 1.82, 90 1.43 / 1.93, 126 3.95 /
+// 1.66.  (Rows that are not repeated: 90 columns 0.049 / 0.046 a 2.6e5, 126
+// 0.038 / 0.031 a 9.4e4.)
+constexpr uint32_t BAND_COOP_MIN = 96;
 __device__ __forceinline__ float sq4(float4 x, float4 y, float s) {
   float t = x.x - y.x;
   s = fmaf(t, t, s);

@@ -1,0 +1,37 @@
+"""Band decisions of repeated points: most candidate pairs are left to them,
+and their rows are in cache.
+
+Rows on both sides of the length from which 8 lanes share a pair's rows."""
+import numpy as np
+import pytest
+
+from helpers import diff_pairs
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _repeated(n, points, d):
+    r = np.random.default_rng(d)
+    return r.random((points, d))[r.integers(0, points, n)]
+
+
+@pytest.mark.parametrize("d", [31, 92, 93, 96, 97, 126, 130])
+def test_repeated_points(handle, d):
+    x = _repeated(9000, 900, d)
+    r = handle.selfjoin(x, 1, 5e-4, mode="bf16", pairs="host", sort_pairs=True)
+    assert r.band_pairs > 0 and r.pairs_ij > 0
+    ref = O.brute_pairs(x, 5e-4)
+    assert np.array_equal(r.pairs, ref), diff_pairs(r.pairs, ref)
+
+
+def test_short_rows_are_not_decided_slowly(handle):
+    """3.3e7 band pairs of 40 columns: 0.88 ms by one lane a pair, half as
+    much again is the limit."""
+    x = _repeated(90000, 1800, 40)
+    ms = []
+    for _ in range(6):
+        r = handle.selfjoin(x, 1, 0.003)
+        assert r.band_pairs > 1e7
+        ms.append(r.ms["join"] - r.ms["join_simt"] - r.ms["join_tc"])
+    assert min(ms) < 1.32
