@@ -11,11 +11,13 @@
 //    sorted, and non-empty bins become contiguous runs of the sorted order.
 //  - the 3^k neighbour search over sorted bin keys, generateRanges /
 //    binarySearch in src/tree.cu:596-759,886-996 (device form
-//    GPUBinarySearch, src/kernel.cu:164-224).  Here one thread per non-empty
-//    bin walks the ±1 neighbourhood depth-first, narrowing a sorted range one
-//    key field at a time (the top fields through a direct-address prefix
-//    table), so empty prefixes are pruned early; only neighbours of index >=
-//    the home bin are emitted (each unordered bin pair once).
+//    GPUBinarySearch, src/kernel.cu:164-224).  Here a warp per non-empty bin
+//    compares the keys that can be near where bins are few; where they are
+//    many, up to 8 threads a bin walk the ±1 neighbourhood depth-first,
+//    narrowing a sorted range one key field at a time (the top fields through
+//    a direct-address prefix table), so empty prefixes are pruned early.  Only
+//    neighbours of index >= the home bin are emitted (each unordered bin pair
+//    once).
 #include <math.h>
 
 #include "internal.cuh"
@@ -1083,9 +1085,10 @@ void prefix_table(mistic_handle_s* h, const uint64_t* bkey, uint32_t m, const En
 // 9,867 bins 0.340 / 0.627, 16,761 0.708 / 0.815, 26,116 1.376 / 1.200.
 bool enum_flat(uint32_t m, const EnumParams& P) { return m <= (P.k > 6 ? 20480u : 10240u); }
 
-// Threads a bin: up to 8, while the device holds them about at once (152 SMs
-// x 1,024 threads); beyond that the extra searches cost more than the shorter
-// chains give.  ms at 1 / 2 / 4 / 8 threads: k = 6: 28,357 bins 0.725 / 0.514
+// Threads a bin: up to 8, while they are 256 K threads in all, or 640 K where
+// three levels or more are walked below the table (1.7 and 4.2 times what the
+// device holds at once): beyond that the extra searches cost more than the
+// shorter chains give.  ms at 1 / 2 / 4 / 8 threads: k = 6: 28,357 bins 0.725 / 0.514
 // / 0.403 / 0.359, 76,372 0.926 / 0.691 / 0.719 / 0.752, 136,090 1.061 / 1.042
 // / 1.166 / 1.289.  With three levels or more below the table the chains are
 // longer: k = 8: 129,896 bins 8.12 / 6.22 / 5.21 / 5.48, 321,117 12.6 / 10.7 /

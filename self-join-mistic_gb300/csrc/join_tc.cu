@@ -1263,7 +1263,7 @@ namespace join {
 
 int tc_kp(uint32_t d) { return (int)(((d + 2) + 15) / 16 * 16); }
 // Home rows per tensor-core unit: G chunks of 128 share each converted
-// candidate tile (G = 2 while the operands leave room for two CTAs per SM).
+// candidate tile, as many as fit beside the stages of one CTA's 200 KB (TcShape).
 // Longer rows go to the K-chunked kernel (join_tcw.cu), 256 home rows a unit.
 uint32_t tc_rows(uint32_t d) {
   const int kp = tc_kp(d);

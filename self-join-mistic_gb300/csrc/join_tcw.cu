@@ -904,7 +904,7 @@ __global__ void __launch_bounds__(WTHREADS, 1)
   } else if (warp >= WEPI0 && warp < WEPI0 + WNEPI) {
     // ============================ epilogue
     // warp w reads TMEM lane quarter w % 4 (the hardware's access rule) and
-    // the 32-column blocks (w - WEPI0) / 4, + 2, + 4, ... of each accumulator
+    // the 32-column blocks (w - WEPI0) / 4, + WNEPI / 4, ... of each accumulator
     const uint32_t quarter = warp & 3;
     const uint32_t cblk0 = (warp - WEPI0) >> 2;
     PairStage ps{pstage + (warp - WEPI0) * PSTAGE, 0, 0, P.pairs_ij != 0};

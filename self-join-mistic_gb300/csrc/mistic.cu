@@ -417,7 +417,16 @@ int bit_length(uint64_t v) {
 //   250,007 x 18:   T = 16: 2.79, 24: 2.66, 32: 2.64, 40: 2.61, 49: 2.64, 66: 2.67
 //   100,000 x 18:   T = 16: 1.65, 24: 1.62, 32: 1.62, 40: 1.62, 49: 1.63, 66: 1.65
 //   515k x 90 (short-row kernel): T = 1: 259.9, 2: 261.9, 4: 261.9, 8: 263.3
-// hence 16000 / d^2, clamped to [1, 96].
+// hence 16000 / d^2, clamped to [1, 96].  Over d, 250,000 points, uniform /
+// clustered (whole join, ms; the rule's T marked):
+//   d = 10: T = 80: 3.02 / 2.01, *96: 3.09 / 2.09, 192: 3.67 / 2.45
+//   d = 14: T = 40: 5.49 / 3.67, *81: 5.59 / 3.92, 192: 7.12 / 4.86
+//   d = 16: T = 31: 6.68 / 4.97, *62: 6.78 / 5.09, 96: 6.95 / 5.36
+//   d = 20: T = 20: 7.23 / 6.12, *40: 7.23 / 6.11, 72: 7.33 / 6.27
+//   d = 24: T = 13: 7.08 / 7.28, *27: 7.09 / 7.23, 50: 7.09 / 7.34
+//   d = 30: T = 8: 7.23 / 8.60, *17: 7.23 / 8.51, 32: 7.23 / 8.57
+// From d = 18 up it is within about 1 % of the best; below, smaller values would
+// be 2 to 7 % faster.
 uint32_t tc_min_bin(uint32_t d, bool wide) {
   const char* e = getenv("MISTIC_TC_MIN_BIN");
   if (e && *e) return (uint32_t)std::max(1l, strtol(e, nullptr, 10));
@@ -457,7 +466,7 @@ double tc_kappa(uint32_t d, bool wide, int prec) {
 // Operand precision of the K-chunked tensor-core join.  TF32 mode: tf32.
 // Otherwise single bf16 (a third of the split's tensor work) when even the
 // widest column's bound -- rows at the largest norm R from the centre --
-// stays within the cap of eps^2 / 10 (no column is left wholly to FP64);
+// stays within eps^2 / 10 (a narrow band);
 // else split bf16.  MISTIC_TC_PREC=split|bf16 overrides (tuning).
 int tc_precision(mistic_mode mode, uint32_t d, double eps2, double R) {
   if (mode == MISTIC_MODE_TF32) return 2;
@@ -983,8 +992,12 @@ void run_selfjoin(mistic_handle h, const void* pts, uint64_t n, uint32_t d, mist
   // The fused batch join drains medium rows with the short-row kernel only;
   // that kernel needs about four times the K-chunked one's time a cell
   // there, so only instances too small to repay a join of their own stay in
-  // it: at 15,000 x 90 (1e8 candidate pairs) that is 0.15 ms fused against
-  // 0.2 ms of launches and read-backs, at 168,656 x 90 about 13 against 5.5 ms.
+  // it.  Batches of 8 members of 16,384 points, short-row / K-chunked kernel,
+  // ms: d = 31 2.95 / 1.98, 57 3.28 / 2.23, 90 4.52 / 2.53, 126 5.75 / 3.42; of
+  // 24,000 points 4.39 / 2.67, 4.73 / 3.05, 7.09 / 3.44, 9.19 / 4.59.  Of smaller
+  // members a batch has many, and the two come closer, fused against each on a
+  // worker of its own: 400 members of 2,000 points d = 57 37.9 / 36.1, 90 46.1 /
+  // 46.1; 200 of 8,000 40.1 / 35.0, 48.2 / 39.6.
   const bool wide = use_tc && (tf32_mode || join::tc_kp(d) > 128 ||
                                ((!ex || n >= 16384) && tcw_for_medium_rows(d, eps2, R)));
   // Rows that the short-row kernel would take with split operands (31 and 32
