@@ -26,12 +26,14 @@ def test_repeated_points(handle, d):
 
 
 def test_short_rows_are_not_decided_slowly(handle):
-    """3.3e7 band pairs of 40 columns: 0.88 ms by one lane a pair, half as
-    much again is the limit."""
-    x = _repeated(90000, 1800, 40)
-    ms = []
-    for _ in range(6):
-        r = handle.selfjoin(x, 1, 0.003)
-        assert r.band_pairs > 1e7
-        ms.append(r.ms["join"] - r.ms["join_simt"] - r.ms["join_tc"])
-    assert min(ms) < 1.32
+    """3.3e7 band pairs of 40 columns take 0.87 ms by one lane a pair and 1.82
+    shared, as many of 126 columns 1.66: 0.52 and 1.1 of it, whatever the
+    clocks.  0.8 is the limit."""
+    ms = {}
+    for d in (40, 126):
+        x = _repeated(90000, 1800, d)
+        for _ in range(6):
+            r = handle.selfjoin(x, 1, 0.003)
+            assert r.band_pairs > 1e7
+            ms[d] = min(ms.get(d, 1e9), r.ms["join"] - r.ms["join_simt"] - r.ms["join_tc"])
+    assert ms[40] < 0.8 * ms[126]

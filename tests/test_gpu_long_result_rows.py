@@ -47,8 +47,9 @@ def test_one_long_row(handle, leaves, n, out):
 
 
 def test_a_lone_long_row_is_not_sorted_slowly(handle):
-    """200,001 rows, one with 200,000 entries.  The radix sort of whole pairs
-    took 0.24 ms whatever the rows; five times that is the limit."""
+    """200,001 rows, one with 200,000 entries: the list takes 0.58 ms, a tenth of
+    the join (2.7 ms, 0.46 of it, where one block ranked an entry a thread); a
+    quarter is the limit, whatever the clocks."""
     x, _ = _star(200000, 200001, 90, 1, first=True)
-    ms = [handle.selfjoin(x, 6, 1.0, pairs="device", sort_pairs=True).ms["d2h"] for _ in range(6)]
-    assert min(ms) < 1.2
+    r = [handle.selfjoin(x, 6, 1.0, pairs="device", sort_pairs=True).ms for _ in range(6)]
+    assert min(m["d2h"] for m in r) < 0.25 * min(m["join"] for m in r)
